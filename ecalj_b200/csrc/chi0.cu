@@ -61,14 +61,6 @@ static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc)
   return (bt.maxcnt + ZG_BK - 1) / ZG_BK;
 }
 
-static int choose_splitk(int ntiles, int nbins, int maxch) {
-  const long long ctas = static_cast<long long>(ntiles) * nbins;
-  const long long slots = 2LL * ctx().sm_count;
-  if (ctas >= slots || maxch < 16) return 1;
-  int sk = static_cast<int>((slots + ctas - 1) / ctas);
-  return std::max(1, std::min(sk, maxch / 8));
-}
-
 static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int nwhis, int npm,
                          int ns1, int ns2, const double2* zmel, int nbb, int nm1, int nm2,
                          int nqtot, int icounkmink, int icounkmaxk, const int* itc, const int* itpc,
@@ -155,7 +147,7 @@ static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int n
   const int herm = (ipr_col == 1 && npr_col == npr) ? 1 : 0;
   const int ntiles = herm ? p.ntm * (p.ntm + 1) / 2 : p.ntm * p.ntn;
   const int nbins = static_cast<int>(bt.cnt.size());
-  const int sk = choose_splitk(ntiles, nbins, maxch);
+  const int sk = zgemm_splitk(static_cast<long long>(ntiles) * nbins, maxch);
   p.kch_per_split = (maxch + sk - 1) / sk;
   rc = zgemm_chi0_launch(p, nbins, herm, sk, s);
   if (rc) return rc;
@@ -342,14 +334,6 @@ int chi0_lorentz_weights(int niw, const double* freq_i, int nk, const int* nocc,
   return QSGW_OK;
 }
 
-static DevBuf g_lz_ident;
-
-__global__ void iota_kernel(int* a, long long n) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    a[i] = static_cast<int>(i);
-}
-
 // chi = Hre + i Him for the real axis (Hre, Him: the Re-weight and Im-weight slots)
 __global__ void combine_re_im_kernel(double2* __restrict__ chi, const double2* __restrict__ hre,
                                      const double2* __restrict__ him, long long n) {
@@ -441,17 +425,11 @@ static int chi0_run(double* chi0_d, int npr, int niw, const double* zcols_d, int
     return chi0_split_f16(reinterpret_cast<double2*>(chi0_d), npr, niw,
                           reinterpret_cast<const double2*>(zcols_d), ldz, npair, w_d, s);
   }
-  rc = g_lz_ident.ensure(npair * sizeof(int));
-  if (rc) return rc;
-  iota_kernel<<<static_cast<int>(std::min<long long>((npair + 255) / 256, 4096)), 256, 0, s>>>(
-      g_lz_ident.as<int>(), npair);
-  count_launch();
-  QSGW_LAUNCH_CHECK("iota_kernel");
   // one bin per iw, all pairs in every bin, bin iw's weights at offset iw*npair
   std::vector<long long> off(2 * niw);
   std::vector<int> cs(2 * niw);
   for (int iw = 0; iw < niw; ++iw) {
-    off[iw] = 0;                                  // column offsets (shared identity list)
+    off[iw] = 0;                                  // no column list
     off[niw + iw] = static_cast<long long>(iw) * npair;   // weight offsets
     cs[iw] = static_cast<int>(npair);
     cs[niw + iw] = iw;                            // slab
@@ -471,11 +449,11 @@ static int chi0_run(double* chi0_d, int npr, int niw, const double* zcols_d, int
   p.bin_woff = reinterpret_cast<const long long*>(base) + niw;
   p.bin_cnt = reinterpret_cast<const int*>(base + 2 * niw * sizeof(long long));
   p.bin_slab = p.bin_cnt + niw;
-  p.colidx = g_lz_ident.as<int>();
+  p.colidx = nullptr;                              // every bin holds every column in order
   p.wts = w_d;
   const int maxch = static_cast<int>((npair + ZG_BK - 1) / ZG_BK);
   const int ntiles = p.ntm * (p.ntm + 1) / 2;
-  const int heur = choose_splitk(ntiles, niw, maxch);
+  const int heur = zgemm_splitk(static_cast<long long>(ntiles) * niw, maxch);
   // split K: the autotuner times the heuristic and its neighbours (x1/2, x2, x4) on this shape
   auto run = [&](int sk, bool clear) -> int {      // trials clear chi0 (it was cleared above)
     ZParams q = p;

@@ -498,11 +498,12 @@ static int sxcf_contract(const qsgw_sxcf_args& a, SigcSplitArgs& sa) {
     p.tile_cols = reinterpret_cast<const int*>(put(sa.tile_cols.data(), sa.tile_cols.size() * sizeof(int)));
     if (cprc) return cprc;
     // ---- 3. imaginary axis + poles in one launch
-    p.M = a.ngb; p.K = a.ngb;
+    p.M = a.ngb; p.N = static_cast<int>(pl.ncol); p.K = a.ngb;
     p.a_rs = sa.ldw; p.a_ks = 1; p.a_conj = 1;          // Wc^H (:492 opA = m_op_C)
     p.B = sa.zmel; p.b_rs = a.ngb; p.b_ks = 1; p.b_conj = 0;
-    p.C = sa.out; p.ldc = a.ngb; p.beta_zero = 1;
-    rc = zgemm_seg_launch(p, static_cast<int>(sa.tile_group.size()), s);
+    p.C = sa.out; p.ldc = a.ngb;
+    const int ntile = static_cast<int>(sa.tile_group.size());
+    rc = zgemm_seg_launch(p, ntile, static_cast<int>(sa.segs.size()) / std::max(ntile, 1), s);
   }
   return rc;
 }

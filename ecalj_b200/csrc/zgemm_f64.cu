@@ -2,6 +2,7 @@
 // replace the reference's BLAS shim zmm_h / zmm_d (m_blas.f90:198-228,
 // 469-498).
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include "zgemm_f64.cuh"
 
@@ -165,6 +166,23 @@ __global__ void zscale_kernel(double2* C, long long ldc, long long c_bs, int m, 
   }
 }
 
+// A launch of ctas * sk CTAs of nch / sk chunks each runs in waves of two CTAs an SM; a last wave of at
+// most one CTA an SM takes about 0.6 of a full one (measured: one CTA alone keeps 0.8 of the DMMA
+// rate that two do).  A split costs its CTA about 4 chunk times of pipeline fill and atomic epilogue.
+int zgemm_splitk(long long ctas, int nch) {
+  const double slots = 2.0 * ctx().sm_count;
+  int best = 1;
+  double tbest = 0.0;
+  for (int sk = 1; sk <= 64 && (sk == 1 || nch / sk >= 4); ++sk) {
+    const double x = static_cast<double>(ctas) * sk / slots;
+    const double full = std::floor(x), rest = x - full;
+    const double waves = full + (rest == 0.0 ? 0.0 : (rest <= 0.5 ? 0.6 : 1.0));
+    const double t = waves * ((nch + sk - 1) / sk + (sk > 1 ? 4.0 : 2.0));
+    if (sk == 1 || t < 0.97 * tbest) { best = sk; tbest = t; }
+  }
+  return best;
+}
+
 int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
               const double2* A, long long lda, long long a_bs,
               const double2* B, long long ldb, long long b_bs, double2 beta,
@@ -190,16 +208,11 @@ int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
   }
   const int nch = (k + ZG_BK - 1) / ZG_BK;
   const long long tiles = static_cast<long long>(p.ntm) * p.ntn * nbatch;
-  const int slots = 2 * ctx().sm_count;
-  int splitk = 1;
-  if (tiles < slots && nch >= 8) {
-    splitk = static_cast<int>((slots + tiles - 1) / tiles);
-    splitk = std::min(splitk, nch / 4);
-    splitk = std::max(splitk, 1);
-  }
+  int splitk = zgemm_splitk(tiles, nch);
   p.kch_per_split = (nch + splitk - 1) / splitk;
   splitk = (nch + p.kch_per_split - 1) / p.kch_per_split;
   p.splitk = splitk;
+  p.acc_c = splitk == 1 && alpha.y == 0.0 && (alpha.x == 1.0 || alpha.x == -1.0) && beta.x == 1.0 && beta.y == 0.0;
   if (splitk > 1) {
     // beta applied up front; the tiles then add alpha*acc atomically
     dim3 g(static_cast<unsigned>(std::min<long long>((static_cast<long long>(m) * n + 255) / 256, 4096)),
@@ -224,14 +237,17 @@ int zgemm_chi0_launch(ZParams p, int nbins, int herm, int splitk, cudaStream_t s
   return launch_kernel<ZM_CHI0, true, true>(p, grid, s);
 }
 
-int zgemm_seg_launch(ZParams p, int ncol_tiles, cudaStream_t s) {
+int zgemm_seg_launch(ZParams p, int ncol_tiles, int mean_nseg, cudaStream_t s) {
   if (ncol_tiles > 65535) {
     set_error("segmented GEMM: %d column tiles exceed the grid limit", ncol_tiles);
     return QSGW_ERR_UNSUPPORTED;
   }
   p.ntm = (p.M + ZG_BM - 1) / ZG_BM;
-  p.splitk = 1;
-  dim3 grid(static_cast<unsigned>(p.ntm), ncol_tiles, 1);
+  // few tiles (one task of a small cell): the segments are split over CTAs that add into C
+  p.splitk = zgemm_splitk(static_cast<long long>(p.ntm) * ncol_tiles, mean_nseg * ((p.K + ZG_BK - 1) / ZG_BK));
+  if (p.splitk > 1)
+    QSGW_CUDA(cudaMemsetAsync(p.C, 0, static_cast<size_t>(p.ldc) * p.N * sizeof(double2), s));
+  dim3 grid(static_cast<unsigned>(p.ntm), ncol_tiles, p.splitk);
   // A = op(W): 'C' / 'T' -> k-contiguous rows, 'N' -> row-contiguous
   if (p.a_rs == 1) return launch_kernel<ZM_SEG, true, false>(p, grid, s);
   return launch_kernel<ZM_SEG, false, false>(p, grid, s);

@@ -1,11 +1,18 @@
 // Complex FP64 GEMM engine on the FP64 tensor pipe (mma.sync m16n8k8 f64,
 // "DMMA"), shared by chi0 (x0gemm), W (basis changes, Gauss-Jordan updates)
-// and Sigma_c.  One CTA computes a 64x64 complex tile with 4 warps (each
-// 32x32 = 2x4 m16n8 fragments, re and im accumulators); operands stream
+// and Sigma_c.  One CTA computes a 64x64 complex tile with 8 warps (each
+// 32x16 = 2x2 m16n8 fragments, re and im accumulators); operands stream
 // through a 3-stage cp.async pipeline in shared memory laid out [k][row]
-// with a pitch of 66 complex (conflict-free fragment loads).  The m16n8k8
-// shape does 4x the work of the m8n8k4 one per instruction with the same
-// shared-memory reads per multiply-add.
+// with a pitch of 66 complex (conflict-free fragment loads).
+//
+// What bounds it: the FP64 tensor pipe (64 FMA a clock and SM, 16 cycles of
+// it for one m16n8k8).  A warp cannot issue its DMMAs back to back, so the
+// pipe needs several warps per SM sub-partition: two CTAs of 8 warps keep
+// four there (128 registers a thread) where 4-warp CTAs of 32x32 a warp kept
+// two and lost a third of the cycles to issue waits and barriers.  1536^3:
+// 32 TFLOP/s, DMMA pipe 90 % busy (cuBLAS 35); the basis change of 24
+// matrices of 600: 1.70 -> 1.46 ms; chi0 of 260 rows, 12 800 pairs and 12
+// frequencies (with the tile rules below) 3.99 -> 2.28 ms.
 //
 // Three problem modes share the main loop:
 //   ZM_GEMM  C = alpha op(A) op(B) + beta C, batched, optional split-K.
@@ -19,11 +26,13 @@
 //            (:556-590) in one launch, weights applied per column in the
 //            B-fragment load.
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 
 namespace qsgw {
 
-constexpr int ZG_BM = 64, ZG_BN = 64, ZG_BK = 16, ZG_STAGES = 3, ZG_THREADS = 128;
+constexpr int ZG_BM = 64, ZG_BN = 64, ZG_BK = 16, ZG_STAGES = 3, ZG_THREADS = 256;
+constexpr int ZG_NI = 2, ZG_NJ = 2;              // m16 and n8 fragments of a warp
 constexpr int ZG_PA = ZG_BM + 2, ZG_PB = ZG_BN + 2;
 
 enum ZMode { ZM_GEMM = 0, ZM_CHI0 = 1, ZM_SEG = 2 };
@@ -43,11 +52,13 @@ struct ZParams {
   double2* C; long long ldc, c_bs;
   double2 alpha, beta;
   int beta_zero;           // do not read C
+  int acc_c;               // alpha = +-1 (real), beta = 1: the accumulators start from alpha C
   int splitk, kch_per_split;
   int ntm, ntn;            // tile counts
   // CHI0
   const int* bin_cnt; const long long* bin_coff; const long long* bin_woff;
-  const int* bin_slab; const int* colidx; const double* wts; int herm;
+  const int* bin_slab; const int* colidx;       // colidx null: entry k of a bin is column k 
+  const double* wts; int herm;
   // SEG
   const int* tile_group; const int* tile_cols; const int* group_seg_off;
   const int* group_nseg; const ZSeg* segs;
@@ -65,6 +76,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
   int sz = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
+  unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  int sz = valid ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -72,8 +88,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // D(16x8) += A(16x8) B(8x8), FP64.  Lane (g = lane / 4, t = lane % 4) holds A(g, t), A(g+8, t),
 // A(g, t+4), A(g+8, t+4); B(t, g), B(t+4, g); D(g, 2t), D(g, 2t+1), D(g+8, 2t), D(g+8, 2t+1).
 __device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[4], double b0, double b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
@@ -94,7 +109,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
   ZSmem& sm = *reinterpret_cast<ZSmem*>(zg_smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp & 1, wn = warp >> 1;
+  const int wm = warp >> 2, wn = warp & 3;       // the row halves on every SM sub-partition (warp mod 4)
 
   // ---- per-CTA problem setup ----
   int tm = 0, tn = 0, batch = 0, split = 0, nchunk = 0, ch0 = 0, ch1 = 0;
@@ -116,98 +131,119 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
     else { tm = blockIdx.x % p.ntm; tn = blockIdx.x / p.ntm; }
     const int bin = blockIdx.y; split = blockIdx.z;
     Kbin = p.bin_cnt[bin];
-    kcol = p.colidx + p.bin_coff[bin];
+    kcol = p.colidx ? p.colidx + p.bin_coff[bin] : nullptr;
     kw = p.wts + p.bin_woff[bin];
     Cb += static_cast<long long>(p.bin_slab[bin]) * p.c_bs;
     nchunk = (Kbin + ZG_BK - 1) / ZG_BK;
   } else {
-    tm = blockIdx.x; tn = blockIdx.y;
+    tm = blockIdx.x; tn = blockIdx.y; split = blockIdx.z;
     group = p.tile_group[tn];
     nseg = p.group_nseg[group];
     seg0 = p.group_seg_off[group];
     nchunk = nseg * ((p.K + ZG_BK - 1) / ZG_BK);
   }
-  ch0 = split * p.kch_per_split;
-  ch1 = min(nchunk, ch0 + p.kch_per_split);
-  if (MODE == ZM_SEG) { ch0 = 0; ch1 = nchunk; }
+  // SEG: the chunks of a tile's segments are dealt evenly (the tiles' segment counts differ)
+  const int kper = MODE == ZM_SEG ? (nchunk + p.splitk - 1) / p.splitk : p.kch_per_split;
+  ch0 = split * kper;
+  ch1 = min(nchunk, ch0 + kper);
   const int m0 = tm * ZG_BM, n0 = tn * ZG_BN;
   const int kch_seg = (p.K + ZG_BK - 1) / ZG_BK;
 
-  auto load_chunk = [&](int c, int st) {
-    int kbase;
-    const double2* Aseg = Ab;
-    const double* sscale = nullptr;
-    int scs = 0;
-    if (MODE == ZM_SEG) {
-      const int s = c / kch_seg;
-      kbase = (c - s * kch_seg) * ZG_BK;
-      const ZSeg sg = p.segs[seg0 + s];
-      Aseg = sg.mat; sscale = sg.scale; scs = sg.scale_cs;
-    } else {
-      kbase = c * ZG_BK;
-    }
-    const int Klim = (MODE == ZM_CHI0) ? Kbin : p.K;
-    // A operand: BK x BM elements, 8 per thread
+  // The thread's operand elements: row and k of the first, and the steps to its others (rows run fastest
+  // over the threads when they are contiguous, else k).  Columns, segment and weight addresses live in
+  // registers or come by cp.async: a plain load here would hold the warp, and with it the block's next
+  // barrier, for a memory round trip per chunk.
+  constexpr int EA = (ZG_BK * ZG_BM) / ZG_THREADS, EB = (ZG_BK * ZG_BN) / ZG_THREADS;
+  constexpr int AR = A_RC ? 0 : ZG_THREADS / ZG_BK, AK = A_RC ? ZG_THREADS / ZG_BM : 0;
+  constexpr int BR = B_RC ? 0 : ZG_THREADS / ZG_BK, BK = B_RC ? ZG_THREADS / ZG_BN : 0;
+  const int ar0 = A_RC ? tid % ZG_BM : tid / ZG_BK, ak0 = A_RC ? tid / ZG_BM : tid % ZG_BK;
+  const int br0 = B_RC ? tid % ZG_BN : tid / ZG_BK, bk0 = B_RC ? tid / ZG_BN : tid % ZG_BK;
+  const int Klim = (MODE == ZM_CHI0) ? Kbin : p.K;
+  int bcol[EB], scol = -1;                       // SEG: the columns the thread loads, and scales
+  if (MODE == ZM_SEG) {
+    const int* tc = p.tile_cols + tn * ZG_BN;
 #pragma unroll
-    for (int i = 0; i < (ZG_BK * ZG_BM) / ZG_THREADS; ++i) {
-      const int e = tid + i * ZG_THREADS;
-      int r, kk;
-      if (A_RC) { r = e % ZG_BM; kk = e / ZG_BM; } else { kk = e % ZG_BK; r = e / ZG_BK; }
-      const int k = kbase + kk, m = m0 + r;
-      bool ok = (k < Klim) && (m < Mrows);
-      const double2* src = Aseg;
-      if (ok) {
-        long long kk_off;
-        if (MODE == ZM_CHI0) kk_off = static_cast<long long>(__ldg(kcol + k));
-        else kk_off = k;
-        src = Aseg + m * p.a_rs + kk_off * p.a_ks;
-      }
-      cp_async16(&sm.a[st][kk][r], src, ok);
-    }
-    // B operand
+    for (int i = 0; i < EB; ++i) bcol[i] = tc[br0 + i * BR];
+    if (tid < ZG_BN) scol = tc[tid];
+  }
+  int kidx[EA];                                  // CHI0: zmel columns of the next chunk's entries (A and B alike)
+  auto fetch_cols = [&](int c) {
 #pragma unroll
-    for (int i = 0; i < (ZG_BK * ZG_BN) / ZG_THREADS; ++i) {
-      const int e = tid + i * ZG_THREADS;
-      int r, kk;
-      if (B_RC) { r = e % ZG_BN; kk = e / ZG_BN; } else { kk = e % ZG_BK; r = e / ZG_BK; }
-      const int k = kbase + kk;
-      bool ok = (k < Klim);
-      const double2* src = Bb;
+    for (int i = 0; i < EA; ++i) {
+      const int k = c * ZG_BK + ak0 + i * AK;
+      kidx[i] = (kcol && k < Kbin) ? __ldg(kcol + k) : k;
+    }
+  };
+  if (MODE == ZM_CHI0) fetch_cols(ch0);
+  int lseg = MODE == ZM_SEG ? ch0 / kch_seg : 0, lin = MODE == ZM_SEG ? ch0 - lseg * kch_seg : 0;
+  const double2* segA = Ab;                      // SEG: the segment load_chunk is in
+  const double* segW = nullptr;
+  auto next_seg = [&]() {
+    const ZSeg sg = p.segs[seg0 + lseg];
+    segA = sg.mat;
+    segW = scol >= 0 ? sg.scale + static_cast<long long>(scol) * sg.scale_cs : nullptr;
+  };
+  if (MODE == ZM_SEG && ch0 < ch1) next_seg();
+  auto load_chunk = [&](int c, int st) {         // chunks in ascending order
+    const int kbase = (MODE == ZM_SEG ? lin : c) * ZG_BK;
+    const double2* pa = segA + (m0 + ar0) * p.a_rs;
+    const double2* pb = Bb + (MODE == ZM_SEG ? 0 : (n0 + br0) * p.b_rs);
+    if (MODE != ZM_CHI0) {
+      pa += (kbase + ak0) * p.a_ks;
+      pb += (kbase + bk0) * p.b_ks;
+    }
+#pragma unroll
+    for (int i = 0; i < EA; ++i) {
+      const bool ok = kbase + ak0 + i * AK < Klim && m0 + ar0 + i * AR < Mrows;
+      const double2* src = MODE == ZM_CHI0 ? pa + kidx[i] * p.a_ks : pa + i * (AR * p.a_rs + AK * p.a_ks);
+      cp_async16(&sm.a[st][ak0 + i * AK][ar0 + i * AR], ok ? src : p.A, ok);
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      bool ok = kbase + bk0 + i * BK < Klim;
+      const double2* src;
       if (MODE == ZM_SEG) {
-        const int col = p.tile_cols[tn * ZG_BN + r];
-        ok = ok && (col >= 0);
-        if (ok) src = Bb + static_cast<long long>(col) * p.b_rs + static_cast<long long>(k) * p.b_ks;
+        ok = ok && bcol[i] >= 0;
+        src = pb + bcol[i] * p.b_rs;
       } else {
-        const int n = n0 + r;
-        ok = ok && (n < p.N);
-        if (ok) {
-          long long kk_off = (MODE == ZM_CHI0) ? static_cast<long long>(__ldg(kcol + k)) : k;
-          src = Bb + n * p.b_rs + kk_off * p.b_ks;
-        }
+        ok = ok && n0 + br0 + i * BR < p.N;
+        src = MODE == ZM_CHI0 ? pb + kidx[i] * p.b_ks : pb + i * (BR * p.b_rs + BK * p.b_ks);
       }
-      cp_async16(&sm.b[st][kk][r], src, ok);
+      cp_async16(&sm.b[st][bk0 + i * BK][br0 + i * BR], ok ? src : p.B, ok);
     }
     if (MODE == ZM_CHI0) {
-      if (tid < ZG_BK) {
-        const int k = kbase + tid;
-        sm.sk[st][tid] = (k < Kbin) ? __ldg(kw + k) : 0.0;
-      }
+      if (tid < ZG_BK) cp_async8(&sm.sk[st][tid], kbase + tid < Kbin ? kw + kbase + tid : kw, kbase + tid < Kbin);
+      fetch_cols(c + 1);
     }
     if (MODE == ZM_SEG) {
-      if (tid < ZG_BN) {
-        const int col = p.tile_cols[tn * ZG_BN + tid];
-        sm.sn[st][tid] = (col >= 0) ? __ldg(sscale + static_cast<long long>(col) * scs) : 0.0;
+      if (tid < ZG_BN) cp_async8(&sm.sn[st][tid], scol >= 0 ? segW : reinterpret_cast<const double*>(p.B), scol >= 0);
+      if (++lin == kch_seg) {
+        lin = 0;
+        ++lseg;
+        if (lseg < nseg) next_seg();
       }
     }
   };
 
-  double accr[2][4][4], acci[2][4][4];       // [m16 block][n8 block][fragment element]
+  double accr[ZG_NI][ZG_NJ][4], acci[ZG_NI][ZG_NJ][4];       // [m16 block][n8 block][fragment element]
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < ZG_NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) accr[i][j][e] = acci[i][j][e] = 0.0;
+
+  // The warp's fragments that hold output: m16 blocks i < ni and n8 blocks j < nj.  A ragged edge tile, and
+  // the upper half of a Hermitian diagonal tile, issue no DMMA for fragments nobody reads.
+  int ncol_tile = p.N - n0;
+  if (MODE == ZM_SEG) {                         // -1 columns fill the end of a tile
+    const int* tc = p.tile_cols + tn * ZG_BN;
+    const int v = (tc[lane] >= 0) + (tc[lane + 32] >= 0);
+    ncol_tile = __reduce_add_sync(0xffffffffu, v);
+  }
+  const int ni = min(2, max(0, (Mrows - m0 - wm * 32 + 15) / 16));
+  int nj = ni > 0 ? min(ZG_NJ, max(0, (ncol_tile - wn * (8 * ZG_NJ) + 7) / 8)) : 0;
+  if (MODE == ZM_CHI0 && p.herm && tm == tn && wm * 32 + 31 < wn * (8 * ZG_NJ)) nj = 0;   // mirrored from the quadrant below
 
   const int nloc = ch1 - ch0;
 #pragma unroll
@@ -215,54 +251,125 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
     if (s < nloc) load_chunk(ch0 + s, s);
     cp_async_commit();
   }
+  if (MODE == ZM_GEMM && p.acc_c) {
+    // C is read while the first operand chunks are in flight, not after the last product: the rank-32
+    // updates of the inverses are two chunks long
+#pragma unroll
+    for (int i = 0; i < ZG_NI; ++i)
+#pragma unroll
+      for (int j = 0; j < ZG_NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int row = m0 + wm * 32 + i * 16 + (e >> 1) * 8 + g;
+          const int col = n0 + wn * (8 * ZG_NJ) + j * 8 + 2 * t + (e & 1);
+          if (row < p.M && col < p.N) {
+            const double2 o = Cb[row + col * p.ldc];
+            accr[i][j][e] = p.alpha.x * o.x;
+            acci[i][j][e] = p.alpha.x * o.y;
+          }
+        }
+  }
   for (int c = 0; c < nloc; ++c) {
     cp_async_wait<ZG_STAGES - 2>();
     __syncthreads();
     const int st = c % ZG_STAGES;
+    const int cg = ch0 + c;                       // K elements left from this chunk on: an empty half is skipped
+    const int krem = MODE == ZM_CHI0 ? Kbin - cg * ZG_BK
+                                     : p.K - (MODE == ZM_SEG ? cg % kch_seg : cg) * ZG_BK;
+    auto mult = [&](auto full_tile) {
+      constexpr bool FULL = decltype(full_tile)::value;
 #pragma unroll
-    for (int k8 = 0; k8 < ZG_BK / 8; ++k8) {
-      const int ka = k8 * 8 + t, kb = ka + 4;       // the lane's two k of the step
-      double ar[2][4], ai[2][4], nai[2][4], br[4][2], bi[4][2];
+      for (int k8 = 0; k8 < ZG_BK / 8; ++k8) {
+        if (k8 * 8 >= krem) break;
+        const int ka = k8 * 8 + t, kb = ka + 4;       // the lane's two k of the step
+        double ar[2][4], ai[2][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int r0 = wm * 32 + i * 16 + g;
-        const double2 v[4] = {sm.a[st][ka][r0], sm.a[st][ka][r0 + 8], sm.a[st][kb][r0], sm.a[st][kb][r0 + 8]};
+        for (int i = 0; i < 2; ++i) {
+          const int r0 = wm * 32 + i * 16 + g;
+          const double2 v[4] = {sm.a[st][ka][r0], sm.a[st][ka][r0 + 8], sm.a[st][kb][r0], sm.a[st][kb][r0 + 8]};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          ar[i][e] = v[e].x;
-          ai[i][e] = p.a_conj ? -v[e].y : v[e].y;
-          nai[i][e] = -ai[i][e];
+          for (int e = 0; e < 4; ++e) {
+            ar[i][e] = v[e].x;
+            ai[i][e] = p.a_conj ? -v[e].y : v[e].y;
+          }
+        }
+        double ska = 1.0, skb = 1.0;
+        if (MODE == ZM_CHI0) { ska = sm.sk[st][ka]; skb = sm.sk[st][kb]; }
+#pragma unroll
+        for (int j = 0; j < ZG_NJ; ++j) {
+          if (!FULL && j >= nj) break;
+          const int nn = wn * (8 * ZG_NJ) + j * 8 + g;
+          const double2 va = sm.b[st][ka][nn], vb = sm.b[st][kb][nn];
+          double sa = ska, sb = skb;
+          if (MODE == ZM_SEG) sa = sb = sm.sn[st][nn];
+          const double bra = va.x * sa, brb = vb.x * sb;
+          const double bia = (p.b_conj ? -va.y : va.y) * sa, bib = (p.b_conj ? -vb.y : vb.y) * sb;
+          // the two products of an accumulator stand apart: issued back to back the second waits for the first
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (FULL || i < ni) {
+              dmma16(accr[i][j], ar[i], bra, brb);
+              dmma16(acci[i][j], ar[i], bia, bib);
+            }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (FULL || i < ni) {
+              dmma16(accr[i][j], ai[i], -bia, -bib);
+              dmma16(acci[i][j], ai[i], bra, brb);
+            }
         }
       }
-      double ska = 1.0, skb = 1.0;
-      if (MODE == ZM_CHI0) { ska = sm.sk[st][ka]; skb = sm.sk[st][kb]; }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int nn = wn * 32 + j * 8 + g;
-        const double2 va = sm.b[st][ka][nn], vb = sm.b[st][kb][nn];
-        double sa = ska, sb = skb;
-        if (MODE == ZM_SEG) sa = sb = sm.sn[st][nn];
-        br[j][0] = va.x * sa;
-        br[j][1] = vb.x * sb;
-        bi[j][0] = (p.b_conj ? -va.y : va.y) * sa;
-        bi[j][1] = (p.b_conj ? -vb.y : vb.y) * sb;
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dmma16(accr[i][j], ar[i], br[j][0], br[j][1]);
-          dmma16(accr[i][j], nai[i], bi[j][0], bi[j][1]);
-          dmma16(acci[i][j], ar[i], bi[j][0], bi[j][1]);
-          dmma16(acci[i][j], ai[i], br[j][0], br[j][1]);
-        }
-    }
+    };
+    if (ni == ZG_NI && nj == ZG_NJ) mult(std::true_type());
+    else if (nj > 0) mult(std::false_type());
     const int cn = c + ZG_STAGES - 1;
     if (cn < nloc) load_chunk(ch0 + cn, cn % ZG_STAGES);
     cp_async_commit();
   }
   cp_async_wait<0>();
-  if (nloc <= 0 && (MODE != ZM_GEMM || p.splitk > 1) && MODE != ZM_SEG) return;
+  if (nloc <= 0 && (MODE == ZM_CHI0 || p.splitk > 1)) return;
+
+  if (MODE == ZM_CHI0) {
+    // The tile leaves through shared memory (the stage buffers are free): its columns, and with herm the
+    // columns of its mirror image, as whole runs of 64 rows.  Bins of a few pairs are bound by this
+    // read-modify-write; straight from the fragments the mirror wrote 16-byte pieces.
+    double2 (*tile)[ZG_PA] = reinterpret_cast<double2 (*)[ZG_PA]>(zg_smem_raw);     // [column][row]
+    static_assert(sizeof(double2) * ZG_BN * ZG_PA <= sizeof(ZSmem), "the tile fits the stage buffers");
+    __syncthreads();
+    if (nj > 0) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < ZG_NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int rl = wm * 32 + i * 16 + (e >> 1) * 8 + g, cl = wn * (8 * ZG_NJ) + j * 8 + 2 * t + (e & 1);
+            const double2 v = make_double2(accr[i][j][e], acci[i][j][e]);
+            tile[cl][rl] = v;
+            if (p.herm && tm == tn && wm == 1 && wn < 2) tile[rl][cl] = make_double2(v.x, -v.y);
+          }
+    }
+    __syncthreads();
+    auto store = [&](int r0, int c0, bool mirror) {
+      const int r = tid % ZG_BM, row = r0 + r;
+      if (row >= (mirror ? p.N : p.M)) return;
+      const int cend = min(ZG_BN, (mirror ? p.M : p.N) - c0);
+#pragma unroll 4
+      for (int cl = tid / ZG_BM; cl < cend; cl += ZG_THREADS / ZG_BM) {
+        double2 v = mirror ? tile[r][cl] : tile[cl][r];
+        if (mirror) v.y = -v.y;
+        double2* dst = Cb + row + static_cast<long long>(c0 + cl) * p.ldc;
+        if (p.splitk > 1) {
+          atomicAdd(&dst->x, v.x); atomicAdd(&dst->y, v.y);
+        } else {
+          double2 o = *dst; o.x += v.x; o.y += v.y; *dst = o;
+        }
+      }
+    };
+    store(m0, n0, false);
+    if (p.herm && tm != tn) store(n0, m0, true);     // rcxq(col, row) += conj(acc(row, col))
+    return;
+  }
 
   // ---- epilogue ----
 #pragma unroll
@@ -271,10 +378,10 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
     for (int h = 0; h < 2; ++h) {
     const int row = m0 + wm * 32 + i * 16 + h * 8 + g;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < ZG_NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int cl = wn * 32 + j * 8 + 2 * t + e;
+        const int cl = wn * (8 * ZG_NJ) + j * 8 + 2 * t + e;
         double vr = accr[i][j][2 * h + e], vi = acci[i][j][2 * h + e];
         if (MODE == ZM_GEMM) {
           const int col = n0 + cl;
@@ -285,36 +392,19 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
           if (p.splitk > 1) {
             atomicAdd(&dst->x, r2);
             atomicAdd(&dst->y, i2);
-          } else if (p.beta_zero) {
+          } else if (p.beta_zero || p.acc_c) {
             *dst = make_double2(r2, i2);
           } else {
             const double2 o = *dst;
             *dst = make_double2(r2 + p.beta.x * o.x - p.beta.y * o.y,
                                 i2 + p.beta.x * o.y + p.beta.y * o.x);
           }
-        } else if (MODE == ZM_CHI0) {
-          const int col = n0 + cl;
-          if (row >= p.M || col >= p.N) continue;
-          double2* dst = Cb + row + col * p.ldc;
-          if (p.splitk > 1) {
-            atomicAdd(&dst->x, vr); atomicAdd(&dst->y, vi);
-          } else {
-            double2 o = *dst; o.x += vr; o.y += vi; *dst = o;
-          }
-          if (p.herm && tm != tn) {   // rcxq(col,row) += conj(acc(row,col))
-            double2* d2 = Cb + col + static_cast<long long>(row) * p.ldc;
-            if (p.splitk > 1) {
-              atomicAdd(&d2->x, vr); atomicAdd(&d2->y, -vi);
-            } else {
-              double2 o = *d2; o.x += vr; o.y -= vi; *d2 = o;
-            }
-          }
         } else {
           const int col = p.tile_cols[tn * ZG_BN + cl];
           if (row >= p.M || col < 0) continue;
           double2* dst = Cb + row + static_cast<long long>(col) * p.ldc;
-          if (p.beta_zero) *dst = make_double2(vr, vi);
-          else { double2 o = *dst; o.x += vr; o.y += vi; *dst = o; }
+          if (p.splitk > 1) { atomicAdd(&dst->x, vr); atomicAdd(&dst->y, vi); }
+          else *dst = make_double2(vr, vi);
         }
       }
   }
@@ -329,7 +419,10 @@ int zgemm_chi0_launch(ZParams p, int nbins, int herm, int splitk, cudaStream_t s
 // C(0:n, 0:n) += A^H B for complex A, B of K x n (column-major), n <= 64, any K (FP64 atomics)
 int zgemm_hn_thin(int n, long long K, const double2* A, long long lda, const double2* B, long long ldb, double2* C,
                   long long ldc, cudaStream_t s);
-int zgemm_seg_launch(ZParams p, int ncol_tiles, cudaStream_t s);
+// C (ldc x p.N, contiguous columns) is overwritten; mean_nseg: the tiles' mean segment count
+int zgemm_seg_launch(ZParams p, int ncol_tiles, int mean_nseg, cudaStream_t s);
+// K splits of a launch of `ctas` equal tiles of nch K chunks (one split when nch is short)
+int zgemm_splitk(long long ctas, int nch);
 // Batched inverses (wv.cu: Hermitian positive definite; zminv_piv.cu: general, partial pivoting).
 int zminv_hpd_batched(double2* A, int n, long long lda, long long a_bs, int nbatch, cudaStream_t s);
 int zminv_general_batched(double2* A, int n, long long lda, long long a_bs, int nbatch, cudaStream_t s);
