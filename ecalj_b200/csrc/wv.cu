@@ -17,83 +17,107 @@ namespace qsgw {
 
 constexpr int GJ_NB = 32;
 
-__global__ void gj_panel_kernel(double2* __restrict__ A, int n, long long lda, long long a_bs,
-                                double2* __restrict__ Rb, double2* __restrict__ Qb, int c0, int w,
-                                int* __restrict__ flag) {
-  __shared__ double2 P[GJ_NB][GJ_NB + 1];
-  const int b = blockIdx.y;
-  double2* Ab = A + b * a_bs;
+// One block per 64 rows and matrix; every block inverts the w x w pivot block for itself (the serial
+// chain of w steps bounds this kernel, not its arithmetic).  Thread (i, jg) keeps the elements
+// (i, jg + 8 u) in registers; a step needs only pivot row and column, passed through one of two shared
+// buffers, so it costs one barrier and one reciprocal.  The block then forms its 64 rows of R P^-1 from
+// shared tiles.  24 matrices of 600: 40 us a panel (102 us with the pivot block swept in shared memory, two
+// barriers and two divisions a step, and R read from global memory once per product).
+constexpr int GJ_ROWS = 64;
+__global__ void __launch_bounds__(256) gj_panel_kernel(double2* __restrict__ A, int n, long long lda, long long a_bs,
+                                                       double2* __restrict__ Rb, double2* __restrict__ Qb, int c0,
+                                                       int w, int* __restrict__ flag) {
+  __shared__ double2 P[GJ_NB][GJ_NB];                 // P^-1, [i][j]
+  __shared__ double2 R[GJ_NB][GJ_ROWS];               // the block's rows of the panel, [l][row]
+  double2 (*rowk)[GJ_NB] = P, (*colk)[GJ_NB] = P + 2; // the step buffers [2][32], until P^-1 is stored
+  const int b = blockIdx.y, r0 = blockIdx.x * GJ_ROWS;
+  const double2* Ab = A + b * a_bs;
   double2* Rbb = Rb + static_cast<long long>(b) * n * GJ_NB;
   double2* Qbb = Qb + static_cast<long long>(b) * n * GJ_NB;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < GJ_NB * GJ_NB; e += blockDim.x) {
-    const int i = e % GJ_NB, j = e / GJ_NB;
-    P[i][j] = (i < w && j < w) ? Ab[(c0 + i) + (c0 + j) * lda] : make_double2(0.0, 0.0);
+  const int tid = threadIdx.x, i = tid & 31, jg = tid >> 5;
+  double2 o[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = jg + 8 * u;
+    o[u] = (i < w && j < w) ? Ab[(c0 + i) + (c0 + j) * lda] : make_double2(0.0, 0.0);
+    if (i == 0) rowk[0][j] = o[u];
+    if (j == 0) colk[0][i] = o[u];
+  }
+#pragma unroll
+  for (int e = 0; e < GJ_NB * GJ_ROWS / 256; ++e) {
+    const int rr = tid & (GJ_ROWS - 1), l = (tid >> 6) + 4 * e;
+    R[l][rr] = (r0 + rr < n && l < w) ? Ab[r0 + rr + (c0 + l) * lda] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  // in-place exchange inverse of the w x w pivot block
   bool bad = false;
   for (int k = 0; k < w; ++k) {
-    const double2 pk = P[k][k];
+    const int s = k & 1;
+    const double2 pk = rowk[s][k], ci = colk[s][i];
     const double den = pk.x * pk.x + pk.y * pk.y;
     if (!(den > 1e-300) || !isfinite(den)) bad = true;
-    const double2 inv = make_double2(pk.x / den, -pk.y / den);
-    double2 nv[GJ_NB * GJ_NB / 128];
-    int cnt = 0;
-    for (int e = tid; e < w * w; e += blockDim.x, ++cnt) {
-      const int i = e % w, j = e / w;
-      double2 r;
-      if (i == k && j == k) {
-        r = inv;
-      } else if (i == k) {            // -P_kj / P_kk
-        const double2 a = P[k][j];
-        r = make_double2(-(a.x * inv.x - a.y * inv.y), -(a.x * inv.y + a.y * inv.x));
-      } else if (j == k) {            //  P_ik / P_kk
-        const double2 a = P[i][k];
-        r = make_double2(a.x * inv.x - a.y * inv.y, a.x * inv.y + a.y * inv.x);
-      } else {                        //  P_ij - P_ik P_kj / P_kk
-        const double2 a = P[i][k], c = P[k][j];
-        const double2 t = make_double2(a.x * inv.x - a.y * inv.y, a.x * inv.y + a.y * inv.x);
-        const double2 o = P[i][j];
-        r = make_double2(o.x - (t.x * c.x - t.y * c.y), o.y - (t.x * c.y + t.y * c.x));
+    const double rden = 1.0 / den;
+    const double2 inv = make_double2(pk.x * rden, -pk.y * rden);
+    const double2 t = make_double2(ci.x * inv.x - ci.y * inv.y, ci.x * inv.y + ci.y * inv.x);   // P_ik / P_kk
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = jg + 8 * u;
+      const double2 a = rowk[s][j];
+      if (i == k) {                                     // 1 / P_kk, -P_kj / P_kk
+        o[u] = j == k ? inv : make_double2(-(a.x * inv.x - a.y * inv.y), -(a.x * inv.y + a.y * inv.x));
+      } else if (j == k) {
+        o[u] = t;
+      } else {                                          // P_ij - P_ik P_kj / P_kk
+        o[u].x -= t.x * a.x - t.y * a.y;
+        o[u].y -= t.x * a.y + t.y * a.x;
       }
-      nv[cnt] = r;
+      if (i == k + 1) rowk[s ^ 1][j] = o[u];
+      if (j == k + 1) colk[s ^ 1][i] = o[u];
     }
-    __syncthreads();
-    cnt = 0;
-    for (int e = tid; e < w * w; e += blockDim.x, ++cnt) P[e % w][e / w] = nv[cnt];
     __syncthreads();
   }
   if (bad && tid == 0) atomicExch(flag, 1);
-  // Rb rows of this CTA's row block
-  const int r0 = blockIdx.x * 64;
-  for (int e = tid; e < 64 * GJ_NB; e += blockDim.x) {
-    const int ii = e % 64, j = e / 64;
-    const int row = r0 + ii;
-    if (row >= n || j >= w) continue;
-    double2 acc;
-    if (row >= c0 && row < c0 + w) {
-      acc = P[row - c0][j];
-      if (row - c0 == j) acc.x += 1.0;
-    } else {
-      acc = make_double2(0.0, 0.0);
-      for (int l = 0; l < w; ++l) {
-        const double2 a = Ab[row + (c0 + l) * lda];
-        const double2 c = P[l][j];
-        acc.x += a.x * c.x - a.y * c.y;
-        acc.y += a.x * c.y + a.y * c.x;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) P[i][jg + 8 * u] = o[u];
+  __syncthreads();
+  // Rb rows of this block: thread = one row, eight columns
+  {
+    const int rr = tid & (GJ_ROWS - 1), j0 = (tid >> 6) * 8, row = r0 + rr;
+    if (row < n) {
+      const bool piv = row >= c0 && row < c0 + w;
+      double2 acc[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = make_double2(0.0, 0.0);
+      if (piv) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc[q] = P[row - c0][j0 + q];
+          if (row - c0 == j0 + q) acc[q].x += 1.0;
+        }
+      } else {
+#pragma unroll 4
+        for (int l = 0; l < GJ_NB; ++l) {               // rows l >= w of P and columns l >= w of R are zero
+          const double2 a = R[l][rr];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const double2 c = P[l][j0 + q];
+            acc[q].x += a.x * c.x - a.y * c.y;
+            acc[q].y += a.x * c.y + a.y * c.x;
+          }
+        }
       }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (j0 + q < w) Rbb[row + static_cast<long long>(j0 + q) * n] = acc[q];
     }
-    Rbb[row + static_cast<long long>(j) * n] = acc;
   }
   // Qb columns of the same index range
-  for (int e = tid; e < 64 * GJ_NB; e += blockDim.x) {
-    const int l = e % GJ_NB, jj = e / GJ_NB;
-    const int col = r0 + jj;
-    if (col >= n || l >= w) continue;
-    double2 v = Ab[(c0 + l) + static_cast<long long>(col) * lda];
-    if (col - c0 == l) v.x -= 1.0;
-    Qbb[l + static_cast<long long>(col) * GJ_NB] = v;
+#pragma unroll
+  for (int e = 0; e < GJ_NB * GJ_ROWS / 256; ++e) {
+    const int col = r0 + jg + 8 * e;
+    if (col >= n || i >= w) continue;
+    double2 v = Ab[(c0 + i) + static_cast<long long>(col) * lda];
+    if (col - c0 == i) v.x -= 1.0;
+    Qbb[i + static_cast<long long>(col) * GJ_NB] = v;
   }
 }
 
@@ -106,7 +130,7 @@ int zminv_hpd_batched(double2* A, int n, long long lda, long long a_bs, int nbat
   if (rc) return rc;
   rc = g_gj_q.ensure(pbytes);
   if (rc) return rc;
-  const dim3 pg((n + 63) / 64, nbatch);
+  const dim3 pg((n + GJ_ROWS - 1) / GJ_ROWS, nbatch);
   QSGW_CUDA(cudaMemsetAsync(ctx().d_flags, 0, sizeof(int), s));
   for (int c0 = 0; c0 < n; c0 += GJ_NB) {
     const int w = std::min(GJ_NB, n - c0);
@@ -127,7 +151,7 @@ int zminv_hpd_batched(double2* A, int n, long long lda, long long a_bs, int nbat
 int zminv_hpd_batched_explicit(double2* A, int n, long long lda, long long a_bs, int nbatch, double2* rb,
                                double2* qb, int* flag, cudaStream_t s) {
   if (n <= 0 || nbatch <= 0) return QSGW_OK;
-  const dim3 pg((n + 63) / 64, nbatch);
+  const dim3 pg((n + GJ_ROWS - 1) / GJ_ROWS, nbatch);
   for (int c0 = 0; c0 < n; c0 += GJ_NB) {
     const int w = std::min(GJ_NB, n - c0);
     gj_panel_kernel<<<pg, 256, 0, s>>>(A, n, lda, a_bs, rb, qb, c0, w, flag);
@@ -232,17 +256,18 @@ static int wvi_device(double2* zxqi, int ngb, int niw, int nspin, const double* 
   const long long en = static_cast<long long>(n) * n;
   rc = g_wv_e.ensure(std::max<long long>(en, 1) * niw * sizeof(double2));
   if (rc) return rc;
+  const double2* einv = g_wv_e.as<double2>();
   if (n > 0) {
     eps_build_kernel<<<grid_for(en * niw), 256, 0, s>>>(g_wv_e.as<double2>(), chi, g_wv_v.as<double>(),
                                                         ngb, ix, ngb, nn, niw);
     count_launch();
     QSGW_LAUNCH_CHECK("eps_build_kernel");
-    rc = general ? zminv_general_batched(g_wv_e.as<double2>(), n, n, en, niw, s)    // :139
+    rc = general ? zminv_general_batched(g_wv_e.as<double2>(), n, n, en, niw, s, &einv)    // :139
                  : zminv_hpd_batched(g_wv_e.as<double2>(), n, n, en, niw, s);       // :350
     if (rc) return rc;
   }
   wc_build_kernel<<<grid_for(static_cast<long long>(ldzw) * ldzw * niw), 256, 0, s>>>(
-      zw, g_wv_e.as<double2>(), g_wv_v.as<double>(), ngb, ix, ldzw, niw);
+      zw, einv, g_wv_v.as<double>(), ngb, ix, ldzw, niw);
   count_launch();
   QSGW_LAUNCH_CHECK("wc_build_kernel");
   if (is_wc_m && iq != 1) {   // W_M = m2e W_E m2e^H (:363-370)

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
   }
 }
 
-// Host launch helpers (defined in zgemm_f64.cu).
+// Host launch helpers (defined in zgemm_f64.cu).  op: 0 'N', 1 'T', 2 'C', 3 conjugated without transposing.
 int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
               const double2* A, long long lda, long long a_bs,
               const double2* B, long long ldb, long long b_bs, double2 beta,
@@ -425,6 +425,9 @@ int zgemm_seg_launch(ZParams p, int ncol_tiles, int mean_nseg, cudaStream_t s);
 int zgemm_splitk(long long ctas, int nch);
 // Batched inverses (wv.cu: Hermitian positive definite; zminv_piv.cu: general, partial pivoting).
 int zminv_hpd_batched(double2* A, int n, long long lda, long long a_bs, int nbatch, cudaStream_t s);
-int zminv_general_batched(double2* A, int n, long long lda, long long a_bs, int nbatch, cudaStream_t s);
+// result (may be null): receives the inverses' scratch copy (ld n, stride n*n), A is then left undefined;
+// without it the inverses are copied back into A.
+int zminv_general_batched(double2* A, int n, long long lda, long long a_bs, int nbatch, cudaStream_t s,
+                          const double2** result = nullptr);
 
 }  // namespace qsgw
