@@ -190,10 +190,10 @@ int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
   if (m <= 0 || n <= 0 || nbatch <= 0) return QSGW_OK;
   ZParams p{};
   p.M = m; p.N = n; p.K = k;
-  p.A = A; p.a_bs = a_bs; p.a_conj = (opa == 2);
-  if (opa == 0) { p.a_rs = 1; p.a_ks = lda; } else { p.a_rs = lda; p.a_ks = 1; }
-  p.B = B; p.b_bs = b_bs; p.b_conj = (opb == 2);
-  if (opb == 0) { p.b_rs = ldb; p.b_ks = 1; } else { p.b_rs = 1; p.b_ks = ldb; }
+  p.A = A; p.a_bs = a_bs; p.a_conj = (opa >= 2);
+  if (opa == 0 || opa == 3) { p.a_rs = 1; p.a_ks = lda; } else { p.a_rs = lda; p.a_ks = 1; }
+  p.B = B; p.b_bs = b_bs; p.b_conj = (opb >= 2);
+  if (opb == 0 || opb == 3) { p.b_rs = ldb; p.b_ks = 1; } else { p.b_rs = 1; p.b_ks = ldb; }
   p.C = C; p.ldc = ldc; p.c_bs = c_bs;
   p.alpha = alpha; p.beta = beta;
   p.beta_zero = (beta.x == 0.0 && beta.y == 0.0);
@@ -222,7 +222,7 @@ int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
     QSGW_LAUNCH_CHECK("zscale_kernel");
   }
   dim3 grid(static_cast<unsigned>(p.ntm * p.ntn), nbatch, splitk);
-  const bool arc = (opa == 0), brc = (opb != 0);
+  const bool arc = (opa == 0 || opa == 3), brc = (opb == 1 || opb == 2);
   if (arc && brc) return launch_kernel<ZM_GEMM, true, true>(p, grid, s);
   if (arc && !brc) return launch_kernel<ZM_GEMM, true, false>(p, grid, s);
   if (!arc && brc) return launch_kernel<ZM_GEMM, false, true>(p, grid, s);

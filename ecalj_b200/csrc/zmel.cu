@@ -4,11 +4,10 @@
 //
 // For every atom the reference runs two batched ZGEMMs with tiny K (the
 // atom's valence channels, nv ~ 10-30): ppbvphiq = ppb_v^T cphiq and
-// zmelt = phase cphim^H ppbvphiq, each a separate library call per atom.
-// Here one launch covers all atoms: a CTA owns (atom, 16 target columns itp,
-// 16 middle states it) and loops over the atom's product functions i, with
-// ppb(:,:,i), the cphiq block and T = ppb^T cphiq staged in shared memory;
-// consecutive threads write consecutive product-basis rows of zmelt.
+// zmelt = phase cphim^H ppbvphiq.  Here one launch forms T = ppb^T cphiq of
+// every atom and product function (and the core states' rows, which need
+// nothing else), then one batched product per atom on the DMMA engine
+// contracts it with cphim for all target columns and writes the atom's rows.
 #include <vector>
 #include "zgemm_f64.cuh"
 #include "ozaki_i8.cuh"
@@ -19,100 +18,63 @@ struct ZmelAtomDev {
   const double* ppb;      // (nlnm, nlnm, mdim) real, column-major
   int nlnm, nc, nv, ias, ics, ims, mdim, ncore;
   double ph_re, ph_im;    // exp(-i 2 pi k . tau)
+  long long toff;         // the atom's T in the scratch
 };
 
-constexpr int ZM_T = 16;          // itp and it block
-constexpr int ZM_NVMAX = 96;      // valence channels per atom handled in shared memory
+constexpr int ZM_NVMAX = 96;      // valence channels per atom
+constexpr int ZM_TQ = 16;         // target columns per block of the first product
 
-__global__ void zmel_mt_kernel(double2* __restrict__ zt, int nbloch, int nm1, int nmtot, int nctot, int ntp0,
-                               int nm1v, int nm2v, int nm1c, int nm2c, const double2* __restrict__ cphim,
-                               int ldm, const double2* __restrict__ cphiq, int ldq,
-                               const ZmelAtomDev* __restrict__ atoms, int nvmax) {
-  // dynamic shared memory, sized for the largest atom:
-  //   sq, sT, sm_ : (nvmax x 16) complex   cphiq block, T = ppb^T cphiq, conj(cphim) block
-  //   sp          : nvmax^2 doubles        ppb valence block of one product function
+// T(itp, i, a) = sum_b ppb(nc+b, nc+a, i) cphiq(ias+b, itp) (m_zmel.f90:358), a fastest, and the core rows
+// zmelt(ims+i, it, itp) = phase sum_b ppb(nc+b, it-ics, i) cphiq(b, itp) (:383).  One block per (product
+// function of the atom, ZM_TQ target columns): the function's real nv x (nv + cores) block and the cphiq
+// columns are staged once, each thread forms whole sums.  The kernel this replaces kept a block on 16 x 16
+// outputs through all product functions (three barriers each, 16-byte writes a row apart): 791 us for two
+// atoms of 25 channels and 150 functions at 200 x 40 states, now 14 us and 67 us of DMMA products.
+__global__ void __launch_bounds__(256) zmel_ppb_kernel(double2* __restrict__ T, double2* __restrict__ zt, int nbloch,
+                                                       int nm1, int nmtot, int nctot, int ntp0, int nm1c, int nm2c,
+                                                       const double2* __restrict__ cphiq, int ldq,
+                                                       const ZmelAtomDev* __restrict__ atoms, int nvmax) {
   extern __shared__ double2 zm_smem[];
-  double2 (*sq)[ZM_T] = reinterpret_cast<double2 (*)[ZM_T]>(zm_smem);
-  double2 (*sT)[ZM_T] = reinterpret_cast<double2 (*)[ZM_T]>(zm_smem + nvmax * ZM_T);
-  double2 (*sm_)[ZM_T] = reinterpret_cast<double2 (*)[ZM_T]>(zm_smem + 2 * nvmax * ZM_T);
-  double* sp = reinterpret_cast<double*>(zm_smem + 3 * nvmax * ZM_T);
-  const ZmelAtomDev at = atoms[blockIdx.x];
-  const int itp0 = blockIdx.y * ZM_T;
-  const int it0 = blockIdx.z * ZM_T;                  // index into [nm1, nm2] (0-based)
-  const int tid = threadIdx.x;
-  const int nv = at.nv, nc = at.nc;
-  const double2 ph = make_double2(at.ph_re, at.ph_im);
-  // stage cphiq(ias:ias+nv-1, itp0:itp0+15)
-  for (int e = tid; e < nv * ZM_T; e += blockDim.x) {
+  double2* sq = zm_smem;                                            // [ZM_TQ][nv]: cphiq columns
+  double* sp = reinterpret_cast<double*>(zm_smem + nvmax * ZM_TQ);  // [nv][nv + 1]: the valence block of ppb(:, :, i)
+  const ZmelAtomDev at = atoms[blockIdx.z];
+  const int i = blockIdx.x, itp0 = blockIdx.y * ZM_TQ, nq = min(ZM_TQ, ntp0 - itp0);
+  if (i >= at.mdim) return;
+  const int nv = at.nv, tid = threadIdx.x;
+  // columns of ppb needed: the valence ones, then the core states of this atom inside nm1c..nm2c
+  const int ncorec = nctot > 0 ? at.ncore : 0;
+  const int it_lo = max(nm1c, at.ics + 1), it_hi = min(nm2c, at.ics + ncorec);
+  const int ncore = max(0, it_hi - it_lo + 1), ncol = nv + ncore;
+  const double* pi = at.ppb + static_cast<long long>(i) * at.nlnm * at.nlnm;
+  for (int e = tid; e < nv * nq; e += 256) {
     const int b = e % nv, j = e / nv;
-    const int itp = itp0 + j;
-    sq[b][j] = (itp < ntp0) ? cphiq[(at.ias - 1 + b) + static_cast<long long>(itp) * ldq] : make_double2(0.0, 0.0);
+    sq[b + j * nv] = cphiq[(at.ias - 1 + b) + static_cast<long long>(itp0 + j) * ldq];
   }
-  // stage conj(cphim) for valence middle states of this block
-  for (int e = tid; e < nv * ZM_T; e += blockDim.x) {
-    const int a = e % nv, j = e / nv;
-    const int it = nm1 + it0 + j;
-    double2 v = make_double2(0.0, 0.0);
-    if (it0 + j < nmtot && it >= nm1v && it <= nm2v) {
-      v = cphim[(at.ias - 1 + a) + static_cast<long long>(it - nm1v) * ldm];
-      v.y = -v.y;
-    }
-    sm_[a][j] = v;
+  for (int e = tid; e < nv * nv; e += 256) {
+    const int b = e % nv, a = e / nv;
+    sp[b + a * (nv + 1)] = pi[at.nc + b + static_cast<long long>(at.nc + a) * at.nlnm];
   }
   __syncthreads();
-  for (int i = 0; i < at.mdim; ++i) {
-    // ppb(nc+1:nc+nv, nc+1:nc+nv, i) valence block
-    for (int e = tid; e < nv * nv; e += blockDim.x) {
-      const int b = e % nv, a = e / nv;
-      sp[e] = at.ppb[(nc + b) + static_cast<long long>(nc + a) * at.nlnm + static_cast<long long>(i) * at.nlnm * at.nlnm];
+  double2* Ta = T + at.toff;
+  for (int e = tid; e < ncol * nq; e += 256) {
+    const int a = e % ncol, j = e / ncol;
+    double2 acc = make_double2(0.0, 0.0);
+    const double* wa = a < nv ? sp + a * (nv + 1)
+                              : pi + at.nc + static_cast<long long>(it_lo + (a - nv) - at.ics - 1) * at.nlnm;
+    for (int b = 0; b < nv; ++b) {
+      const double w = wa[b];
+      const double2 q = sq[b + j * nv];
+      acc.x += w * q.x;
+      acc.y += w * q.y;
     }
-    __syncthreads();
-    for (int e = tid; e < nv * ZM_T; e += blockDim.x) {   // T(a, itp) (m_zmel.f90:358)
-      const int a = e % nv, j = e / nv;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int b = 0; b < nv; ++b) {
-        const double w = sp[b + a * nv];
-        acc.x += w * sq[b][j].x;
-        acc.y += w * sq[b][j].y;
-      }
-      sT[a][j] = acc;
+    if (a < nv) {
+      Ta[a + static_cast<long long>(nv) * (i + static_cast<long long>(at.mdim) * (itp0 + j))] = acc;
+    } else {
+      const int itl = it_lo + (a - nv) - nm1;
+      zt[(at.ims - 1 + i) + static_cast<long long>(itl) * nbloch +
+         static_cast<long long>(itp0 + j) * nbloch * nmtot] =
+          make_double2(at.ph_re * acc.x - at.ph_im * acc.y, at.ph_re * acc.y + at.ph_im * acc.x);
     }
-    __syncthreads();
-    // zmelt(ims+i-1, it, itp) for this block (valence :365, core :383)
-    for (int e = tid; e < ZM_T * ZM_T; e += blockDim.x) {
-      const int jt = e % ZM_T, jp = e / ZM_T;
-      const int itl = it0 + jt, itp = itp0 + jp;
-      if (itl >= nmtot || itp >= ntp0) continue;
-      const int it = nm1 + itl;
-      double2 acc = make_double2(0.0, 0.0);
-      bool write = false;
-      if (it >= nm1v && it <= nm2v) {
-        for (int a = 0; a < nv; ++a) {
-          const double2 m = sm_[a][jt], t = sT[a][jp];
-          acc.x += m.x * t.x - m.y * t.y;
-          acc.y += m.x * t.y + m.y * t.x;
-        }
-        write = true;
-      } else if (it >= nm1c && it <= nm2c) {
-        const int ncorec = nctot > 0 ? at.ncore : 0;
-        if (it > at.ics && it <= at.ics + ncorec) {
-          // sum_b ppb(nc+b, it-ics, i) cphiq(b, itp)
-          const double* pc = at.ppb + static_cast<long long>(it - at.ics - 1) * at.nlnm +
-                             static_cast<long long>(i) * at.nlnm * at.nlnm;
-          for (int b = 0; b < nv; ++b) {
-            const double w = pc[nc + b];
-            acc.x += w * sq[b][jp].x;
-            acc.y += w * sq[b][jp].y;
-          }
-          write = true;
-        }
-      }
-      if (write) {
-        const double2 o = make_double2(ph.x * acc.x - ph.y * acc.y, ph.x * acc.y + ph.y * acc.x);
-        zt[(at.ims - 1 + i) + static_cast<long long>(itl) * nbloch + static_cast<long long>(itp) * nbloch * nmtot] = o;
-      }
-    }
-    __syncthreads();
   }
 }
 
@@ -122,7 +84,7 @@ __global__ void conj_kernel(double2* a, long long n) {
     a[e].y = -a[e].y;
 }
 
-static DevBuf g_zm_atoms;
+static DevBuf g_zm_atoms, g_zm_t;
 
 // ---- interstitial plane-wave part (m_zmel.f90:418-535)
 // M(c, g) = ggg(sg * vg(g) - vc(c) - nadd) or 0 when that vector is not in the ggg table.
@@ -216,7 +178,9 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
   else { nm1c = nm1; nm2c = nm2; nm1v = 0; nm2v = -1; }
   QSGW_ARG(nm2v < nm1v || cphim_d, "zmel_mt: cphim required for valence middle states");
   std::vector<ZmelAtomDev> h(natom);
-  int nvmax = 1;
+  const bool valence = nm2v >= nm1v;
+  int nvmax = 1, mdmax = 0;
+  long long tsize = 0;
   for (int ia = 0; ia < natom; ++ia) {
     const qsgw_zmel_atom& a = atoms[ia];
     QSGW_ARG(a.nv >= 1 && a.nv <= ZM_NVMAX && a.nc >= 0 && a.nc + a.nv <= a.nlnm && a.ppb_d,
@@ -224,27 +188,45 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
     QSGW_ARG(a.ims >= 1 && a.ims - 1 + a.mdim <= nbloch && a.ias >= 1 && a.ias - 1 + a.nv <= ldq,
              "zmel_mt: atom %d offsets outside zmelt/cphi", ia);
     QSGW_ARG(a.ncore <= a.nc, "zmel_mt: atom %d ncore=%d > nc=%d", ia, a.ncore, a.nc);
-    h[ia] = ZmelAtomDev{a.ppb_d, a.nlnm, a.nc, a.nv, a.ias, a.ics, a.ims, a.mdim, a.ncore, a.phase_re, a.phase_im};
+    h[ia] = ZmelAtomDev{a.ppb_d, a.nlnm, a.nc, a.nv, a.ias, a.ics, a.ims, a.mdim, a.ncore, a.phase_re, a.phase_im,
+                        tsize};
+    tsize += static_cast<long long>(a.nv) * std::max(a.mdim, 0) * ntp0;
     nvmax = std::max(nvmax, a.nv);
+    mdmax = std::max(mdmax, a.mdim);
   }
-  const size_t smem = static_cast<size_t>(3 * nvmax * ZM_T) * sizeof(double2) + static_cast<size_t>(nvmax) * nvmax * sizeof(double);
-  static uint64_t attr = 0;                       // one bit per device
-  rc = smem_limit_once(reinterpret_cast<const void*>(zmel_mt_kernel),
-                       static_cast<int>(3 * ZM_NVMAX * ZM_T * sizeof(double2) + ZM_NVMAX * ZM_NVMAX * sizeof(double)),
-                       attr);
-  if (rc) return rc;
+  if (mdmax <= 0) return QSGW_OK;
   cudaStream_t s = ctx().stream;
+  const int nmtot = nm2 - nm1 + 1;
   rc = g_zm_atoms.ensure(natom * sizeof(ZmelAtomDev));
   if (rc) return rc;
+  if ((rc = g_zm_t.ensure(static_cast<size_t>(tsize) * sizeof(double2)))) return rc;
   QSGW_CUDA(cudaMemcpyAsync(g_zm_atoms.p, h.data(), natom * sizeof(ZmelAtomDev), cudaMemcpyHostToDevice, s));
-  const int nmtot = nm2 - nm1 + 1;
-  dim3 grid(natom, (ntp0 + ZM_T - 1) / ZM_T, (nmtot + ZM_T - 1) / ZM_T);
-  zmel_mt_kernel<<<grid, 128, smem, s>>>(reinterpret_cast<double2*>(zmelt_d), nbloch, nm1, nmtot, nctot, ntp0, nm1v,
-                                         nm2v, nm1c, nm2c, reinterpret_cast<const double2*>(cphim_d), ldm,
-                                         reinterpret_cast<const double2*>(cphiq_d), ldq, g_zm_atoms.as<ZmelAtomDev>(),
-                                         nvmax);
+  // cphiq columns and one product function's valence block (99 KB at 96 channels)
+  auto smem_of = [](int nv) {
+    return static_cast<size_t>(nv) * ZM_TQ * sizeof(double2) + static_cast<size_t>(nv + 1) * nv * sizeof(double);
+  };
+  static uint64_t attr = 0;                       // one bit per device
+  rc = smem_limit_once(reinterpret_cast<const void*>(zmel_ppb_kernel), static_cast<int>(smem_of(ZM_NVMAX)), attr);
+  if (rc) return rc;
+  const size_t smem = smem_of(nvmax);
+  double2* zt = reinterpret_cast<double2*>(zmelt_d);
+  zmel_ppb_kernel<<<dim3(mdmax, (ntp0 + ZM_TQ - 1) / ZM_TQ, natom), 256, smem, s>>>(
+      g_zm_t.as<double2>(), zt, nbloch, nm1, nmtot, nctot, ntp0, nm1c, nm2c,
+      reinterpret_cast<const double2*>(cphiq_d), ldq, g_zm_atoms.as<ZmelAtomDev>(), nvmax);
   count_launch();
-  QSGW_LAUNCH_CHECK("zmel_mt_kernel");
+  QSGW_LAUNCH_CHECK("zmel_ppb_kernel");
+  if (!valence) return QSGW_OK;
+  // zmelt(ims.., it, itp) = phase sum_a T(itp, i, a) conj(cphim(ias+a, it)) (:365): per target column one
+  // mdim x nmv product over nv
+  for (int ia = 0; ia < natom; ++ia) {
+    const ZmelAtomDev& a = h[ia];
+    rc = zgemm_f64(1, 3, a.mdim, nm2v - nm1v + 1, a.nv, make_double2(a.ph_re, a.ph_im), g_zm_t.as<double2>() + a.toff,
+                   a.nv, static_cast<long long>(a.nv) * a.mdim,
+                   reinterpret_cast<const double2*>(cphim_d) + (a.ias - 1), ldm, 0, make_double2(0.0, 0.0),
+                   zt + (a.ims - 1) + static_cast<long long>(nm1v - nm1) * nbloch, nbloch,
+                   static_cast<long long>(nbloch) * nmtot, ntp0, s);
+    if (rc) return rc;
+  }
   return QSGW_OK;
 }
 
@@ -266,11 +248,11 @@ extern "C" int qsgw_zmel_m2e_d(double* zmel_d, const double* zmelt_d, int ngb, i
                      reinterpret_cast<const double2*>(m2e_d), ngb, reinterpret_cast<const double2*>(zmelt_d), ngb,
                      ctx().nslices > 0 ? ctx().nslices : 4, s);
     if (rc) return rc;
-  } else {                                                         // zmel = m2e^H zmelt (:559-560)
-    rc = zgemm_f64(2, 0, nbb, static_cast<int>(ncol), ngb, make_double2(1, 0), reinterpret_cast<const double2*>(m2e_d),
+  } else {   // zmel = m2e^H zmelt (:559-560); its conjugate m2e^T conj(zmelt) when asked for, in the same pass
+    rc = zgemm_f64(zmelconjg ? 1 : 2, zmelconjg ? 3 : 0, nbb, static_cast<int>(ncol), ngb, make_double2(1, 0), reinterpret_cast<const double2*>(m2e_d),
                    ngb, 0, reinterpret_cast<const double2*>(zmelt_d), ngb, 0, make_double2(0, 0),
                    reinterpret_cast<double2*>(zmel_d), nbb, 0, 1, s);
-    if (rc) return rc;
+    return rc;
   }
   if (zmelconjg) {                                                 // :590-594
     const long long n = static_cast<long long>(nbb) * ncol;
