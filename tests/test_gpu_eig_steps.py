@@ -1,0 +1,27 @@
+"""The Jacobi steps at odd sizes, at the edges of their 16-pair and 64-row blocks, and with a padded leading
+dimension: residual, orthonormality and eigenvalues against LAPACK within 64 n eps of the matrix norm."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,pad", [(3, 0), (31, 2), (32, 0), (33, 0), (34, 1), (63, 0), (65, 3), (129, 0)])
+def test_jacobi_block_edges(qsgw, n, pad):
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    v = g @ g.conj().T * 10.0 ** rng.uniform(-3, 3)
+    v = 0.5 * (v + v.conj().T)
+    v[0, :] = v[:, 0] = 0.0                                   # a decoupled state: no rotation at all
+    v[0, 0] = 1.0
+    buf = np.full((n + pad, n), 7.0 + 0j, order="F")
+    buf[:n] = v
+    d = qsgw.to_device(buf)
+    lam = qsgw.zhegv_d(d, n, lda=n + pad)
+    z = qsgw.from_device(d, buf.shape)
+    tol = 64 * n * np.finfo(float).eps
+    norm = np.linalg.norm(v, 2)
+    assert np.abs(lam - np.linalg.eigvalsh(v)[::-1]).max() <= tol * norm
+    assert np.abs(v @ z[:n] - z[:n] * lam).max() <= tol * norm
+    assert np.abs(z[:n].conj().T @ z[:n] - np.eye(n)).max() <= tol
+    assert np.all(z[n:] == 7.0)
