@@ -9,8 +9,11 @@
 //     chi0(w_r(t))  = i rcxq(t) + sum_i rcxq(i) rmatt(t, i)     (:243-257)
 // with imatt, rmatt from hilbertmat (hilbertmat.f90:14-79, FP64 logs).  Here
 // the normalisation and the i rcxq(t) term are folded into one small complex
-// matrix B (slots 0..nwhis x [niw imaginary | nw+1 real] columns), built on
-// the host in FP64 as the reference's dpsion_init builds its matrices, and
+// matrix B (slots 0..nwhis x [niw imaginary | nw+1 real] columns), built in
+// FP64 by a kernel, one thread per element (the host loop of the reference's
+// dpsion_init, 28 000 complex logarithms at 96 bins and 73 frequencies, took
+// 1.7 ms, most of a q point of 16 k at 233 rows; against 40 digits the kernel's
+// elements are 1.2e-15 off, the loop's 5.2e-14); it remains for the SmearX0 filter and qsgw_dpsion_matrix), and
 // the N^2-sized work is two passes of the DMMA GEMM over rcxq:
 //     zxqi = rcxq . B[:, imag],   zxq = rcxq . B[:, real].
 // rcxq is not modified (the reference leaves chi0(w_r) in rcxq(:, :, 0:nw);
@@ -127,9 +130,72 @@ void build_transform(int nwhis, const double* frhis, int niw, const double* freq
   }
 }
 
+// ---- the same matrix on the device (no SmearX0 filter)
+// int_a^b (m w + n) / (w - z) dw = m facm + n facn, as hm2; log((z - b) / (z - a)) = log(1 + q),
+// q = (a - b) / (z - a), by log1p where q is small (a bin far from z), which keeps facm's cancellation
+// z log + (b - a) accurate
+__device__ void hm2_d(double2 z, double a, double b, double2& facm, double2& facn) {
+  const double2 da = make_double2(z.x - a, z.y), db = make_double2(z.x - b, z.y);
+  facm = facn = make_double2(0.0, 0.0);
+  const double na = hypot(da.x, da.y), nb = hypot(db.x, db.y);
+  if (!(na > 1e-8 && nb > 1e-8)) return;
+  const double f = (a - b) / (na * na);
+  const double2 q = make_double2(f * da.x, -f * da.y);
+  const double mag = fabs(q.x) + fabs(q.y);
+  facn.x = mag < 0.5 ? 0.5 * log1p(q.x * (2.0 + q.x) + q.y * q.y) : log(nb / na);
+  facn.y = atan2(q.y, 1.0 + q.x);
+  facm = make_double2(z.x * facn.x - z.y * facn.y + (b - a), z.x * facn.y + z.y * facn.x);
+}
+
+// Re rmat(i), i = +-1..+-nwhis, of hilbertmat_h: the two half bins of i itself and the neighbours' halves
+// that interpolate towards its centre, added in the host's order
+__device__ double rmat_re(double2 z, int nwhis, const double* fr, int i) {
+  auto left = [&](int k) { return k > 0 ? fr[k - 1] : -fr[-k]; };
+  auto right = [&](int k) { return k > 0 ? fr[k] : -fr[-k - 1]; };
+  auto centre = [&](int k) { return 0.5 * (left(k) + right(k)); };
+  double2 m, f;
+  double r = 0.0;
+  const double ci = centre(i);
+  if (i != -nwhis && i != 1) {                       // the right half of bin i - 1
+    const double c = centre(i - 1);
+    hm2_d(z, c, right(i - 1), m, f);
+    r += (m.x - f.x * c) / (ci - c);
+  }
+  const double cim = i == -nwhis ? left(i) : (i == 1 ? 0.0 : centre(i - 1));
+  hm2_d(z, left(i), ci, m, f);
+  r += (m.x - f.x * cim) / (ci - cim);
+  const double cip = i == nwhis ? right(i) : (i == -1 ? 0.0 : centre(i + 1));
+  hm2_d(z, ci, right(i), m, f);
+  r += (-m.x + f.x * cip) / (cip - ci);
+  if (i != nwhis && i != -1) {                       // the left half of bin i + 1
+    const double c = centre(i + 1);
+    hm2_d(z, left(i + 1), c, m, f);
+    r += (-m.x + f.x * c) / (c - ci);
+  }
+  return r;
+}
+
+// B(i, j) as build_transform's, smear = 0; freq: niw imaginary then nw + 1 real frequencies
+__global__ void transform_kernel(double2* __restrict__ B, int nwhis, const double* __restrict__ fr, int niw, int ncol,
+                                 const double* __restrict__ freq, double ecut) {
+  const int K = nwhis + 1, e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= K * ncol) return;
+  const int i = e % K, j = e / K;
+  double2 v = make_double2(0.0, 0.0);
+  double fnorm = 1.0;                                // slot 0 is not normalised
+  if (i > 0) {
+    const double c = 0.5 * (fr[i - 1] + fr[i]);
+    fnorm = -(ecut < 1e9 ? exp(-(c / ecut) * (c / ecut)) : 1.0) / (fr[i] - fr[i - 1]);
+    const double2 z = j < niw ? make_double2(0.0, freq[j] + 1e-13) : make_double2(freq[j], 1e-13);
+    v.x = fnorm * ((rmat_re(z, nwhis, fr, i) - rmat_re(z, nwhis, fr, -i)) / 3.14159265358979323846);
+  }
+  if (j >= niw && i == j - niw) v.y += fnorm;
+  B[e] = v;
+}
+
 }  // namespace
 
-static DevBuf g_dp_b;
+static DevBuf g_dp_b, g_dp_t;
 
 }  // namespace qsgw
 
@@ -154,13 +220,26 @@ extern "C" int qsgw_dpsion_chiq_d(const double* rcxq, int npr, int npr_col, int 
   QSGW_ARG(M <= INT_MAX, "dpsion_chiq: npr*npr_col = %lld too large", M);
   QSGW_ARG(((reinterpret_cast<uintptr_t>(rcxq) | reinterpret_cast<uintptr_t>(zxqi) |
              reinterpret_cast<uintptr_t>(zxq)) & 15) == 0, "dpsion_chiq: complex arrays must be 16-byte aligned");
-  std::vector<cd> B;
-  build_transform(nwhis, frhis, niw, freq_i, nw, freq_r, ecut, smearx0, B);
-  const int K = nwhis + 1;
+  const int K = nwhis + 1, ncol = niw + nw + 1;
   cudaStream_t s = ctx().stream;
-  rc = g_dp_b.ensure(B.size() * sizeof(cd));
+  rc = g_dp_b.ensure(static_cast<size_t>(K) * ncol * sizeof(cd));
   if (rc) return rc;
-  if ((rc = h2d(g_dp_b.p, B.data(), B.size() * sizeof(cd), s))) return rc;
+  if (std::fabs(smearx0) > 1e-15) {
+    std::vector<cd> B;
+    build_transform(nwhis, frhis, niw, freq_i, nw, freq_r, ecut, smearx0, B);
+    if ((rc = h2d(g_dp_b.p, B.data(), B.size() * sizeof(cd), s))) return rc;
+  } else if (ncol > 0) {
+    std::vector<double> tab(frhis, frhis + K);
+    tab.insert(tab.end(), freq_i, freq_i + niw);
+    if (nw >= 0) tab.insert(tab.end(), freq_r, freq_r + nw + 1);
+    if ((rc = g_dp_t.ensure(tab.size() * sizeof(double)))) return rc;
+    if ((rc = h2d(g_dp_t.p, tab.data(), tab.size() * sizeof(double), s))) return rc;
+    const double* d_fr = g_dp_t.as<double>();
+    QSGW_ARG(static_cast<long long>(K) * ncol < INT_MAX, "dpsion_chiq: %d bins x %d frequencies too large", K, ncol);
+    transform_kernel<<<(K * ncol + 63) / 64, 64, 0, s>>>(g_dp_b.as<double2>(), nwhis, d_fr, niw, ncol, d_fr + K, ecut);
+    count_launch();
+    QSGW_LAUNCH_CHECK("transform_kernel");
+  }
   const double2* A = reinterpret_cast<const double2*>(rcxq);
   const double2* Bd = g_dp_b.as<double2>();
   const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
