@@ -11,8 +11,6 @@
 //      W matrices; every column is written once (no scatter races).
 //   4. zsec += czmelwc^H zmel (:599) with split-K, then Im zsec_ii <= 0 (:601-607).
 #include <cmath>
-#include <map>
-#include <set>
 #include <string>
 #include <algorithm>
 #include <vector>
@@ -126,6 +124,21 @@ __global__ void hermitize_kernel(double2* __restrict__ out, const double2* __res
   }
 }
 
+// The pole weights of a task: scale[r ncol + col] = w3[i] where record r = rec[i] of the entry is used, zero
+// elsewhere (cleared by the caller).  An entry's three records differ and a column has one entry.
+struct PoleEntry { int col; int ixs; double w3[3]; };
+__global__ void pole_scatter_kernel(double* __restrict__ scale, const PoleEntry* __restrict__ ent, int nent,
+                                    const int* __restrict__ slot_of_bin, long long ncol) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nent) return;
+  const PoleEntry p = ent[e];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int r = slot_of_bin[p.ixs - 1 + i];
+    if (r >= 0) scale[r * ncol + p.col] = p.w3[i];
+  }
+}
+
 __global__ void clamp_diag_kernel(double2* zsec, int ntqxx, int ntq) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < ntqxx) {
@@ -170,8 +183,6 @@ static void inverse33_h(const double m[3][3], double inv[3][3]) {
     for (int j = 0; j < 3; ++j) inv[i][j] = c[i][j] / det;   // inv = transpose(cof) / det
 }
 
-struct PoleEntry { int col; int ixs; double w3[3]; };
-
 static int pole_table_h(const qsgw_sxcf_args& a, std::vector<PoleEntry>& out) {
   const int nm = a.ns2 - a.ns1 + 1;
   int nt0p = 0, nt0m = 0;
@@ -179,40 +190,63 @@ static int pole_table_h(const qsgw_sxcf_args& a, std::vector<PoleEntry>& out) {
     if (a.ekc[i] < a.ef + 10.0 * a.esmr) ++nt0p;
     if (a.ekc[i] < a.ef - 10.0 * a.esmr) ++nt0m;
   }
+  const bool sorted = std::is_sorted(a.freq_r + 1, a.freq_r + a.nw + 1);
+  std::vector<double> invs(9 * static_cast<size_t>(a.nw + 1));     // the 3-point matrices of the bins met so far
+  std::vector<char> have(a.nw + 1, 0);
   for (int itp = 1; itp <= a.ntqxx; ++itp) {
     const double omg = a.omega[itp - 1];
     const int itini = omg >= a.ef ? std::max(a.ns1, nt0m + 1) : a.ns1;
     const int itend = omg >= a.ef ? a.ns2r : std::min(nt0p, a.ns2r);
+    const double el = std::min(omg, a.ef), eh = std::max(omg, a.ef);
+    if (eh - el < 1e-6) continue;                                  // wfacx2 = 0
+    // more than 6.5 sqrt(2) esmr from both window ends the two error functions saturate: inside the
+    // window wfacx2 is 1 and weavx2 is the level itself to the last bit (0.5 erfc(6.5) = 1.9e-20), outside
+    // wfacx2 is below the 1e-8 cut
+    const double far = 6.5 * std::sqrt(2.0) * a.esmr;
     for (int it = itini; it <= itend; ++it) {
-      double wf = wfacx2_h(omg, a.ef, a.ekc[it - 1], it <= a.nctot ? 0.0 : a.esmr);
+      const double ek = a.ekc[it - 1];
+      const double esmrx = it <= a.nctot ? 0.0 : a.esmr;
+      const bool inside = eh - ek > far && ek - el > far;
+      if (ek - eh > far || el - ek > far) continue;
+      double wf = inside ? 1.0 : wfacx2_h(omg, a.ef, ek, esmrx);
       if (wf < 1e-8) continue;
       wf = wf * a.wkkr * (std::signbit(omg - a.ef) ? -1.0 : 1.0);
-      const double we = 0.5 * std::fabs(omg - weavx2_h(omg, a.ef, a.ekc[it - 1], a.esmr));
+      const double we = 0.5 * std::fabs(omg - (inside ? ek : weavx2_h(omg, a.ef, ek, a.esmr)));
       int ixs = 0;
-      for (int i = 1; i <= a.nw; ++i)
-        if (a.freq_r[i] > we) { ixs = i; break; }
+      if (sorted) {
+        ixs = static_cast<int>(std::upper_bound(a.freq_r + 1, a.freq_r + a.nw + 1, we) - a.freq_r);
+        if (ixs > a.nw) ixs = 0;
+      } else {
+        for (int i = 1; i <= a.nw; ++i)
+          if (a.freq_r[i] > we) { ixs = i; break; }
+      }
       if (ixs == 0 || ixs + 1 > a.nw) {
         set_error("sxcf: pole frequency %g outside the real-axis mesh (freq_r(nw)=%g)", we, a.freq_r[a.nw]);
         return QSGW_ERR_ARG;
       }
-      double am[3][3], inv[3][3];
-      for (int r = 0; r < 3; ++r) {
-        const double xi = a.freq_r[ixs - 1 + r];
-        am[r][0] = 1.0; am[r][1] = xi * xi; am[r][2] = xi * xi * xi * xi;
+      double* iv = invs.data() + 9 * static_cast<size_t>(ixs);
+      if (!have[ixs]) {
+        double am[3][3], inv[3][3];
+        for (int r = 0; r < 3; ++r) {
+          const double xi = a.freq_r[ixs - 1 + r];
+          am[r][0] = 1.0; am[r][1] = xi * xi; am[r][2] = xi * xi * xi * xi;
+        }
+        inverse33_h(am, inv);
+        for (int r = 0; r < 9; ++r) iv[r] = inv[r / 3][r % 3];
+        have[ixs] = 1;
       }
-      inverse33_h(am, inv);
       const double v[3] = {1.0, we * we, we * we * we * we};
       PoleEntry e;
       e.col = (it - a.ns1) + nm * (itp - 1);
       e.ixs = ixs;
-      for (int j = 0; j < 3; ++j) e.w3[j] = wf * (v[0] * inv[0][j] + v[1] * inv[1][j] + v[2] * inv[2][j]);
+      for (int j = 0; j < 3; ++j) e.w3[j] = wf * (v[0] * iv[j] + v[1] * iv[3 + j] + v[2] * iv[6 + j]);
       out.push_back(e);
     }
   }
   return QSGW_OK;
 }
 
-static DevBuf g_sc_wg, g_sc_w3, g_sc_cz, g_sc_wi, g_sc_wr, g_sc_tabs, g_sc_recs, g_sc_tmp;
+static DevBuf g_sc_wg, g_sc_w3, g_sc_cz, g_sc_wi, g_sc_wr, g_sc_tabs, g_sc_recs, g_sc_tmp, g_sc_ent;
 static DevBuf g_sc_host_zs;
 static DevBuf g_sc_trial;                // Sigma_c of the slice-count trials
 // zmel, W(i omega), W(omega) records of the host-pointer calls: twelve slots (about 0.6 GB each
@@ -241,13 +275,14 @@ static int sxcf_check(const qsgw_sxcf_args* a) {
 // host plan: pole entries, the real-axis records they read, and the column tiles.  Columns are
 // sorted by their pole bin ixs (0 = no pole) and cut into tiles of the kernel's column width; a
 // tile's segments are the niw+1 imaginary slots and the union of its columns' real-axis bins.
-// scale_bin[r][col] = the column's pole weight on record r (zero when the column has no pole
+// On the device scale[r][col] = the column's pole weight on record r (zero when the column has no pole
 // there), so mixing bins in a tile adds no padding columns.
 struct SxcfPlan {
   int nm = 0;
   long long ncol = 0;
   std::vector<int> recs;                 // real-axis bins used, in record order
-  std::vector<double> scale_bin;         // [nrec][ncol]
+  std::vector<PoleEntry> poles;
+  std::vector<int> slot_of_bin;          // [nw + 1] record of a bin, -1 = unused
   std::vector<int> tile_cols, tile_group, gseg_off, gnseg, seg_slot;   // slot niw+1+r = record r
 };
 
@@ -256,46 +291,44 @@ static int sxcf_plan(const qsgw_sxcf_args& a, int tilew, SxcfPlan& pl) {
   pl.nm = a.ns2 - a.ns1 + 1;
   pl.ncol = static_cast<long long>(pl.nm) * a.ntqxx;
   const long long ncol = pl.ncol;
-  std::vector<PoleEntry> poles;
-  int rc = pole_table_h(a, poles);
+  int rc = pole_table_h(a, pl.poles);
   if (rc) return rc;
   // bins needed by the pole entries, restricted to [nwxi, nwx] (:557)
-  std::map<int, int> bin_slot;
-  for (const auto& e : poles)
-    for (int i = 0; i < 3; ++i) {
-      const int b = e.ixs - 1 + i;
-      if (b >= a.nwxi && b <= a.nwx && !bin_slot.count(b)) bin_slot.emplace(b, 0);
-    }
+  pl.slot_of_bin.assign(a.nw + 1, -1);
+  for (const auto& e : pl.poles)
+    for (int b = e.ixs - 1; b <= e.ixs + 1; ++b)
+      if (b >= a.nwxi && b <= a.nwx) pl.slot_of_bin[b] = 0;
   pl.recs.clear();
-  for (auto& kv : bin_slot) { kv.second = static_cast<int>(pl.recs.size()); pl.recs.push_back(kv.first); }
-  const int nrec = static_cast<int>(pl.recs.size());
-  std::vector<int> key(ncol, 0);
-  for (const auto& e : poles) key[e.col] = e.ixs;
-  pl.scale_bin.assign(static_cast<size_t>(std::max(nrec, 1)) * ncol, 0.0);
-  for (const auto& e : poles)
-    for (int i = 0; i < 3; ++i) {
-      auto it = bin_slot.find(e.ixs - 1 + i);
-      if (it != bin_slot.end()) pl.scale_bin[static_cast<size_t>(it->second) * ncol + e.col] = e.w3[i];
+  for (int b = 0; b <= a.nw; ++b)
+    if (pl.slot_of_bin[b] == 0) {
+      pl.slot_of_bin[b] = static_cast<int>(pl.recs.size());
+      pl.recs.push_back(b);
     }
-  std::vector<int> order(ncol);
-  for (long long c = 0; c < ncol; ++c) order[c] = static_cast<int>(c);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return key[x] < key[y]; });
+  // columns in the order of their bins (0 = no pole), stable: a counting sort
+  std::vector<int> key(ncol, 0), start(a.nw + 2, 0), order(ncol);
+  for (const auto& e : pl.poles) key[e.col] = e.ixs;
+  for (long long c = 0; c < ncol; ++c) ++start[key[c] + 1];
+  for (int b = 0; b <= a.nw; ++b) start[b + 1] += start[b];
+  for (long long c = 0; c < ncol; ++c) order[start[key[c]]++] = static_cast<int>(c);
   pl.tile_cols.clear(); pl.tile_group.clear(); pl.gseg_off.clear(); pl.gnseg.clear(); pl.seg_slot.clear();
   int gidx = 0;
   for (long long t0 = 0; t0 < ncol; t0 += tilew) {
     const long long t1 = std::min<long long>(ncol, t0 + tilew);
     pl.gseg_off.push_back(static_cast<int>(pl.seg_slot.size()));
     for (int sgi = 0; sgi <= niw; ++sgi) pl.seg_slot.push_back(sgi);
-    std::set<int> rset;                          // records used by the tile's columns
+    // records used by the tile's columns: their keys ascend, so do the records
+    int last = -1;
     for (long long j = t0; j < t1; ++j) {
       const int k = key[order[j]];
-      if (k <= 0) continue;
-      for (int i = 0; i < 3; ++i) {
-        auto it = bin_slot.find(k - 1 + i);
-        if (it != bin_slot.end()) rset.insert(it->second);
+      if (k <= 0 || (j > t0 && k == key[order[j - 1]])) continue;
+      for (int b = k - 1; b <= k + 1; ++b) {
+        const int r = pl.slot_of_bin[b];
+        if (r > last) {
+          pl.seg_slot.push_back(niw + 1 + r);
+          last = r;
+        }
       }
     }
-    for (int r : rset) pl.seg_slot.push_back(niw + 1 + r);
     pl.gnseg.push_back(static_cast<int>(pl.seg_slot.size()) - pl.gseg_off.back());
     pl.tile_group.push_back(gidx++);
     for (int j = 0; j < tilew; ++j) pl.tile_cols.push_back(t0 + j < t1 ? order[t0 + j] : -1);
@@ -321,11 +354,12 @@ static int sxcf_bind(const qsgw_sxcf_args& a, SxcfPlan& pl, const SxcfBufs& b, S
   if (rc) return rc;
   double* dt = g_sc_tabs.as<double>();
   double *d_x = dt, *d_wt = dt + niw, *d_ex = dt + 2 * niw, *d_om = dt + 3 * niw, *d_ekc = d_om + a.ntq;
-  if ((rc = h2d(d_x, a.freqx, niw * sizeof(double), s))) return rc;
-  if ((rc = h2d(d_wt, a.wwx, niw * sizeof(double), s))) return rc;
-  if ((rc = h2d(d_ex, a.expa, niw * sizeof(double), s))) return rc;
-  if ((rc = h2d(d_om, a.omega, a.ntq * sizeof(double), s))) return rc;
-  if ((rc = h2d(d_ekc, a.ekc, a.nekc * sizeof(double), s))) return rc;
+  std::vector<double> tab(a.freqx, a.freqx + niw);
+  tab.insert(tab.end(), a.wwx, a.wwx + niw);
+  tab.insert(tab.end(), a.expa, a.expa + niw);
+  tab.insert(tab.end(), a.omega, a.omega + a.ntq);
+  tab.insert(tab.end(), a.ekc, a.ekc + a.nekc);
+  if ((rc = h2d(dt, tab.data(), tab.size() * sizeof(double), s))) return rc;
   if ((rc = b.wg->ensure(ncol * (niw + 1) * sizeof(double)))) return rc;
   wgtim_kernel<<<static_cast<int>((ncol + 127) / 128), 128, 0, s>>>(
       b.wg->as<double>(), niw, a.ns1, pl.nm, a.ntqxx, a.nctot, d_om, d_ekc, a.esmr, a.wkkr, a.ua, d_x, d_wt, d_ex);
@@ -366,8 +400,24 @@ static int sxcf_bind(const qsgw_sxcf_args& a, SxcfPlan& pl, const SxcfBufs& b, S
     }
     wr = b.wr->as<double2>();
   }
-  if ((rc = b.w3->ensure(pl.scale_bin.size() * sizeof(double)))) return rc;
-  if ((rc = h2d(b.w3->p, pl.scale_bin.data(), pl.scale_bin.size() * sizeof(double), s))) return rc;
+  // pole weights: the entries travel and are spread on the device (the full table, 35 records x 16 000
+  // columns of the benchmark's tasks, was 4.5 MB of pageable memory a task and held the host until its turn
+  // in the stream)
+  const size_t w3n = static_cast<size_t>(std::max(nrec, 1)) * ncol;
+  if ((rc = b.w3->ensure(w3n * sizeof(double)))) return rc;
+  if (nrec > 0) {
+    const int nent = static_cast<int>(pl.poles.size());
+    const size_t eb = pl.poles.size() * sizeof(PoleEntry), bb = pl.slot_of_bin.size() * sizeof(int);
+    if ((rc = g_sc_ent.ensure(eb + bb))) return rc;
+    PoleEntry* d_ent = g_sc_ent.as<PoleEntry>();
+    int* d_bin = reinterpret_cast<int*>(g_sc_ent.as<char>() + eb);
+    if ((rc = h2d(d_ent, pl.poles.data(), eb, s))) return rc;
+    if ((rc = h2d(d_bin, pl.slot_of_bin.data(), bb, s))) return rc;
+    QSGW_CUDA(cudaMemsetAsync(b.w3->p, 0, w3n * sizeof(double), s));
+    pole_scatter_kernel<<<(nent + 127) / 128, 128, 0, s>>>(b.w3->as<double>(), d_ent, nent, d_bin, ncol);
+    count_launch();
+    QSGW_LAUNCH_CHECK("pole_scatter_kernel");
+  }
   if ((rc = b.cz->ensure(static_cast<size_t>(ngb) * ncol * sizeof(double2)))) return rc;
   sa = SigcSplitArgs();
   sa.ngb = ngb; sa.ldw = ldw;
