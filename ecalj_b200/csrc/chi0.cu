@@ -6,6 +6,7 @@
 // The host builds the (jpm, iw) bin lists in the reference's icoun order
 // (x0gemm.f90:37-64); the GPU never materialises zw / wzw: the pair gather
 // and the weight are folded into the operand loads of the DMMA engine.
+#include <algorithm>
 #include <memory>
 #include <cmath>
 #include <vector>
@@ -225,42 +226,61 @@ extern "C" int qsgw_x0gemm(double* rcxq, int npr, int ipr_col, int npr_col, int 
 // All-k chi0 with Lorentzian weights built on the device.
 namespace qsgw {
 
-__global__ void lorentz_weight_kernel(double* __restrict__ w, const int* __restrict__ peo,
-                                      const int* __restrict__ peu, const double* __restrict__ eo,
-                                      const double* __restrict__ eu, const double* __restrict__ fi,
-                                      long long npair, int niw, double inv_nk) {
-  const long long total = npair * niw;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long pr = i % npair;
-    const int iw = static_cast<int>(i / npair);
-    const double de = eu[peu[pr]] - eo[peo[pr]];
-    const double om = fi[iw];
-    w[i] = -2.0 * de / (de * de + om * om) * inv_nk;   // chi0(iw) <= 0 (dpsion5.f90:218)
+// A k-point's pairs: columns [col0, next col0) = (it - 1) + nocc (itp - 1), as zmel(:, it, itp); o0 and u0 are
+// its first occupied and unoccupied energy.
+struct KPairs {
+  long long col0;
+  int nocc, o0, u0, pad;
+};
+// the excitation energy of pair column pr
+__device__ __forceinline__ double pair_energy(long long pr, const KPairs* __restrict__ kp, int nk,
+                                              const double* __restrict__ eo, const double* __restrict__ eu) {
+  int lo = 0, hi = nk - 1;                         // the last k with col0 <= pr (k-points without pairs share one)
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (kp[mid].col0 <= pr) lo = mid;
+    else hi = mid - 1;
+  }
+  const KPairs k = kp[lo];
+  const int c = static_cast<int>(pr - k.col0);
+  return eu[k.u0 + c / k.nocc] - eo[k.o0 + c % k.nocc];
+}
+
+// One thread a pair, all frequencies: the pair's energies are found from the k table (pair index maps from the
+// host were 8 bytes a pair of pageable copies, formed in a host loop).
+__global__ void lorentz_weight_kernel(double* __restrict__ w, const KPairs* __restrict__ kp, int nk,
+                                      const double* __restrict__ eo, const double* __restrict__ eu,
+                                      const double* __restrict__ fi, long long npair, int niw, double inv_nk) {
+  for (long long pr = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; pr < npair;
+       pr += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const double de = pair_energy(pr, kp, nk, eo, eu);
+    for (int iw = blockIdx.y; iw < niw; iw += gridDim.y) {
+      const double om = fi[iw];
+      w[iw * npair + pr] = -2.0 * de / (de * de + om * om) * inv_nk;   // chi0(iw) <= 0 (dpsion5.f90:218)
+    }
   }
 }
 
 // Real frequency axis: f(w) = [1/(w - de + i eta) - 1/(w + de + i eta)] / nk, whose value at
 // w = i nu is the imaginary-axis weight above.  Slot iw holds Re f, slot nw + iw holds Im f.
-__global__ void lorentz_real_weight_kernel(double* __restrict__ w, const int* __restrict__ peo,
-                                           const int* __restrict__ peu, const double* __restrict__ eo,
-                                           const double* __restrict__ eu, const double* __restrict__ fr,
-                                           long long npair, int nw, double eta, double inv_nk) {
-  const long long total = npair * nw;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long pr = i % npair;
-    const int iw = static_cast<int>(i / npair);
-    const double de = eu[peu[pr]] - eo[peo[pr]];
-    const double om = fr[iw];
-    const double a = om - de, b = om + de, e2 = eta * eta;
-    const double da = 1.0 / (a * a + e2), db = 1.0 / (b * b + e2);
-    w[i] = (a * da - b * db) * inv_nk;
-    w[static_cast<long long>(nw) * npair + i] = (-eta * da + eta * db) * inv_nk;
+__global__ void lorentz_real_weight_kernel(double* __restrict__ w, const KPairs* __restrict__ kp, int nk,
+                                           const double* __restrict__ eo, const double* __restrict__ eu,
+                                           const double* __restrict__ fr, long long npair, int nw, double eta,
+                                           double inv_nk) {
+  for (long long pr = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; pr < npair;
+       pr += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const double de = pair_energy(pr, kp, nk, eo, eu);
+    for (int iw = blockIdx.y; iw < nw; iw += gridDim.y) {
+      const double om = fr[iw];
+      const double a = om - de, b = om + de, e2 = eta * eta;
+      const double da = 1.0 / (a * a + e2), db = 1.0 / (b * b + e2);
+      w[iw * npair + pr] = (a * da - b * db) * inv_nk;
+      w[static_cast<long long>(nw + iw) * npair + pr] = (-eta * da + eta * db) * inv_nk;
+    }
   }
 }
 
-static DevBuf g_lz_map, g_lz_e, g_lz_w, g_lz_bins, g_lz_fi;
+static DevBuf g_lz_map, g_lz_e, g_lz_w, g_lz_bins;
 
 // eta < 0: imaginary axis, nw slots of weights; eta >= 0: real axis, 2 nw slots (Re, Im).
 // classes (out): bit 0 when a weight can be negative, bit 1 when one can be positive
@@ -276,59 +296,47 @@ int chi0_lorentz_weights(int niw, const double* freq_i, int nk, const int* nocc,
     no_tot += nocc[k];
     nu_tot += nun[k];
   }
-  std::vector<int> peo(npair), peu(npair);
+  std::vector<KPairs> kp(nk);
   long long c = 0, oo = 0, uo = 0;
+  int cl = 0;
   for (int k = 0; k < nk; ++k) {
-    // column order of zcols: (it - 1) + nocc_k * (itp - 1), as zmel(:, it, itp)
-    for (int itp = 0; itp < nun[k]; ++itp)
-      for (int it = 0; it < nocc[k]; ++it) {
-        peo[c] = static_cast<int>(oo + it);
-        peu[c] = static_cast<int>(uo + itp);
-        ++c;
-      }
+    kp[k] = KPairs{c, std::max(nocc[k], 1), static_cast<int>(oo), static_cast<int>(uo), 0};
+    // imaginary axis: w = -2 de / (de^2 + w^2) / nk has the sign of -de, de between the extremes of this k
+    if (classes && nocc[k] > 0 && nun[k] > 0) {
+      const auto o = std::minmax_element(eocc + oo, eocc + oo + nocc[k]);
+      const auto u = std::minmax_element(eunocc + uo, eunocc + uo + nun[k]);
+      cl |= (*u.second - *o.first > 0.0 ? 1 : 0) | (*u.first - *o.second < 0.0 ? 2 : 0);
+    }
+    c += static_cast<long long>(nocc[k]) * nun[k];
     oo += nocc[k];
     uo += nun[k];
   }
-  if (classes) {
-    // imaginary axis: w = -2 de / (de^2 + w^2) / nk has the sign of -de; the real axis has both
-    int cl = 0;
-    if (eta >= 0.0) cl = 3;
-    else
-      for (long long i = 0; i < npair && cl != 3; ++i) {
-        const double de = eunocc[peu[i]] - eocc[peo[i]];
-        cl |= (de > 0.0 ? 1 : 0) | (de < 0.0 ? 2 : 0);
-      }
-    *classes = cl;
-  }
-  int rc = g_lz_map.ensure(2 * std::max<long long>(npair, 1) * sizeof(int));
+  if (classes) *classes = eta >= 0.0 ? 3 : cl;       // the real axis has both signs
+  int rc = g_lz_map.ensure(nk * sizeof(KPairs));
   if (rc) return rc;
-  rc = g_lz_e.ensure((no_tot + nu_tot + 1) * sizeof(double));
+  rc = g_lz_e.ensure((no_tot + nu_tot + niw) * sizeof(double));
   if (rc) return rc;
   rc = g_lz_w.ensure(std::max<long long>(npair, 1) * niw * (eta >= 0.0 ? 2 : 1) * sizeof(double));
   if (rc) return rc;
-  rc = g_lz_fi.ensure(niw * sizeof(double));
-  if (rc) return rc;
-  int* dpeo = g_lz_map.as<int>();
-  int* dpeu = dpeo + npair;
   double* deo = g_lz_e.as<double>();
-  double* deu = deo + no_tot;
-  if ((rc = h2d(dpeo, peo.data(), npair * sizeof(int), s))) return rc;
-  if ((rc = h2d(dpeu, peu.data(), npair * sizeof(int), s))) return rc;
-  if ((rc = h2d(deo, eocc, no_tot * sizeof(double), s))) return rc;
-  if ((rc = h2d(deu, eunocc, nu_tot * sizeof(double), s))) return rc;
-  if ((rc = h2d(g_lz_fi.p, freq_i, niw * sizeof(double), s))) return rc;
-  const long long tot = npair * niw;
-  const int blocks = static_cast<int>(std::min<long long>((tot + 255) / 256, 8LL * ctx().sm_count));
-  if (tot > 0 && eta < 0.0) {
-    lorentz_weight_kernel<<<std::max(blocks, 1), 256, 0, s>>>(g_lz_w.as<double>(), dpeo, dpeu, deo, deu,
-                                                              g_lz_fi.as<double>(), npair, niw, inv_nk);
+  double *deu = deo + no_tot, *dfi = deu + nu_tot;
+  std::vector<double> tab(eocc, eocc + no_tot);
+  tab.insert(tab.end(), eunocc, eunocc + nu_tot);
+  tab.insert(tab.end(), freq_i, freq_i + niw);
+  if ((rc = h2d(g_lz_map.p, kp.data(), nk * sizeof(KPairs), s))) return rc;
+  if ((rc = h2d(deo, tab.data(), tab.size() * sizeof(double), s))) return rc;
+  if (npair > 0) {
+    const KPairs* dkp = g_lz_map.as<KPairs>();
+    const unsigned gx = static_cast<unsigned>(std::min<long long>((npair + 255) / 256, 8LL * ctx().sm_count));
+    // few pairs: the frequencies are spread over the grid as well
+    const unsigned gy = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(niw, 4LL * ctx().sm_count / gx)));
+    if (eta < 0.0)
+      lorentz_weight_kernel<<<dim3(gx, gy), 256, 0, s>>>(g_lz_w.as<double>(), dkp, nk, deo, deu, dfi, npair, niw, inv_nk);
+    else
+      lorentz_real_weight_kernel<<<dim3(gx, gy), 256, 0, s>>>(g_lz_w.as<double>(), dkp, nk, deo, deu, dfi, npair, niw,
+                                                              eta, inv_nk);
     count_launch();
-    QSGW_LAUNCH_CHECK("lorentz_weight_kernel");
-  } else if (tot > 0) {
-    lorentz_real_weight_kernel<<<std::max(blocks, 1), 256, 0, s>>>(g_lz_w.as<double>(), dpeo, dpeu, deo, deu,
-                                                                   g_lz_fi.as<double>(), npair, niw, eta, inv_nk);
-    count_launch();
-    QSGW_LAUNCH_CHECK("lorentz_real_weight_kernel");
+    QSGW_LAUNCH_CHECK("lorentz weight kernel");
   }
   w_d = g_lz_w.as<double>();
   return QSGW_OK;
