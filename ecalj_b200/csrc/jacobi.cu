@@ -2,22 +2,24 @@
 // diagonalisation that feeds v^1/2 and the E basis (main_hvccfp0.f90:322-367,
 // zhgv_d / zhgv_h in m_lapack.f90:64-104, 203-229).
 //
-// Parallel cyclic two-sided Jacobi: each step applies N/2 disjoint plane
-// rotations chosen by a round-robin tournament ordering; a sweep is N-1
-// steps.  A step is ONE kernel: the rotations of pairs k and l touch the
-// 2 x 2 block (rows of k, columns of l) and nothing else, so each thread
-// takes one block from A to the next A (two copies, as the angles of a step
-// come from diagonal blocks that other blocks of threads are rotating) and
-// further threads rotate the columns of V.  The complex rotation first
-// removes the phase of a_pq, then applies the real Jacobi rotation with
+// Parallel cyclic block Jacobi.  The matrix is cut into blocks of 16 rows; a
+// step pairs the blocks by a round-robin tournament (a sweep meets every
+// pair of blocks once) and is two kernels: jacobi_solve_kernel runs one
+// sweep of plane rotations over the 32 x 32 diagonal problem of each pair in
+// shared memory and leaves its unitary U, jacobi_apply_kernel forms
+// A <- U^H A U and V <- V U block by block.  A plane rotation first removes
+// the phase of a_pq, then applies the real Jacobi rotation with
 // t = sgn(tau) / (|tau| + sqrt(1 + tau^2)).  Sweeps stop when the
 // off-diagonal norm is below 1e-14 of the Frobenius norm.
 //
-// What bounds it: the chain of N-1 dependent steps a sweep, each a few
-// microseconds of launch, L2 round trips and the angle's square roots.
-// Programmatic dependent launch starts a step's blocks while the previous
-// step ends.  n = 260: 3.9 us a step, 14.1 ms in all (12.8 us a step with
-// three kernels, 46.3 ms).
+// What bounds it: chains of dependent steps, not arithmetic.  Rotations
+// between global steps cost a launch and an L2 round trip each (3.9 us at
+// n = 260, N-1 of them a sweep); inside a block's 32 x 32 problem a step is
+// two barriers and the angle's square roots (0.9 us).  Programmatic
+// dependent launch overlaps the launches.  n = 260: 29 us a solve and 10 us
+// an update, 17 of them a sweep: 10.0 ms (14.1 with a global step per
+// rotation set, 46.3 with three launches for each).  Angles formed in FP32
+// (rotations normalised in FP64) did not converge at n = 160.
 // The generalised problem (-v) z = lambda O z is reduced with O^-1/2 built
 // from a Jacobi solve of O.
 #include <algorithm>
@@ -73,79 +75,150 @@ __device__ __forceinline__ void rotate(double2& xp, double2& xq, const Rot& r, d
   xq = make_double2(r.s * a.x + r.c * eb.x, r.s * a.y + r.c * eb.y);
 }
 
-// One step t: B <- J^H A J and V <- V J.  Blocks x < nA take JT x JT pairs of A (thread = one 2 x 2 block),
-// the others JT pairs x JVR rows of V.  An odd n pairs one index with the absent player ne - 1: it keeps
-// its row and column.
-constexpr int JT = 16, JVR = 64;
-__global__ void __launch_bounds__(JT * JT) jacobi_step_kernel(const double2* A, double2* B, double2* V, int n, int ne, int t,
-                                                              int nA, int ntile) {
-  __shared__ Rot rk[JT], rl[JT];
-  __shared__ int pl[JT][2];
-  const int tid = threadIdx.x, npair = ne / 2;
-  const bool isA = static_cast<int>(blockIdx.x) < nA;
-  const int bi = isA ? blockIdx.x % ntile : (blockIdx.x - nA) / ntile;   // A: row pairs; V: row block
-  const int bl = isA ? blockIdx.x / ntile : (blockIdx.x - nA) % ntile;   // column pairs
-  // the previous step has to be complete before anything of it is read or overwritten
+constexpr int JB = 16, JW = 2 * JB, JP = JW + 1;     // block width, pair width, shared-memory pitch
+
+// global index of slot i (0..31) of the block pair (P, Q): P's rows, then Q's; n for an absent one
+__device__ __forceinline__ int slot_index(int i, int P, int Q, int n) {
+  const int blk = i < JB ? P : Q, g = blk * JB + (i & (JB - 1));
+  return g < n ? g : n;
+}
+
+// One sweep of the 32-slot problem of every block pair of step t; U[pair] (32 x 32, column-major) <- its
+// unitary.  Absent slots are zero rows and columns: nothing rotates with them.  Thread = one 2 x 2 block
+// of a step; two copies of the problem, as a step's angles come from blocks other threads are rotating.
+// No __restrict__ on A: the previous kernel, which may still run when these blocks start, writes it.
+__global__ void __launch_bounds__(JB * JB) jacobi_solve_kernel(const double2* A, double2* U, int n, int ne, int t) {
+  extern __shared__ double2 jac_smem[];
+  double2* sa[2] = {jac_smem, jac_smem + JW * JP};
+  double2* su = jac_smem + 2 * JW * JP;
+  __shared__ Rot rot[JB];
+  const int tid = threadIdx.x, kb = tid & (JB - 1), lb = tid / JB;
+  int P, Q;
+  pair_of(t, blockIdx.x, ne, P, Q);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // a block's elements are requested before the angles are formed
-  const int ta = tid & (JT - 1), tb = tid / JT;
-  int p0 = n, p1 = n, q0 = n, q1 = n;
-  const double2 zero = make_double2(0.0, 0.0);
-  double2 a00 = zero, a01 = zero, a10 = zero, a11 = zero;
-  if (isA) {
-    if (bi * JT + ta < npair) pair_of(t, bi * JT + ta, ne, p0, p1);
-    if (bl * JT + tb < npair) pair_of(t, bl * JT + tb, ne, q0, q1);
-    const double2 *c0 = A + static_cast<long long>(q0) * n, *c1 = A + static_cast<long long>(q1) * n;
-    if (p0 < n && q0 < n) a00 = c0[p0];
-    if (p0 < n && q1 < n) a01 = c1[p0];
-    if (p1 < n && q0 < n) a10 = c0[p1];
-    if (p1 < n && q1 < n) a11 = c1[p1];
-  }
-  if (tid < 2 * JT) {
-    const bool col = tid < JT;
-    const int k = (col ? bl : bi) * JT + ta;
-    int p = n, q = n;
-    Rot r{1.0, 0.0, make_double2(1.0, 0.0)};
-    if ((col || isA) && k < npair) {
-      pair_of(t, k, ne, p, q);
-      if (q < n) r = rotation(A, n, p, q);
-    }
-    (col ? rl : rk)[ta] = r;
-    if (col) { pl[ta][0] = p; pl[ta][1] = q; }
+#pragma unroll
+  for (int e = 0; e < JW * JW / (JB * JB); ++e) {
+    const int i = tid & (JW - 1), j = tid / JW + e * (JB * JB / JW);
+    const int gi = slot_index(i, P, Q, n), gj = slot_index(j, P, Q, n);
+    sa[0][i + j * JP] = (gi < n && gj < n) ? A[gi + static_cast<long long>(gj) * n] : make_double2(0.0, 0.0);
+    su[i + j * JP] = make_double2(i == j ? 1.0 : 0.0, 0.0);
   }
   __syncthreads();
-  if (isA) {
-    const Rot r = rk[ta], c = rl[tb];
+  for (int st = 0; st < JW - 1; ++st) {
+    const double2* cur = sa[st & 1];
+    double2* nxt = sa[(st & 1) ^ 1];
+    if (tid < JB) {
+      int p, q;
+      pair_of(st, tid, JW, p, q);
+      rot[tid] = rotation(cur, JP, p, q);
+    }
+    int p0, p1, q0, q1;
+    pair_of(st, kb, JW, p0, p1);
+    pair_of(st, lb, JW, q0, q1);
+    double2 a00 = cur[p0 + q0 * JP], a01 = cur[p0 + q1 * JP], a10 = cur[p1 + q0 * JP], a11 = cur[p1 + q1 * JP];
+    __syncthreads();
+    const Rot r = rot[kb], c = rot[lb];
+    rotate(a00, a01, c, c.ph);
+    rotate(a10, a11, c, c.ph);
+    const double2 cph = make_double2(r.ph.x, -r.ph.y);              // rows: the conjugate phase
+    rotate(a00, a10, r, cph);
+    rotate(a01, a11, r, cph);
+    nxt[p0 + q0 * JP] = a00;
+    nxt[p0 + q1 * JP] = a01;
+    nxt[p1 + q0 * JP] = a10;
+    nxt[p1 + q1 * JP] = a11;
     if (c.s != 0.0) {
-      rotate(a00, a01, c, c.ph);
-      rotate(a10, a11, c, c.ph);
-    }
-    if (r.s != 0.0) {                                 // rows: the conjugate phase
-      const double2 cph = make_double2(r.ph.x, -r.ph.y);
-      rotate(a00, a10, r, cph);
-      rotate(a01, a11, r, cph);
-    }
-    double2 *c0 = B + static_cast<long long>(q0) * n, *c1 = B + static_cast<long long>(q1) * n;
-    if (p0 < n && q0 < n) c0[p0] = a00;
-    if (p0 < n && q1 < n) c1[p0] = a01;
-    if (p1 < n && q0 < n) c0[p1] = a10;
-    if (p1 < n && q1 < n) c1[p1] = a11;
-  } else {
-    const int i = bi * JVR + (tid & (JVR - 1));
-    if (i >= n) return;
 #pragma unroll
-    for (int u = 0; u < JT * JVR / (JT * JT); ++u) {
-      const int l = tid / JVR + u * (JT * JT / JVR);
-      const Rot c = rl[l];
-      if (c.s == 0.0) continue;                       // also the pairs without a second index
-      double2 *xp = V + i + static_cast<long long>(pl[l][0]) * n, *xq = V + i + static_cast<long long>(pl[l][1]) * n;
-      double2 a = *xp, b = *xq;
-      rotate(a, b, c, c.ph);
-      *xp = a;
-      *xq = b;
+      for (int h = 0; h < 2; ++h) {                                  // U's columns q0, q1: rows kb, kb + 16
+        double2 *xp = su + (kb + h * JB) + q0 * JP, *xq = su + (kb + h * JB) + q1 * JP;
+        double2 x = *xp, y = *xq;
+        rotate(x, y, c, c.ph);
+        *xp = x;
+        *xq = y;
+      }
     }
+    __syncthreads();
   }
+  double2* Up = U + static_cast<long long>(blockIdx.x) * JW * JW;
+#pragma unroll
+  for (int e = 0; e < JW * JW / (JB * JB); ++e) {
+    const int i = tid & (JW - 1), j = tid / JW + e * (JB * JB / JW);
+    Up[i + j * JW] = su[i + j * JP];
+  }
+}
+
+// out(2 x 4 per thread) = op(X) Y for 32 x 32 tiles in shared memory; CONJ: X^H
+template <bool CONJ>
+__device__ __forceinline__ void tile_product(double2 (&o)[2][4], const double2* X, const double2* Y, int i0, int j0) {
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) o[u][v] = make_double2(0.0, 0.0);
+#pragma unroll 4
+  for (int k = 0; k < JW; ++k) {
+    double2 x[2], y[4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      x[u] = CONJ ? X[k + (i0 + 16 * u) * JP] : X[i0 + 16 * u + k * JP];
+      if (CONJ) x[u].y = -x[u].y;
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) y[v] = Y[k + (j0 + v) * JP];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        o[u][v].x += x[u].x * y[v].x - x[u].y * y[v].y;
+        o[u][v].y += x[u].x * y[v].y + x[u].y * y[v].x;
+      }
+  }
+}
+
+// A <- U^H A U (blocks x < npair^2: pair of rows k, pair of columns l, in place) and V <- V U (the others: 32
+// rows of V, pair l)
+__global__ void __launch_bounds__(128) jacobi_apply_kernel(double2* A, double2* V, const double2* U, int n, int ne,
+                                                           int t, int npair) {
+  extern __shared__ double2 jac_smem[];
+  double2 *sx = jac_smem, *sl = sx + JW * JP, *sk = sl + JW * JP;
+  const int tid = threadIdx.x, i0 = tid & 15, j0 = (tid >> 4) * 4;
+  const bool isA = static_cast<int>(blockIdx.x) < npair * npair;
+  const int b = isA ? blockIdx.x : blockIdx.x - npair * npair;
+  const int l = b % npair, k = b / npair;               // V: k = row block
+  int P, Q, R, S;
+  pair_of(t, l, ne, P, Q);
+  pair_of(t, k, ne, R, S);                              // unused for V
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  double2* M = isA ? A : V;
+#pragma unroll
+  for (int e = 0; e < JW * JW / 128; ++e) {
+    const int i = tid & (JW - 1), j = tid / JW + e * (128 / JW);
+    const int gi = isA ? slot_index(i, R, S, n) : (k * JW + i < n ? k * JW + i : n), gj = slot_index(j, P, Q, n);
+    sx[i + j * JP] = (gi < n && gj < n) ? M[gi + static_cast<long long>(gj) * n] : make_double2(0.0, 0.0);
+    sl[i + j * JP] = U[static_cast<long long>(l) * JW * JW + i + j * JW];
+    if (isA) sk[i + j * JP] = U[static_cast<long long>(k) * JW * JW + i + j * JW];
+  }
+  __syncthreads();
+  double2 o[2][4];
+  tile_product<false>(o, sx, sl, i0, j0);
+  if (isA) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) sx[i0 + 16 * u + (j0 + v) * JP] = o[u][v];
+    __syncthreads();
+    tile_product<true>(o, sk, sx, i0, j0);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int i = i0 + 16 * u;
+      const int gi = isA ? slot_index(i, R, S, n) : (k * JW + i < n ? k * JW + i : n), gj = slot_index(j0 + v, P, Q, n);
+      if (gi < n && gj < n) M[gi + static_cast<long long>(gj) * n] = o[u][v];
+    }
 }
 
 // off-diagonal and total squared norms -> out[0], out[1]
@@ -211,39 +284,48 @@ static int grid_for(long long n) {
 
 // A (n x n Hermitian, kept): V (n x n) <- eigenvectors; d <- unsorted eigenvalues (host).
 static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vector<double>& d, cudaStream_t s) {
-  const int ne = n + (n & 1);
-  const int npair = ne / 2;
-  // the two copies the steps go back and forth between (ld n)
-  int rc = g_jc_b.ensure(2 * static_cast<size_t>(n) * n * sizeof(double2));
+  const int nb = (n + JB - 1) / JB;
+  const int ne = nb + (nb & 1);                         // an odd block count pairs one block with an absent one
+  const int npair = ne / 2, nrow = (n + JW - 1) / JW;
+  const size_t nn = static_cast<size_t>(n) * n;
+  // working copy of A (ld n), then the pairs' unitaries
+  int rc = g_jc_b.ensure((nn + static_cast<size_t>(npair) * JW * JW) * sizeof(double2));
   if (rc) return rc;
   rc = g_jc_norm.ensure(2 * sizeof(double));
   if (rc) return rc;
   rc = g_jc_d.ensure(n * sizeof(double));
   if (rc) return rc;
   double2* cur = g_jc_b.as<double2>();
-  double2* nxt = cur + static_cast<size_t>(n) * n;
+  double2* U = cur + nn;
   const size_t row = static_cast<size_t>(n) * sizeof(double2);
   QSGW_CUDA(cudaMemcpy2DAsync(cur, row, A, lda * sizeof(double2), row, n, cudaMemcpyDeviceToDevice, s));
-  const int ntile = (npair + JT - 1) / JT, nA = ntile * ntile, nV = ntile * ((n + JVR - 1) / JVR);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(nA + nV));
-  cfg.blockDim = dim3(JT * JT);
-  cfg.stream = s;
+  constexpr int SMEM = 3 * JW * JP * static_cast<int>(sizeof(double2));
+  static uint64_t at_solve = 0, at_apply = 0;           // one bit per device
+  if ((rc = smem_limit_once(reinterpret_cast<const void*>(jacobi_solve_kernel), SMEM, at_solve))) return rc;
+  if ((rc = smem_limit_once(reinterpret_cast<const void*>(jacobi_apply_kernel), SMEM, at_apply))) return rc;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchConfig_t solve{}, apply{};
+  solve.gridDim = dim3(static_cast<unsigned>(npair));
+  solve.blockDim = dim3(JB * JB);
+  apply.gridDim = dim3(static_cast<unsigned>(npair * npair + nrow * npair));
+  apply.blockDim = dim3(128);
+  for (cudaLaunchConfig_t* c : {&solve, &apply}) {
+    c->dynamicSmemBytes = SMEM;
+    c->stream = s;
+    c->attrs = &attr;
+    c->numAttrs = 1;
+  }
   set_identity_kernel<<<grid_for(static_cast<long long>(n) * n), 256, 0, s>>>(V, n, n);
   count_launch();
   bool converged = (n <= 1);
   for (int sweep = 0; sweep < 40 && !converged; ++sweep) {
     for (int t = 0; t < ne - 1; ++t) {
-      QSGW_CUDA(cudaLaunchKernelEx(&cfg, jacobi_step_kernel, static_cast<const double2*>(cur), nxt, V, n, ne, t, nA,
-                                   ntile));
-      std::swap(cur, nxt);
+      QSGW_CUDA(cudaLaunchKernelEx(&solve, jacobi_solve_kernel, static_cast<const double2*>(cur), U, n, ne, t));
+      QSGW_CUDA(cudaLaunchKernelEx(&apply, jacobi_apply_kernel, cur, V, static_cast<const double2*>(U), n, ne, t, npair));
     }
-    count_launch(ne - 1);
+    count_launch(2 * (ne - 1));
     QSGW_LAUNCH_CHECK("jacobi sweep");
     QSGW_CUDA(cudaMemsetAsync(g_jc_norm.p, 0, 2 * sizeof(double), s));
     offdiag_norm_kernel<<<grid_for(static_cast<long long>(n) * n), 256, 0, s>>>(cur, n, n, g_jc_norm.as<double>());
