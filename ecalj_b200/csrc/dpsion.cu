@@ -13,8 +13,8 @@
 // FP64 by a kernel, one thread per element (the host loop of the reference's
 // dpsion_init, 28 000 complex logarithms at 96 bins and 73 frequencies, took
 // 1.7 ms, most of a q point of 16 k at 233 rows; against 40 digits the kernel's
-// elements are 1.2e-15 off, the loop's 5.2e-14); it remains for the SmearX0 filter and qsgw_dpsion_matrix), and
-// the N^2-sized work is two passes of the DMMA GEMM over rcxq:
+// elements are 1.2e-15 off, the loop's 5.2e-14); the loop remains for the
+// SmearX0 filter and qsgw_dpsion_matrix), and the N^2-sized work is two passes of the DMMA GEMM over rcxq:
 //     zxqi = rcxq . B[:, imag],   zxq = rcxq . B[:, real].
 // rcxq is not modified (the reference leaves chi0(w_r) in rcxq(:, :, 0:nw);
 // here it goes to zxq).

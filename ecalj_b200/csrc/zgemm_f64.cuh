@@ -354,15 +354,27 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
       const int r = tid % ZG_BM, row = r0 + r;
       if (row >= (mirror ? p.N : p.M)) return;
       const int cend = min(ZG_BN, (mirror ? p.M : p.N) - c0);
-#pragma unroll 4
-      for (int cl = tid / ZG_BM; cl < cend; cl += ZG_THREADS / ZG_BM) {
-        double2 v = mirror ? tile[r][cl] : tile[cl][r];
-        if (mirror) v.y = -v.y;
-        double2* dst = Cb + row + static_cast<long long>(c0 + cl) * p.ldc;
-        if (p.splitk > 1) {
-          atomicAdd(&dst->x, v.x); atomicAdd(&dst->y, v.y);
-        } else {
-          double2 o = *dst; o.x += v.x; o.y += v.y; *dst = o;
+      constexpr int STEP = ZG_THREADS / ZG_BM, NCOL = ZG_BN / STEP, RUN = 8;   // a thread's columns, in runs
+      for (int q0 = 0; q0 < NCOL; q0 += RUN) {
+        double2 v[RUN], o[RUN];
+#pragma unroll
+        for (int q = 0; q < RUN; ++q) {                // a run's old values are requested together
+          const int cl = tid / ZG_BM + (q0 + q) * STEP;
+          o[q] = make_double2(0.0, 0.0);
+          if (cl < cend && p.splitk == 1) o[q] = Cb[row + static_cast<long long>(c0 + cl) * p.ldc];
+        }
+#pragma unroll
+        for (int q = 0; q < RUN; ++q) {
+          const int cl = tid / ZG_BM + (q0 + q) * STEP;
+          if (cl >= cend) continue;
+          v[q] = mirror ? tile[r][cl] : tile[cl][r];
+          if (mirror) v[q].y = -v[q].y;
+          double2* dst = Cb + row + static_cast<long long>(c0 + cl) * p.ldc;
+          if (p.splitk > 1) {
+            atomicAdd(&dst->x, v[q].x); atomicAdd(&dst->y, v[q].y);
+          } else {
+            *dst = make_double2(o[q].x + v[q].x, o[q].y + v[q].y);
+          }
         }
       }
     };
