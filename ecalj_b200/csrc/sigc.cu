@@ -24,11 +24,14 @@ namespace qsgw {
 
 static constexpr double kPi = 3.14159265358979323846264338327950288;
 
-__global__ void wgtim_kernel(double* __restrict__ wg, int niw, int ns1, int nm, int ntqxx, int nctot,
-                             const double* __restrict__ omega, const double* __restrict__ ekc,
-                             double esmr, double wkkr, double ua, const double* __restrict__ x,
-                             const double* __restrict__ wt, const double* __restrict__ expa) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp a column (it, itp), its lanes over the frequencies: a thread walking all of a column's
+// exponentials left the launch with too few threads (14 us at 3600 columns, now 5).
+__global__ void __launch_bounds__(256) wgtim_kernel(double* __restrict__ wg, int niw, int ns1, int nm, int ntqxx,
+                                                    int nctot, const double* __restrict__ omega,
+                                                    const double* __restrict__ ekc, double esmr, double wkkr, double ua,
+                                                    const double* __restrict__ x, const double* __restrict__ wt,
+                                                    const double* __restrict__ expa) {
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (c >= nm * ntqxx) return;
   const int itl = c % nm, itp = c / nm;
   const int it = ns1 + itl;
@@ -38,20 +41,15 @@ __global__ void wgtim_kernel(double* __restrict__ wg, int niw, int ns1, int nm, 
   const double sig2 = 2.0 * (0.5 * esmr) * (0.5 * esmr);
   const double sgn = signbit(we) ? -1.0 : 1.0;
   double* out = wg + static_cast<long long>(c) * (niw + 1);
-  if (it <= nctot) {
-    double s0 = 0.0;
-    for (int i = 0; i < niw; ++i) {
+  const bool core = it <= nctot;
+  double s0 = 0.0;
+  for (int i = lane; i < niw; i += 32) {
+    if (core) {
       const double cons = 1.0 / (we * we * x[i] * x[i] + (1.0 - x[i]) * (1.0 - x[i]));
       const double w = we * cons * wt[i] * (-1.0 / pi);
       out[1 + i] = wkkr * w;
       s0 += w * expa[i];
-    }
-    double w0 = 0.0;
-    if (fabs(we) < 2.0 / ua) w0 = -s0 - 0.5 * sgn * exp(we * we * ua * ua) * erfc(ua * fabs(we));
-    out[0] = wkkr * w0;
-  } else {
-    double s0 = 0.0;
-    for (int i = 0; i < niw; ++i) {
+    } else {
       const double omd = 1.0 / x[i] - 1.0;
       const double omd2w = omd * omd + we * we;
       const double r = omd2w / sig2;
@@ -67,35 +65,49 @@ __global__ void wgtim_kernel(double* __restrict__ wg, int niw, int ns1, int nm, 
       out[1 + i] = wkkr * (-we * cons * wt[i] / (x[i] * x[i]) / pi);
       s0 += cons * expa[i] * wt[i] / (x[i] * x[i]);
     }
-    const double w0 = we * s0 / pi + sgn * 0.5 * exp(aw2) * (erfc(sqrt(aw2 + we * we / sig2)) - erfc(aw));
+  }
+  for (int o = 16; o; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+  if (lane == 0) {
+    double w0;
+    if (core) w0 = fabs(we) < 2.0 / ua ? -s0 - 0.5 * sgn * exp(we * we * ua * ua) * erfc(ua * fabs(we)) : 0.0;
+    else w0 = we * s0 / pi + sgn * 0.5 * exp(aw2) * (erfc(sqrt(aw2 + we * we / sig2)) - erfc(aw));
     out[0] = wkkr * w0;
   }
 }
 
-// full Hermitian (ld = n) from a packed upper triangle, column order (j, i <= j) (:327-358, :468-474)
-__global__ void unpack_upper_kernel(double2* __restrict__ w, const double2* __restrict__ up, int n,
-                                    int nmat) {
-  const long long np = static_cast<long long>(n) * (n + 1) / 2;
-  const long long tot = static_cast<long long>(n) * n * nmat;
-  for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < tot;
-       e += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n);
-    const long long r = e / n;
-    const int j = static_cast<int>(r % n);
-    const long long m = r / n;
-    double2 v;
-    if (i < j) {
-      v = up[m * np + static_cast<long long>(j) * (j + 1) / 2 + i];
-    } else if (i == j) {
-      // wc(i,j) = up then wc(j,i) = conjg(up) in the same iteration: the
-      // diagonal ends up conjugated (m_sxcf_gemm.f90:470-473)
-      const double2 u = up[m * np + static_cast<long long>(j) * (j + 1) / 2 + i];
-      v = make_double2(u.x, -u.y);
-    } else {
-      const double2 u = up[m * np + static_cast<long long>(i) * (i + 1) / 2 + j];
-      v = make_double2(u.x, -u.y);
+// full Hermitian (ld = n) from packed upper triangles, column order (j, i <= j) (:327-358, :468-474): matrix q
+// from record recs[q] (q without recs).  Block (32, 8) per 32 x 32 tile of the upper triangle (grid x) and
+// matrix (grid y); the tile is read once, coalesced, and written with its mirror image through shared memory.
+// The diagonal ends up conjugated: wc(i,j) = up then wc(j,i) = conjg(up) in the same iteration
+// (m_sxcf_gemm.f90:470-473).  68 matrices of 1500 in two launches: 0.6 ms, by writing 2.4 GB (0.9 ms in 36
+// launches with a 64-bit division per element and the triangle read by rows).
+__global__ void __launch_bounds__(256) unpack_upper_kernel(double2* __restrict__ w, const double2* __restrict__ up,
+                                                           const int* __restrict__ recs, int n) {
+  __shared__ double2 tile[32][33];
+  int tj, ti;
+  tri_decode(blockIdx.x, tj, ti);                        // ti <= tj
+  const int q = blockIdx.y;
+  const double2* u = up + static_cast<long long>(recs ? recs[q] : q) * n * (n + 1LL) / 2;
+  double2* wq = w + static_cast<long long>(q) * n * n;
+  const int i = ti * 32 + threadIdx.x;
+  for (int b = threadIdx.y; b < 32; b += 8) {
+    const int j = tj * 32 + b;
+    double2 v = make_double2(0.0, 0.0);
+    if (j < n && i <= j) {
+      v = u[static_cast<long long>(j) * (j + 1) / 2 + i];
+      if (i == j) v.y = -v.y;
+      wq[i + static_cast<long long>(j) * n] = v;
     }
-    w[e] = v;
+    tile[threadIdx.x][b] = v;
+  }
+  __syncthreads();
+  const int jr = tj * 32 + threadIdx.x;                  // the mirror: rows jr of column ic
+  for (int b = threadIdx.y; b < 32; b += 8) {
+    const int ic = ti * 32 + b;
+    if (jr < n && ic < jr) {
+      const double2 v = tile[b][threadIdx.x];
+      wq[jr + static_cast<long long>(ic) * n] = make_double2(v.x, -v.y);
+    }
   }
 }
 
@@ -361,18 +373,19 @@ static int sxcf_bind(const qsgw_sxcf_args& a, SxcfPlan& pl, const SxcfBufs& b, S
   tab.insert(tab.end(), a.ekc, a.ekc + a.nekc);
   if ((rc = h2d(dt, tab.data(), tab.size() * sizeof(double), s))) return rc;
   if ((rc = b.wg->ensure(ncol * (niw + 1) * sizeof(double)))) return rc;
-  wgtim_kernel<<<static_cast<int>((ncol + 127) / 128), 128, 0, s>>>(
+  wgtim_kernel<<<static_cast<int>((ncol + 7) / 8), 256, 0, s>>>(
       b.wg->as<double>(), niw, a.ns1, pl.nm, a.ntqxx, a.nctot, d_om, d_ekc, a.esmr, a.wkkr, a.ua, d_x, d_wt, d_ex);
   count_launch();
   QSGW_LAUNCH_CHECK("wgtim_kernel");
   // ---- W operands
   const long long ldw = a.keepwv ? ngb : a.nblochpmx;
   const long long wsz = ldw * ldw;
+  const unsigned nt32 = static_cast<unsigned>((ngb + 31) / 32), ntri = nt32 * (nt32 + 1) / 2;
   const double2* wi = reinterpret_cast<const double2*>(a.wc_imag);
   const double2* wr_src = reinterpret_cast<const double2*>(a.wc_real);
   if (a.keepwv) {
     if ((rc = b.wi->ensure(wsz * (niw + 1) * sizeof(double2)))) return rc;
-    unpack_upper_kernel<<<grid_for(wsz * (niw + 1)), 256, 0, s>>>(b.wi->as<double2>(), wi, ngb, niw + 1);
+    unpack_upper_kernel<<<dim3(ntri, niw + 1), dim3(32, 8), 0, s>>>(b.wi->as<double2>(), wi, nullptr, ngb);
     count_launch();
     QSGW_LAUNCH_CHECK("unpack_upper_kernel");
     wi = b.wi->as<double2>();
@@ -381,18 +394,13 @@ static int sxcf_bind(const qsgw_sxcf_args& a, SxcfPlan& pl, const SxcfBufs& b, S
   const double2* wr = nullptr;
   if (nrec > 0) {
     if ((rc = b.wr->ensure(wsz * nrec * sizeof(double2)))) return rc;
-    if (a.keepwv) {
-      // packed records are already (W+W^H)/2; unpack only the used ones
-      const long long np = static_cast<long long>(ngb) * (ngb + 1) / 2;
-      for (int q = 0; q < nrec; ++q) {
-        unpack_upper_kernel<<<grid_for(wsz), 256, 0, s>>>(b.wr->as<double2>() + q * wsz, wr_src + pl.recs[q] * np,
-                                                          ngb, 1);
-        count_launch();
-        QSGW_LAUNCH_CHECK("unpack_upper_kernel");
-      }
+    if ((rc = g_sc_recs.ensure(nrec * sizeof(int)))) return rc;
+    if ((rc = h2d(g_sc_recs.p, pl.recs.data(), nrec * sizeof(int), s))) return rc;
+    if (a.keepwv) {                                      // packed records are already (W+W^H)/2
+      unpack_upper_kernel<<<dim3(ntri, nrec), dim3(32, 8), 0, s>>>(b.wr->as<double2>(), wr_src, g_sc_recs.as<int>(), ngb);
+      count_launch();
+      QSGW_LAUNCH_CHECK("unpack_upper_kernel");
     } else {
-      if ((rc = g_sc_recs.ensure(nrec * sizeof(int)))) return rc;
-      if ((rc = h2d(g_sc_recs.p, pl.recs.data(), nrec * sizeof(int), s))) return rc;
       hermitize_kernel<<<dim3((ngb + 31) / 32, (ngb + 31) / 32, nrec), dim3(32, 8), 0, s>>>(
           b.wr->as<double2>(), wr_src, g_sc_recs.as<int>(), ngb, ldw, nrec);
       count_launch();
@@ -775,7 +783,7 @@ extern "C" int qsgw_sxcf_wgtim_d(double* wgtim_d, int niw, int ns1, int ns2, int
   QSGW_CUDA(cudaMemcpyAsync(d_om, omega, ntqxx * sizeof(double), cudaMemcpyHostToDevice, s));
   QSGW_CUDA(cudaMemcpyAsync(d_ekc, ekc, nekc * sizeof(double), cudaMemcpyHostToDevice, s));
   const long long ncol = static_cast<long long>(nm) * ntqxx;
-  wgtim_kernel<<<static_cast<int>((ncol + 127) / 128), 128, 0, s>>>(wgtim_d, niw, ns1, nm, ntqxx, nctot, d_om, d_ekc,
+  wgtim_kernel<<<static_cast<int>((ncol + 7) / 8), 256, 0, s>>>(wgtim_d, niw, ns1, nm, ntqxx, nctot, d_om, d_ekc,
                                                                     esmr, wkkr, ua, d_x, d_wt, d_ex);
   count_launch();
   QSGW_LAUNCH_CHECK("wgtim_kernel");
