@@ -114,14 +114,18 @@ struct SegCfg {
 };
 
 // kind::i8, A = B = signed 8-bit, D = S32, both K-major, M = 128, N = BN
-constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
-                              (static_cast<uint32_t>(BM >> 4) << 24);
+constexpr uint32_t idesc_i8(int n) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
+         (static_cast<uint32_t>(BM >> 4) << 24);
+}
+constexpr uint32_t IDESC_I8 = idesc_i8(BN);
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
+                                        uint32_t idesc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 // The MMA above preceded by a non-blocking test (mbarrier.test_wait, acquire) of phase `parity` of
 // the barrier at shared address `bar`, whose answer (1 = complete) is read only after the MMA has
@@ -129,7 +133,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 // wait between two K chunks leaves the tensor core idle; the test's latency is spent inside the
 // MMA issue instead.
 __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
-                                                      uint32_t bar, uint32_t parity) {
+                                                      uint32_t bar, uint32_t parity, uint32_t idesc) {
   uint32_t ok;
   asm volatile(
       "{\n .reg .pred p, q;\n"
@@ -138,7 +142,7 @@ __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t 
       " tcgen05.mma.cta_group::1.kind::i8 [%1], %2, %3, %7, p;\n"
       " selp.u32 %0, 1, 0, q;\n}\n"
       : "=r"(ok)
-      : "r"(tmem_d), "l"(da), "l"(db), "r"(accumulate), "r"(bar), "r"(parity), "r"(IDESC_I8)
+      : "r"(tmem_d), "l"(da), "l"(db), "r"(accumulate), "r"(bar), "r"(parity), "r"(idesc)
       : "memory");
   return ok;
 }
@@ -146,22 +150,23 @@ __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t 
 // keeps it, USE reads the kept copy (same A descriptor), LAST reads it and releases the buffer.
 enum { A_FILL = 0, A_USE = 1, A_LAST = 2 };
 template <int MODE>
-__device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+__device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
+                                           uint32_t idesc) {
   if (MODE == A_FILL)
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::fill [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
   else if (MODE == A_USE)
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::use [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
   else
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::lastuse [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 
 // The slice products of one K step: for each A slice pa (one shared-memory read through the
@@ -172,7 +177,7 @@ __device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_
 template <int NS>
 __device__ __forceinline__ uint32_t slice_products(uint32_t tmem, uint64_t da0, uint64_t db0, uint32_t a_step,
                                                    uint32_t b_step, bool start, uint32_t test_bar = 0,
-                                                   uint32_t test_parity = 0) {
+                                                   uint32_t test_parity = 0, uint32_t idesc = IDESC_I8) {
   uint32_t ready = 0;
 #pragma unroll
   for (int pa = 0; pa < NS; ++pa) {
@@ -183,12 +188,12 @@ __device__ __forceinline__ uint32_t slice_products(uint32_t tmem, uint64_t da0, 
       const uint32_t d = tmem + static_cast<uint32_t>((pa + qb) * kOzTileN);
       const uint32_t acc = (start && pa == 0) ? 0u : 1u;
       if (NS - pa == 1) {
-        if (test_bar) ready = umma_i8_then_test(d, da, db, acc, test_bar, test_parity);
-        else umma_i8(d, da, db, acc);
+        if (test_bar) ready = umma_i8_then_test(d, da, db, acc, test_bar, test_parity, idesc);
+        else umma_i8(d, da, db, acc, idesc);
       }
-      else if (qb == 0) umma_i8_ca<A_FILL>(d, da, db, acc);
-      else if (qb == NS - pa - 1) umma_i8_ca<A_LAST>(d, da, db, acc);
-      else umma_i8_ca<A_USE>(d, da, db, acc);
+      else if (qb == 0) umma_i8_ca<A_FILL>(d, da, db, acc, idesc);
+      else if (qb == NS - pa - 1) umma_i8_ca<A_LAST>(d, da, db, acc, idesc);
+      else umma_i8_ca<A_USE>(d, da, db, acc, idesc);
     }
   }
   return ready;
@@ -594,6 +599,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L::OFF_MISC + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nper = (nchunk + PER - 1) / PER;
+  // the tile whose 64 rows are the first 64 of its 128 columns: the other columns lie above the diagonal and
+  // come from the mirror, so its MMAs are 64 columns wide
+  const bool half = p.herm && mt * 64 + 63 < nt * BN + 64;
+  const uint32_t idesc = idesc_i8(half ? BN / 2 : BN);
 
   if (tid == 0) {
     for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&cfull[i], NCONV); mbar_init(&empty[i], 1); }
@@ -646,7 +655,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int kk = 0; kk < K8 / 32; ++kk)
         ready = slice_products<NS>(tmem, dA0 + static_cast<uint32_t>((st * NS * SLA8) >> 4) + 2 * kk,
                                    dB0 + static_cast<uint32_t>((st * NS * SLB8) >> 4) + 2 * kk, SLA8 >> 4,
-                                   SLB8 >> 4, first && kk == 0, kk == K8 / 32 - 1 ? nbar : 0u, npar);
+                                   SLB8 >> 4, first && kk == 0, kk == K8 / 32 - 1 ? nbar : 0u, npar, idesc);
       umma_commit(&empty[st]);
       if (last) umma_commit(accfull);
       if (++st == NST) { st = 0; ph ^= 1; }
@@ -694,6 +703,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       // drain the period: exact int64 sums of the combined levels
       if (!mbar_wait_warp(accfull, per & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
+      if (half && c_lo >= BN / 2) {                    // nothing was accumulated there
+        __syncwarp();
+        if (lane == 0) mbar_arrive(accempty);
+        ++per;
+        continue;
+      }
 #pragma unroll
       for (int blk = 0; blk < 8; ++blk) {
         uint32_t v[NS][4];
@@ -716,23 +731,58 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       ++per;
     }
-    if (ok && per == nper && !*abort_flag) {
-      const int m = mt * 64 + (row & 63);
-      const int part = row >= 64 ? 1 : 0;
-      if (m < p.M) {
-        const double* mub = p.mu + static_cast<long long>(bin) * p.Rows;
-        const double fm = mub[m] * p.post * p.sign;
-        double2* Cb = p.C + static_cast<long long>(p.bin_slab[bin]) * p.c_bs;
+    // The tile leaves through the stage buffers (free: the last period's MMAs are done), so its columns and
+    // the columns of its mirror image are whole runs.  Straight from the registers every mirrored element
+    // was an atomic on a sector of its own: about 15 us a CTA, most of a bin of few pairs.
+    double2* tile = reinterpret_cast<double2*>(sm);      // [column 0..127][row 0..63], pitch TP
+    constexpr int TP = 65;
+    static_assert(BN * TP * static_cast<int>(sizeof(double2)) <= L::OFF_W, "the tile fits the stage buffers");
+    const bool good = ok && per == nper;
+    if (!good) *abort_flag = 1;
+    {
+      const int ml = row & 63, part = row >= 64 ? 1 : 0;
+      const double* mub = p.mu + static_cast<long long>(bin) * p.Rows;
+      const int m = mt * 64 + ml;
+      const double fm = m < p.M ? mub[m] * p.post * p.sign : 0.0;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int n = nt * BN + c_lo + j;
-          // the upper part of a Hermitian output comes from the mirror
-          if (n < p.N && !(p.herm && m < n)) {
-            const double val = static_cast<double>(acc[j]) * fm * mub[p.row_b0 + n];
-            atomicAdd(reinterpret_cast<double*>(Cb + m + static_cast<long long>(n) * p.ldc) + part, val);
-            if (p.herm && m > n)                          // C(n, m) = conj(C(m, n))
-              atomicAdd(reinterpret_cast<double*>(Cb + n + static_cast<long long>(m) * p.ldc) + part,
-                        part ? -val : val);
+      for (int j = 0; j < 32; ++j) {
+        const int n = nt * BN + c_lo + j;
+        const double val = n < p.N ? static_cast<double>(acc[j]) * fm * mub[p.row_b0 + n] : 0.0;
+        reinterpret_cast<double*>(tile + (c_lo + j) * TP + ml)[part] = val;
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(NDW * 32) : "memory");
+    if (!*abort_flag) {
+      double2* Cb = p.C + static_cast<long long>(p.bin_slab[bin]) * p.c_bs;
+      const bool alone = gridDim.z == 1;                 // no other CTA adds to these elements
+      auto add = [&](double2* dst, double2 v) {
+        if (alone) {
+          const double2 o = *dst;
+          *dst = make_double2(o.x + v.x, o.y + v.y);
+        } else {
+          atomicAdd(&dst->x, v.x);
+          atomicAdd(&dst->y, v.y);
+        }
+      };
+      const int dt = dw * 32 + lane;                     // 0..511
+      {
+        // columns: 64 rows of 8 columns at a time; the upper part of a Hermitian output comes from the mirror
+        const int ml = dt & 63, m = mt * 64 + ml;
+#pragma unroll 4
+        for (int c = dt >> 6; c < BN; c += NDW * 32 / 64) {
+          const int n = nt * BN + c;
+          if (m < p.M && n < p.N && !(p.herm && m < n)) add(Cb + m + static_cast<long long>(n) * p.ldc, tile[c * TP + ml]);
+        }
+      }
+      if (p.herm) {                                      // C(n, m) = conj(C(m, n)), m > n
+        const int c = dt & (BN - 1), n = nt * BN + c;
+#pragma unroll 4
+        for (int ml = dt >> 7; ml < 64; ml += NDW * 32 / BN) {
+          const int m = mt * 64 + ml;
+          if (m < p.M && n < p.N && m > n) {
+            double2 v = tile[c * TP + ml];
+            v.y = -v.y;
+            add(Cb + n + static_cast<long long>(m) * p.ldc, v);
           }
         }
       }
@@ -1474,12 +1524,21 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
     for (int mt = 0; mt < ntm; ++mt)
       if (!herm || mt * 64 + 63 >= nt * BN) ++units;
   units *= nbins;
-  // split K so that one wave of CTAs covers whole (bin, K part) units: the tiles of a unit share its
-  // rows of Y8 through L2 only while they run together
-  const long long tiles_per_bin = units / nbins;
+  // K splits: whole waves of one CTA an SM, counted in chunk times; a CTA's start and end (TMEM, pipeline
+  // fill, the drain and the FP64 additions of its tile) cost about as much as 24 chunks.  The tiles of a
+  // (bin, K part) unit are adjacent in the grid and share its rows of Y8 through L2.  (Splitting until one
+  // wave held a whole unit gave 37 splits of 5 chunks at 180 rows and 6000 pairs: 208 us.)
   const int maxsplit = std::max(1, std::min(maxch / 4, 64));
-  int heur = static_cast<int>(std::max<long long>(1, (ctx().sm_count + tiles_per_bin / 2) / tiles_per_bin));
-  heur = std::min(heur, maxsplit);
+  auto cost = [&](int sp) {
+    return static_cast<double>((units * sp + ctx().sm_count - 1) / ctx().sm_count) * ((maxch + sp - 1) / sp + 24);
+  };
+  double tbest = cost(1);
+  for (int sp = 2; sp <= maxsplit; ++sp) tbest = std::min(tbest, cost(sp));
+  // of the counts within 2 % the largest: shorter parts keep the CTAs that share rows of Y8 closer together
+  // (600 rows, 390 834 pairs, 24 bins: 65.3 ms unsplit, 62.5 at 20)
+  int heur = 1;
+  for (int sp = 1; sp <= maxsplit; ++sp)
+    if (cost(sp) <= 1.02 * tbest) heur = sp;
   // every bin over the same columns in order, weights at ew[b * n + e]: z is sliced in one pass
   bool dense = ecol_d == nullptr;
   for (int b = 0; b < nbins && dense; ++b) dense = bins.cnt[b] == bins.cnt[0] && bins.ebeg[b] == static_cast<long long>(b) * bins.cnt[0];
@@ -1548,7 +1607,7 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
   std::vector<int> cands;
   for (int c : {1, 2, 3, 4, 5, 6, 8})
     if (c <= maxsplit) cands.push_back(c);
-  if (heur > 8) cands.push_back(heur);
+  if (heur == 7 || heur > 8) cands.push_back(heur);
   char key[200];
   std::snprintf(key, sizeof(key), "%s i8x%d M=%d N=%d bins=%d chunks~2^%.3f", tune_key ? tune_key : "-", ns, M, N, nbins,
                 std::round(8.0 * std::log2(static_cast<double>(std::max(1, maxch)))) / 8.0);

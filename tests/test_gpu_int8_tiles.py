@@ -1,0 +1,117 @@
+"""The int8 kernels at the edges of their tiles and splits, against the FP64 path on the same inputs.
+
+Bounds: an operand element is rounded to 2^-(7 ns) (chi0) or about 2^-(8 ns - 1) (Sigma_c, M -> E) of the largest of
+its row or column, products below the last slice are dropped (ns of them), and the rounding errors of K terms add
+with random signs: relative to the row and column scales the error of an element stays below
+(ns + 2) unit sqrt(K) and the tests compare Frobenius norms of whole outputs."""
+import numpy as np
+import pytest
+
+from ecalj_b200 import sched, synth
+from oracle import sxcf
+
+pytestmark = pytest.mark.gpu
+
+
+def _rc(rng, *shape):
+    return np.asfortranarray(rng.standard_normal(shape) + 1j * rng.standard_normal(shape))
+
+
+@pytest.fixture
+def i8(qsgw):
+    yield lambda ns: qsgw.set_precision(qsgw.PREC_SPLIT_I8, ns)
+    qsgw.set_precision(qsgw.PREC_FP64, 1)
+
+
+# largest element over rms of a normal sample of these sizes: under 5
+PEAK = 5.0
+
+
+@pytest.mark.parametrize("ns", [2, 3, 4])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 127, 128, 129, 192, 193])
+def test_chi0_hermitian_tiles(qsgw, i8, n, ns):
+    """Diagonal tiles half a tile wide, their mirror, one and several K parts."""
+    import torch
+    for nun in (3, 40):
+        p = synth.chi0_problem(N=n, nk=3, nocc=2, nun=(nun, nun + 2), niw=3, seed=n + nun)
+        z = qsgw.to_device(p["zcols"])
+        out = []
+        for mode in ("fp64", "i8"):
+            if mode == "i8":
+                i8(ns)
+            else:
+                qsgw.set_precision(qsgw.PREC_FP64, 1)
+            chi = torch.zeros(n * n * 3, dtype=torch.complex128, device="cuda")
+            qsgw.chi0_lorentz_d(chi, n, 3, p["freq_i"], 3, p["nocc"], p["nun"], p["eocc_h"], p["eun_h"], z)
+            qsgw.synchronize()
+            out.append(qsgw.from_device(chi, (n, n, 3)))
+        ref, got = out
+        for iw in range(3):
+            # row scale: sqrt(max |w|) max |z| rounded up to a power of two, against sqrt(|w|) |z| (weights span 80)
+            unit = 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** (-7 * ns)
+            assert np.linalg.norm(got[:, :, iw] - ref[:, :, iw]) <= (ns + 2) * unit * np.linalg.norm(ref[:, :, iw])
+            assert np.array_equal(got[:, :, iw], got[:, :, iw].conj().T)
+
+
+@pytest.mark.parametrize("npr,ipr_col,npr_col", [(130, 1, 130), (70, 3, 129)])
+def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col):
+    rng = np.random.default_rng(npr)
+    nbb, nm, nq, nwhis, ncoun = 140, 4, 6, 5, 60
+    z = _rc(rng, nbb, nm, nq)
+    tabs = (rng.integers(1, nm + 1, ncoun), rng.integers(1, nq + 1, ncoun), np.ones(ncoun, int),
+            *(2 * [rng.integers(1, nwhis + 1, ncoun)]), np.arange(1, ncoun + 1))
+    w = rng.uniform(-1, 1, ncoun)
+    r0 = _rc(rng, npr, npr_col, nwhis + 1)
+    out = []
+    for ns in (0, 4):
+        if ns:
+            i8(ns)
+        r = r0.copy(order="F")
+        qsgw.x0gemm(r, npr, ipr_col, npr_col, nwhis, 1, 1, nm, z, 1, 1, ncoun, *tabs, w)
+        out.append(r)
+    inc = np.linalg.norm(out[0] - r0)
+    assert np.linalg.norm(out[1] - out[0]) <= 6 * 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** -28 * inc + 1e-14 * np.linalg.norm(r0)
+
+
+def _sigma(qsgw, t, wi, wr, n, nm, ntq, keepwv=False):
+    nwxi, nwx, ntmax = sched.get_nwx(t["omega"], t["ekc"], t["freq_r"], t["ef"], t["esmr"])
+    if keepwv:
+        pack = lambda w: np.asfortranarray(np.stack([np.concatenate([w[:j + 1, j, k] for j in range(n)])
+                                                     for k in range(w.shape[2])], axis=1))
+        wi, wr = pack(wi), pack(wr)
+    zs = np.zeros((ntq, ntq), complex, order="F")
+    qsgw.sxcf_correlation(zs, t["zmel"], 1, nm, min(nm, ntmax), nwxi, nwx, ntq, wi, wr, t["omega"], t["ekc"], 0, t["ef"],
+                          t["esmr"], 1 / 8, t["ua"], t["x"], t["wx"], t["expa"], t["freq_r"], keepwv=keepwv)
+    return zs
+
+
+@pytest.mark.parametrize("ns", [2, 3, 4])
+@pytest.mark.parametrize("n,nm,ntq", [(1, 3, 2), (31, 5, 2), (32, 40, 3), (33, 40, 4), (64, 60, 5), (65, 9, 2),
+                                      (96, 70, 2), (97, 33, 6)])
+def test_sigma_segment_splits_and_chunks(qsgw, i8, n, nm, ntq, ns):
+    """K extents of one, one and a half and two chunks; few tiles (segments split over CTAs); the paired last row tile
+    alone (n <= 32), beside full ones (65, 96) and absent (64)."""
+    t = synth.sigc_task(n, ntq, nm, 11, 30, seed=n, esmr=0.02, ef=0.05)
+    rng = np.random.default_rng(n)
+    w = _rc(rng, n, n, 12)
+    wi, wr = np.asfortranarray(w + w.conj().transpose(1, 0, 2)), _rc(rng, n, n, 30)
+    ref = _sigma(qsgw, t, wi, wr, n, nm, ntq)
+    i8(ns)
+    got = _sigma(qsgw, t, wi, wr, n, nm, ntq)
+    # Sigma adds nm n terms of czmelwc^H zmel; its elements cancel, so the scale is that of the unsigned sum
+    wg = sxcf.wgtim(t["omega"], t["ekc"], 0, 1, nm, ntq, t["esmr"], 1 / 8, t["ua"], t["x"], t["wx"], t["expa"])
+    scale = np.abs(wg).sum(0).max() * np.linalg.norm(t["zmel"]) ** 2 * max(np.linalg.norm(x, 2) for x in
+                                                                          wi.transpose(2, 0, 1))
+    assert np.linalg.norm(got - ref) <= 2 * (ns + 2) * PEAK * 2.0 ** (1 - 8 * ns) * scale
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 65])
+def test_packed_w_equals_full_w(qsgw, n):
+    """Packed upper triangles are unpacked to the matrices they came from (Hermitian, real diagonal)."""
+    t = synth.sigc_task(n, 3, 12, 5, 30, seed=n, esmr=0.02, ef=0.05)
+    rng = np.random.default_rng(n)
+    herm = lambda k: np.asfortranarray((lambda w: w + w.conj().transpose(1, 0, 2))(_rc(rng, n, n, k)))
+    wi, wr = herm(6), herm(30)
+    full = _sigma(qsgw, t, wi, wr, n, 12, 3)
+    packed = _sigma(qsgw, t, wi, wr, n, 12, 3, keepwv=True)
+    assert np.linalg.norm(full - packed) <= 1e-13 * np.linalg.norm(full)
