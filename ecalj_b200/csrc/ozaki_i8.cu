@@ -334,9 +334,16 @@ __global__ void __launch_bounds__(THREADS, 1)
   // the row tiles of a column tile adjacent; the paired launch covers the last row tile only
   const int mt = PAIRED ? p.T - 1 : blockIdx.x % p.ntm, nt = PAIRED ? blockIdx.x : blockIdx.x / p.ntm;
   const int group = p.tile_group[nt];
-  const int nseg = p.group_nseg[group];
-  const int seg0 = p.group_seg_off[group];
+  int nseg = p.group_nseg[group];
+  int seg0 = p.group_seg_off[group];
   constexpr bool paired = PAIRED;
+  if (gridDim.y > 1) {                                // this CTA's share of the segments (or segment pairs)
+    const int steps = paired ? (nseg + 1) / 2 : nseg;
+    const int per = (steps + gridDim.y - 1) / gridDim.y, b = blockIdx.y * per * (paired ? 2 : 1);
+    if (b >= nseg) return;
+    seg0 += b;
+    nseg = min(nseg - b, per * (paired ? 2 : 1));
+  }
   const int nstep = paired ? (nseg + 1) / 2 : nseg;   // accumulation periods: segments or segment pairs
   const int nchunk = nstep * p.cps;
 
@@ -527,7 +534,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int col = p.tile_cols[rtile + j];
-            if (col >= 0) reinterpret_cast<double*>(C + m + static_cast<long long>(col) * p.ldc)[part] = acc[j];
+            if (col < 0) continue;
+            double* dst = reinterpret_cast<double*>(C + m + static_cast<long long>(col) * p.ldc) + part;
+            if (gridDim.y > 1) atomicAdd(dst, acc[j]);
+            else *dst = acc[j];
           }
         }
       }
@@ -1174,6 +1184,21 @@ int rel_diff_fro(const double2* a, const double2* b, long long n, cudaStream_t s
 static DevBuf g_cols;                                   // Sigma_c column map of every tile of a batch
 static DevBuf g_t8;                                     // Sigma_c half-height tail slices (paired tail)
 
+// CTAs per tile of the Sigma_c contraction: `steps` segments of cps chunks each, one CTA an SM.  The waves
+// are counted in chunk times; a CTA's start and end (TMEM, pipeline fill, output) cost about 16 of them.
+// One CTA a tile leaves a last wave of few CTAs that run through all segments: 29 tiles of the paired last
+// row of 350 took 218 us beside 453 us for the other 145.
+static int seg_split(long long ctas, int steps, int cps) {
+  const int sms = ctx().sm_count;
+  int best = 1;
+  double tbest = 0.0;
+  for (int sp = 1; sp <= std::min(steps, 64); ++sp) {
+    const double t = static_cast<double>((ctas * sp + sms - 1) / sms) * ((steps + sp - 1) / sp * cps + 16);
+    if (sp == 1 || t < 0.97 * tbest) { best = sp; tbest = t; }
+  }
+  return best;
+}
+
 // the last row tile runs segment pairs when it has at most 32 valid rows
 static bool paired_tail(int M) { return M % 64 != 0 && M % 64 <= 32; }
 
@@ -1199,7 +1224,7 @@ int OzSigcBatch::reserve(int ns, int ngb, int mrows, long long ldc, long long ns
   cap_slot_ = nslot; cap_tiles_ = ntiles;
   nslot_ = 0; ntiles_ = 0;
   tile_group_.clear(); group_seg_off_.clear(); group_nseg_.clear(); seg_slot_.clear();
-  segs_.clear(); tile_out_.clear();
+  segs_.clear(); tile_out_.clear(); outs_.clear();
   int rc = g_a8.ensure(static_cast<size_t>(ns) * nslot * T * 128 * Kp);
   if (rc) return rc;
   if ((rc = g_b8.ensure(static_cast<size_t>(ns) * ntiles * BN * Kp))) return rc;
@@ -1310,6 +1335,7 @@ int OzSigcBatch::add(const SigcSplitArgs& a, cudaStream_t s) {
     tile_group_.push_back(g0 + a.tile_group[t]);
     tile_out_.push_back(a.out);
   }
+  outs_.push_back({a.out, a.ncol});
   nslot_ += nslot;
   ntiles_ += ntiles;
   return QSGW_OK;
@@ -1386,11 +1412,20 @@ int OzSigcBatch::launch(cudaStream_t s) {
   p.ntm = tmain;
   const long long nt_all = ntiles_;
   nslot_ = 0; ntiles_ = 0; cap_slot_ = 0; cap_tiles_ = 0;      // the next batch starts with reserve()
+  // segments of a tile over several CTAs where the tiles leave SMs idle
+  const int steps = static_cast<int>(segs_.size() / std::max<size_t>(group_nseg_.size(), 1));
+  const int smain = tmain > 0 ? seg_split(tmain * nt_all, steps, p.cps) : 1;
+  const int stail = tail ? seg_split(nt_all, (steps + 1) / 2, p.cps) : 1;
+  if (smain > 1 || stail > 1) {
+    for (const auto& o : outs_)
+      QSGW_CUDA(cudaMemset2DAsync(o.first, static_cast<size_t>(ldc_) * sizeof(double2), 0,
+                                  static_cast<size_t>(M_) * sizeof(double2), static_cast<size_t>(o.second), s));
+  }
   auto run = [&](auto nsc) -> int {
     constexpr int NSV = decltype(nsc)::value;
     int r = QSGW_OK;
-    if (tmain > 0) r = launch_seg<NSV, false>(ma, mb, mt, p, dim3(static_cast<unsigned>(tmain * nt_all)), s);
-    if (!r && tail) r = launch_seg<NSV, true>(ma, mb, mt, p, dim3(static_cast<unsigned>(nt_all)), s);
+    if (tmain > 0) r = launch_seg<NSV, false>(ma, mb, mt, p, dim3(static_cast<unsigned>(tmain * nt_all), smain), s);
+    if (!r && tail) r = launch_seg<NSV, true>(ma, mb, mt, p, dim3(static_cast<unsigned>(nt_all), stail), s);
     return r;
   };
   if (ns == 2) return run(std::integral_constant<int, 2>());

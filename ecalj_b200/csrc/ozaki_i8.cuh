@@ -2,6 +2,7 @@
 // accumulation): the Sigma_c segmented product and the binned chi0 rank-k
 // update.  ozaki_i8.cu holds the kernels and the scheme.
 #pragma once
+#include <utility>
 #include <vector>
 #include "split_f16.cuh"
 
@@ -20,7 +21,8 @@ int sigc_split_i8(const SigcSplitArgs& a, int ns, cudaStream_t s);
 // add() slices one task into them on stream s -- its W records and zmel may be overwritten by
 // work enqueued after add(), its weight tables (the ZSeg scales) and output must stay valid until
 // launch(); launch() runs the tiles of every added task, task after task, and ends the batch.
-// The outputs are those of one sigc_split_i8 call per task, bit for bit.  One batch at a time
+// The outputs are those of one sigc_split_i8 call per task up to the order of the FP64 sums over the
+// segments (few tiles split them over several CTAs).  One batch at a time
 // (the slice buffers are the library's).
 class OzSigcBatch {
  public:
@@ -36,6 +38,7 @@ class OzSigcBatch {
   std::vector<int> tile_group_, group_seg_off_, group_nseg_, seg_slot_;
   std::vector<ZSeg> segs_;
   std::vector<double2*> tile_out_;
+  std::vector<std::pair<double2*, long long>> outs_;    // every task's output and its columns
 };
 
 // Binned chi0 rank-k update:
