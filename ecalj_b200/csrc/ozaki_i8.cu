@@ -1,6 +1,6 @@
 // Ozaki-scheme complex contractions on the 5th-generation tensor cores: int8
 // slices, tcgen05.mma kind::i8 with exact INT32 accumulation in TMEM, operands
-// streamed by TMA into 64-byte-swizzled shared memory.
+// streamed by TMA into swizzled shared memory.
 //
 // Why int8.  The FP32 accumulation of tcgen05 kind::f16 truncates: the split
 // FP16 path carries a bias that grows with the accumulation length (about 4e-8
@@ -89,28 +89,26 @@ struct Cfg {
   static_assert(NS * BN <= static_cast<int>(TMEM8), "one TMEM accumulator per level");
 };
 
-// The Sigma_c kernel's shared memory: NBUF chunk buffers (NS A' slices and NS B slices of one
-// 64-byte K chunk each), grouped into NST stages of CPS consecutive chunks.  A stage is one
-// full/empty barrier pair: the producer fills its CPS chunks under one expected byte count and the
-// MMA thread waits for it and releases it once, so the fixed cost of a stage (barrier test or
-// wait, commit, TMA bookkeeping) is paid once per CPS chunks.  Two chunks a stage up to 3 slices
-// (3 stages of 64 KB at 2, 2 stages of 96 KB at 3), one at 4 slices (3 stages of 64 KB).
+// The Sigma_c kernel's shared memory: NST stages of one K chunk, NS A' slices and NS B slices each.  Up to 3
+// slices a chunk is 128 bytes of K (128-byte swizzled rows; 3 stages of 64 KB at 2 slices, 2 of 96 KB at 3),
+// at 4 slices 64 bytes (3 stages of 64 KB): a stage is one full/empty barrier pair, and the TMA unit works
+// through a box row by row, so a row of 128 bytes costs it half the rows of two boxes of 64.
 template <int NS>
 struct SegCfg {
-  static constexpr int CPS = NS <= 3 ? 2 : 1;
-  static constexpr int CHUNK = NS * (SLA8 + SLB8);
-  static constexpr int NBUF = STAGE_BUDGET / CHUNK / CPS * CPS;   // 6, 4, 3 chunk buffers for NS = 2, 3, 4
-  static constexpr int NST = NBUF / CPS;                          // 3, 2, 3 stages
-  static constexpr int OFF_A = 0;                                 // [NBUF][NS] A' slices
-  static constexpr int OFF_B = OFF_A + NBUF * NS * SLA8;          // [NBUF][NS] B slices
-  static constexpr int OFF_W = OFF_B + NBUF * NS * SLB8;          // drain column factors [16][2][32]
+  static constexpr int KB = NS <= 3 ? 128 : 64;                   // bytes of K per chunk
+  static constexpr int SLA = BM * KB, SLB = BN * KB;              // one slice of the A' / B tile of a stage
+  static constexpr int STAGE = NS * (SLA + SLB);
+  static constexpr int NST = STAGE_BUDGET / STAGE;                // 3, 2, 3 stages for NS = 2, 3, 4
+  static constexpr int OFF_A = 0;                                 // [NST][NS] A' slices
+  static constexpr int OFF_B = OFF_A + NST * NS * SLA;            // [NST][NS] B slices
+  static constexpr int OFF_W = OFF_B + NST * NS * SLB;            // drain column factors [16][2][32]
   static constexpr int OFF_BAR = OFF_W + NDW * 64 * 8;
   static constexpr int NBAR = 2 * NST + 3;                        // full, empty [NST]; accfull, accempty, done
   static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_MISC + 64 + 1024;
   static_assert(NST >= 2, "a ring of at least two stages");
   static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
-  static_assert(NBUF * NS * SLA8 >= 8 * 32 * 32 * 8, "the paired tail's cross-half sums fit in the A' buffers");
+  static_assert(NST * NS * SLA >= 8 * 32 * 32 * 8, "the paired tail's cross-half sums fit in the A' buffers");
 };
 
 // kind::i8, A = B = signed 8-bit, D = S32, both K-major, M = 128, N = BN
@@ -288,7 +286,8 @@ __device__ __forceinline__ double w_extent(const double* wr, int b, double sign)
 struct SegParams {
   int M;                      // complex rows (ngb)
   int ntm;                    // 64-row tiles
-  int cps;                    // chunks per segment
+  int cps;                    // K chunks per segment
+  int klast;                  // 32-byte K steps of a segment's last chunk
   int nslot, T;               // A' tile coordinate (q nslot + slot) T + mt
   int nrows;                  // B rows per slice (tile-ordered columns)
   const int* tile_group;
@@ -315,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     oz_seg_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                   const __grid_constant__ CUtensorMap mapT, const SegParams p) {
   using L = SegCfg<NS>;
-  constexpr int NST = L::NST, CPS = L::CPS;
+  constexpr int NST = L::NST, KB = L::KB, SLA = L::SLA, SLB = L::SLB;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char* sA = sm + L::OFF_A;
@@ -368,8 +367,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (nchunk > 0) {
     if (warp == 0 && lane == 0) {
       // ---------------- TMA producer: NS slices of the segment's A' tile and of the B tile
-      constexpr uint32_t bytes = NS * (SLA8 + SLB8);
-      int issued = 0, sg = 0, cin = 0, st = 0, ph = 0, sub = 0;   // issued: stages begun
+      constexpr uint32_t bytes = NS * (SLA + SLB);     // rows beyond the slices' K extent arrive as zeros
+      int issued = 0, sg = 0, cin = 0, st = 0, ph = 0;
       // this step's slot (paired: the slots of segments 2 sg and 2 sg + 1, the second repeated when absent)
       auto step_slots = [&](int g, int& s0, int& s1) {
         if (!paired) { s0 = s1 = p.seg_slot[seg0 + g]; return; }
@@ -379,67 +378,61 @@ __global__ void __launch_bounds__(THREADS, 1)
       int slot = 0, slot1 = 0;
       step_slots(0, slot, slot1);
       for (int c = 0; c < nchunk; ++c) {
-        if (sub == 0) {                               // a new stage: its CPS chunks (fewer at the end)
-          if (issued >= NST && !mbar_wait(&empty[st], ph ^ 1, abort_flag)) break;
-          ++issued;
-          mbar_expect_tx(&full[st], bytes * static_cast<uint32_t>(min(CPS, nchunk - c)));
-        }
-        const int buf = st * CPS + sub;
-        const int x = cin * K8;
+        if (c >= NST && !mbar_wait(&empty[st], ph ^ 1, abort_flag)) break;
+        issued = c + 1;
+        mbar_expect_tx(&full[st], bytes);
+        const int x = cin * KB;
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
-          unsigned char* dA = sA + (buf * NS + q) * SLA8;
+          unsigned char* dA = sA + (st * NS + q) * SLA;
           if constexpr (PAIRED) {                     // rows 0-31 / 32-63 re, 64-95 / 96-127 im
             tma_load_4d(dA, &mapT, &full[st], x, 0, 0, q * p.nslot + slot);
-            tma_load_4d(dA + SLA8 / 4, &mapT, &full[st], x, 0, 0, q * p.nslot + slot1);
-            tma_load_4d(dA + SLA8 / 2, &mapT, &full[st], x, 0, 1, q * p.nslot + slot);
-            tma_load_4d(dA + 3 * SLA8 / 4, &mapT, &full[st], x, 0, 1, q * p.nslot + slot1);
+            tma_load_4d(dA + SLA / 4, &mapT, &full[st], x, 0, 0, q * p.nslot + slot1);
+            tma_load_4d(dA + SLA / 2, &mapT, &full[st], x, 0, 1, q * p.nslot + slot);
+            tma_load_4d(dA + 3 * SLA / 4, &mapT, &full[st], x, 0, 1, q * p.nslot + slot1);
           } else {
             tma_load_4d(dA, &mapA, &full[st], x, 0, 0, (q * p.nslot + slot) * p.T + mt);
           }
-          tma_load_3d(sB + (buf * NS + q) * SLB8, &mapB, &full[st], x, nt * BN, q);
+          tma_load_3d(sB + (st * NS + q) * SLB, &mapB, &full[st], x, nt * BN, q);
         }
         if (++cin == p.cps) {
           cin = 0;
           if (++sg < nstep) step_slots(sg, slot, slot1);
         }
-        if (++sub == CPS) {
-          sub = 0;
-          if (++st == NST) { st = 0; ph ^= 1; }
-        }
+        if (++st == NST) { st = 0; ph ^= 1; }
       }
       for (int g = max(0, issued - NST); g < issued; ++g) mbar_drain(&full[g % NST], (g / NST) & 1);
     } else if (warp == 1 && lane == 0) {
       // ---------------- MMA issuer: NS level accumulators, one accumulation period per segment
-      const uint64_t dA0 = sw64_desc(smem_u32(sA)), dB0 = sw64_desc(smem_u32(sB));
-      int seg = 0, cin = 0, st = 0, ph = 0, sub = 0;
+      const uint64_t dA0 = KB == 128 ? sw128_desc(smem_u32(sA)) : sw64_desc(smem_u32(sA));
+      const uint64_t dB0 = KB == 128 ? sw128_desc(smem_u32(sB)) : sw64_desc(smem_u32(sB));
+      int seg = 0, cin = 0, st = 0, ph = 0;
       uint32_t ready = 0;                            // the next stage was seen full by the last test
       for (int c = 0; c < nchunk && !*abort_flag; ++c) {
         const bool first = cin == 0, last = cin == p.cps - 1;
-        const bool stage_end = sub == CPS - 1 || c + 1 == nchunk;
         if (first && seg >= 1 && !mbar_wait(accempty, (seg - 1) & 1, abort_flag)) break;
-        if (sub == 0 && !ready && !mbar_wait(&full[st], ph, abort_flag)) break;
+        if (!ready && !mbar_wait(&full[st], ph, abort_flag)) break;
         tc_fence_after();
-        // the next stage is tested during the last MMA of this stage's last chunk
-        const uint32_t nbar = stage_end && c + 1 < nchunk ? smem_u32(&full[st + 1 == NST ? 0 : st + 1]) : 0u;
+        // the next stage is tested during the last MMA of this one
+        const uint32_t nbar = c + 1 < nchunk ? smem_u32(&full[st + 1 == NST ? 0 : st + 1]) : 0u;
         const uint32_t npar = st + 1 == NST ? (ph ^ 1) : ph;
-        const int buf = st * CPS + sub;
+        const uint64_t dA = dA0 + static_cast<uint32_t>((st * NS * SLA) >> 4), dB = dB0 + static_cast<uint32_t>((st * NS * SLB) >> 4);
+        // 32 int8 = 32 B along K = 2 descriptor units; the step count is a constant in the loop that matters (a
+        // run-time one cost 5 % of the contraction)
+        auto steps = [&](auto nk) -> uint32_t {
+          constexpr int N = decltype(nk)::value;
+          uint32_t r = 0u;
 #pragma unroll
-        for (int kk = 0; kk < K8 / 32; ++kk) {        // 32 int8 = 32 B along K = 2 descriptor units
-          const uint32_t r = slice_products<NS>(tmem, dA0 + static_cast<uint32_t>((buf * NS * SLA8) >> 4) + 2 * kk,
-                                                dB0 + static_cast<uint32_t>((buf * NS * SLB8) >> 4) + 2 * kk,
-                                                SLA8 >> 4, SLB8 >> 4, first && kk == 0,
-                                                kk == K8 / 32 - 1 ? nbar : 0u, npar);
-          if (kk == K8 / 32 - 1) ready = nbar ? r : 0u;
-        }
+          for (int kk = 0; kk < N; ++kk)
+            r = slice_products<NS>(tmem, dA + 2 * kk, dB + 2 * kk, SLA >> 4, SLB >> 4, first && kk == 0,
+                                   kk == N - 1 ? nbar : 0u, npar);
+          return nbar ? r : 0u;
+        };
+        if (KB == 64 || !last || p.klast == KB / 32) ready = steps(std::integral_constant<int, KB / 32>());
+        else ready = steps(std::integral_constant<int, KB / 64>());   // half a chunk: the K extent is a multiple of 64
         if (last) umma_commit(accfull);
-        if (stage_end) {
-          umma_commit(&empty[st]);
-          sub = 0;
-          if (++st == NST) { st = 0; ph ^= 1; }
-        } else {
-          ++sub;
-        }
+        umma_commit(&empty[st]);
+        if (++st == NST) { st = 0; ph ^= 1; }
         if (++cin == p.cps) { cin = 0; ++seg; }
       }
       umma_commit(done);
@@ -1184,7 +1177,7 @@ int rel_diff_fro(const double2* a, const double2* b, long long n, cudaStream_t s
 static DevBuf g_cols;                                   // Sigma_c column map of every tile of a batch
 static DevBuf g_t8;                                     // Sigma_c half-height tail slices (paired tail)
 
-// CTAs per tile of the Sigma_c contraction: `steps` segments of cps chunks each, one CTA an SM.  The waves
+// CTAs per tile of the Sigma_c contraction: `steps` segments of cps 64-byte chunks each, one CTA an SM.  The waves
 // are counted in chunk times; a CTA's start and end (TMEM, pipeline fill, output) cost about 16 of them.
 // One CTA a tile leaves a last wave of few CTAs that run through all segments: 29 tiles of the paired last
 // row of 350 took 218 us beside 453 us for the other 145.
@@ -1365,25 +1358,28 @@ int OzSigcBatch::launch(cudaStream_t s) {
   p.seg_slot = reinterpret_cast<const int*>(put(seg_slot_.data(), seg_slot_.size() * sizeof(int)));
   if (cprc) return cprc;
   const long long nrows = cap_tiles_ * BN;
-  // maps: A' [Kp, 64, 2, ns * cap_slot * T] box {64, 64, 2, 1}; B [Kp, cap_rows, ns] box {64, 128, 1}
+  // maps: A' [Kp, 64, 2, ns * cap_slot * T] box {kb, 64, 2, 1}; B [Kp, cap_rows, ns] box {kb, 128, 1}
+  const cuuint32_t kb = ns <= 3 ? SegCfg<3>::KB : SegCfg<4>::KB;       // bytes of K per chunk
+  static_assert(SegCfg<2>::KB == SegCfg<3>::KB, "one chunk width up to 3 slices");
+  const CUtensorMapSwizzle swz = kb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   CUtensorMap ma, mb;
   {
     const cuuint64_t dims[4] = {static_cast<cuuint64_t>(Kp), 64, 2, static_cast<cuuint64_t>(ns) * cap_slot_ * T};
     const cuuint64_t str[3] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(Kp) * 64,
                                static_cast<cuuint64_t>(Kp) * 128};
-    const cuuint32_t box[4] = {K8, 64, 2, 1};
-    rc = make_tensor_map(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_a8.p, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    const cuuint32_t box[4] = {kb, 64, 2, 1};
+    rc = make_tensor_map(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_a8.p, 4, dims, str, box, swz);
     if (rc) return rc;
   }
   {
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(nrows),
                                 static_cast<cuuint64_t>(ns)};
     const cuuint64_t str[2] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(Kp) * nrows};
-    const cuuint32_t box[3] = {K8, BN, 1};
-    rc = make_tensor_map(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_b8.p, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    const cuuint32_t box[3] = {kb, BN, 1};
+    rc = make_tensor_map(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_b8.p, 3, dims, str, box, swz);
     if (rc) return rc;
   }
-  // paired tail: T8 [Kp, 32, 2, ns * cap_slot] box {64, 32, 1, 1} (one half of one slot's tail rows);
+  // paired tail: T8 [Kp, 32, 2, ns * cap_slot] box {kb, 32, 1, 1} (one half of one slot's tail rows);
   // without it the map is a copy of A's and never read
   CUtensorMap mt = ma;
   const bool tail = paired_tail(M_);
@@ -1391,14 +1387,15 @@ int OzSigcBatch::launch(cudaStream_t s) {
     const cuuint64_t dims[4] = {static_cast<cuuint64_t>(Kp), 32, 2, static_cast<cuuint64_t>(ns) * cap_slot_};
     const cuuint64_t str[3] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(Kp) * 32,
                                static_cast<cuuint64_t>(Kp) * 64};
-    const cuuint32_t box[4] = {K8, 32, 1, 1};
-    rc = make_tensor_map(&mt, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_t8.p, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    const cuuint32_t box[4] = {kb, 32, 1, 1};
+    rc = make_tensor_map(&mt, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_t8.p, 4, dims, str, box, swz);
     if (rc) return rc;
   }
   p.tail = tail ? 1 : 0;
   p.M = M_;
   p.ntm = T;
-  p.cps = Kp / K8;
+  p.cps = (Kp + static_cast<int>(kb) - 1) / static_cast<int>(kb);
+  p.klast = (Kp - (p.cps - 1) * static_cast<int>(kb)) / 32;
   p.nslot = static_cast<int>(cap_slot_);
   p.T = T;
   p.nrows = static_cast<int>(nrows);
@@ -1414,8 +1411,8 @@ int OzSigcBatch::launch(cudaStream_t s) {
   nslot_ = 0; ntiles_ = 0; cap_slot_ = 0; cap_tiles_ = 0;      // the next batch starts with reserve()
   // segments of a tile over several CTAs where the tiles leave SMs idle
   const int steps = static_cast<int>(segs_.size() / std::max<size_t>(group_nseg_.size(), 1));
-  const int smain = tmain > 0 ? seg_split(tmain * nt_all, steps, p.cps) : 1;
-  const int stail = tail ? seg_split(nt_all, (steps + 1) / 2, p.cps) : 1;
+  const int smain = tmain > 0 ? seg_split(tmain * nt_all, steps, Kp / K8) : 1;
+  const int stail = tail ? seg_split(nt_all, (steps + 1) / 2, Kp / K8) : 1;
   if (smain > 1 || stail > 1) {
     for (const auto& o : outs_)
       QSGW_CUDA(cudaMemset2DAsync(o.first, static_cast<size_t>(ldc_) * sizeof(double2), 0,
