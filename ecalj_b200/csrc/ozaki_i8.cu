@@ -22,9 +22,7 @@
 // and scales v by mu_row nu_col 2^-(12 + 7 (NS - 1)) in FP64.  A level holds at
 // most NS products of |s| <= 64 over K' real K, so |acc| < NS 2^12 K', which
 // bounds K' between drains (INT32).  These base-128 digits are the chi0
-// kernel's: symmetric, so negation commutes with the slicing (rint is
-// symmetric) and the slices of -x are the negated slices of x, which the chi0
-// kernel uses to build rows in shared memory.
+// kernel's.
 //
 // The Sigma_c kernel (also behind the zmel M -> E product) slices every
 // operand in HBM, negated parts included, and so uses base-256 digits over the
@@ -35,16 +33,16 @@
 // hold 23 bits, four base-128 ones 27: six slice products instead of ten for
 // an error within the QP-energy target.  |acc| < NS 2^14 K'.
 //
-// A complex product C = A B is one real GEMM with M doubled and K interleaved
-// (k' = 2k + {re, im}): rows (m, re) of A' = [Re a, -Im a], rows (m, im) =
-// [Im a, Re a], B' row n = [Re b, Im b]; lanes 0..63 of an accumulator hold
-// Re C, 64..127 Im C.
+// Sigma_c: a complex product C = A B is one real GEMM with M doubled and K
+// interleaved (k' = 2k + {re, im}): rows (m, re) of A' = [Re a, -Im a], rows
+// (m, im) = [Im a, Re a], B' row n = [Re b, Im b]; lanes 0..63 of an
+// accumulator hold Re C, 64..127 Im C.  chi0 keeps real and imaginary parts
+// as separate rows of both operands (oz_herk_kernel).
 //
 // Kernels (576 threads, one CTA per SM):
 //     warp 0        TMA producer
 //     warp 1        TMEM owner and MMA issuer (one thread)
-//     warps 2..17   drain (chi0: they also build the (m, im) rows of A' from
-//                   the (m, re) rows in shared memory, a byte shuffle)
+//     warps 2..17   drain
 // Every mbarrier wait is bounded; on time-out the CTA records an error, waits
 // (bounded) for its own TMA and MMA work, frees TMEM and exits.
 #include <algorithm>
@@ -66,28 +64,8 @@ constexpr int BN = kOzTileN;             // accumulator columns (UMMA N)
 constexpr int K8 = 64;                   // int8 K per chunk: one 64-byte swizzled row
 constexpr int THREADS = 576;
 constexpr int NDW = 16;                  // drain warps 2..17
-constexpr int NCONV = 12;                // chi0: the drain warps that also convert (warp mod 4 != 1)
-constexpr int SLA8 = BM * K8;         // 8 KB: one slice of the A' tile of a stage
-constexpr int SLB8 = BN * K8;         // 8 KB: one slice of the B tile of a stage
 constexpr int STAGE_BUDGET = 192 * 1024;
 constexpr uint32_t TMEM8 = 512;
-
-template <int NS>
-struct Cfg {
-  static constexpr int STAGE = NS * (SLA8 + SLB8);
-  static constexpr int NST = STAGE_BUDGET / STAGE;                // 6, 4, 3 stages for NS = 2, 3, 4
-  static constexpr int OFF_A = 0;                                 // [NST][NS] A' slices
-  static constexpr int OFF_B = OFF_A + NST * NS * SLA8;        // [NST][NS] B slices
-  static constexpr int OFF_W = OFF_B + NST * NS * SLB8;        // drain column factors [16][2][32]
-  static constexpr int OFF_BAR = OFF_W + NDW * 64 * 8;
-  static constexpr int NBAR = 3 * NST + 3;                        // full, cfull, empty [NST]; accfull, accempty, done
-  static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;
-  static constexpr int SMEM = OFF_MISC + 64 + 1024;               // + slack for the 1024-byte alignment
-  // exact INT32 levels: at most NS products of |s| <= 64 per K element
-  static constexpr int MAX_PERIOD = static_cast<int>((1LL << 30) / (NS * 4096LL * K8));
-  static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
-  static_assert(NS * BN <= static_cast<int>(TMEM8), "one TMEM accumulator per level");
-};
 
 // The Sigma_c kernel's shared memory: NST stages of one K chunk, NS A' slices and NS B slices each.  Up to 3
 // slices a chunk is 128 bytes of K (128-byte swizzled rows; 3 stages of 64 KB at 2 slices, 2 of 96 KB at 3),
@@ -111,19 +89,34 @@ struct SegCfg {
   static_assert(NST * NS * SLA >= 8 * 32 * 32 * 8, "the paired tail's cross-half sums fit in the A' buffers");
 };
 
-// kind::i8, A = B = signed 8-bit, D = S32, both K-major, M = 128, N = BN
-constexpr uint32_t idesc_i8(int n) {
-  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-         (static_cast<uint32_t>(BM >> 4) << 24);
-}
-constexpr uint32_t IDESC_I8 = idesc_i8(BN);
+// The chi0 kernel's: stages of one chunk of KB pairs, a tile being 128 rows of KB bytes (64 rows of Re y,
+// then 64 of Im y).
+template <int NS>
+struct HerkCfg {
+  static constexpr int KB = NS <= 3 ? 128 : 64;                   // pairs (bytes of a row) per chunk
+  static constexpr int SL = BM * KB;                              // one slice of a tile
+  static constexpr int NST = STAGE_BUDGET / (2 * NS * SL);        // 3, 2, 3 stages for NS = 2, 3, 4
+  static constexpr int OFF_A = 0;                                 // [NST][NS] A slices
+  static constexpr int OFF_B = OFF_A + NST * NS * SL;             // [NST][NS] B slices
+  static constexpr int OFF_BAR = OFF_B + NST * NS * SL;
+  static constexpr int NBAR = 2 * NST + 3;                        // full, empty [NST]; accfull, accempty, done
+  static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;
+  static constexpr int SMEM = OFF_MISC + 64 + 1024;               // + slack for the 1024-byte alignment
+  // exact INT32 levels: at most NS products of |s| <= 64 per pair
+  static constexpr int MAX_PERIOD = static_cast<int>((1LL << 30) / (NS * 4096LL * KB));
+  static_assert(NST >= 2, "a ring of at least two stages");
+  static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
+  static_assert(NS * BN <= static_cast<int>(TMEM8), "one TMEM accumulator per level");
+};
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
-                                        uint32_t idesc) {
+// kind::i8, A = B = signed 8-bit, D = S32, both K-major, M = 128, N = BN
+constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
+                              (static_cast<uint32_t>(BM >> 4) << 24);
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
 }
 // The MMA above preceded by a non-blocking test (mbarrier.test_wait, acquire) of phase `parity` of
 // the barrier at shared address `bar`, whose answer (1 = complete) is read only after the MMA has
@@ -131,7 +124,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 // wait between two K chunks leaves the tensor core idle; the test's latency is spent inside the
 // MMA issue instead.
 __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
-                                                      uint32_t bar, uint32_t parity, uint32_t idesc) {
+                                                      uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n .reg .pred p, q;\n"
@@ -140,7 +133,7 @@ __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t 
       " tcgen05.mma.cta_group::1.kind::i8 [%1], %2, %3, %7, p;\n"
       " selp.u32 %0, 1, 0, q;\n}\n"
       : "=r"(ok)
-      : "r"(tmem_d), "l"(da), "l"(db), "r"(accumulate), "r"(bar), "r"(parity), "r"(idesc)
+      : "r"(tmem_d), "l"(da), "l"(db), "r"(accumulate), "r"(bar), "r"(parity), "r"(IDESC_I8)
       : "memory");
   return ok;
 }
@@ -148,23 +141,22 @@ __device__ __forceinline__ uint32_t umma_i8_then_test(uint32_t tmem_d, uint64_t 
 // keeps it, USE reads the kept copy (same A descriptor), LAST reads it and releases the buffer.
 enum { A_FILL = 0, A_USE = 1, A_LAST = 2 };
 template <int MODE>
-__device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate,
-                                           uint32_t idesc) {
+__device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
   if (MODE == A_FILL)
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::fill [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
   else if (MODE == A_USE)
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::use [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
   else
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8.collector::a::lastuse [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate));
 }
 
 // The slice products of one K step: for each A slice pa (one shared-memory read through the
@@ -175,7 +167,7 @@ __device__ __forceinline__ void umma_i8_ca(uint32_t tmem_d, uint64_t da, uint64_
 template <int NS>
 __device__ __forceinline__ uint32_t slice_products(uint32_t tmem, uint64_t da0, uint64_t db0, uint32_t a_step,
                                                    uint32_t b_step, bool start, uint32_t test_bar = 0,
-                                                   uint32_t test_parity = 0, uint32_t idesc = IDESC_I8) {
+                                                   uint32_t test_parity = 0) {
   uint32_t ready = 0;
 #pragma unroll
   for (int pa = 0; pa < NS; ++pa) {
@@ -186,12 +178,12 @@ __device__ __forceinline__ uint32_t slice_products(uint32_t tmem, uint64_t da0, 
       const uint32_t d = tmem + static_cast<uint32_t>((pa + qb) * kOzTileN);
       const uint32_t acc = (start && pa == 0) ? 0u : 1u;
       if (NS - pa == 1) {
-        if (test_bar) ready = umma_i8_then_test(d, da, db, acc, test_bar, test_parity, idesc);
-        else umma_i8(d, da, db, acc, idesc);
+        if (test_bar) ready = umma_i8_then_test(d, da, db, acc, test_bar, test_parity);
+        else umma_i8(d, da, db, acc);
       }
-      else if (qb == 0) umma_i8_ca<A_FILL>(d, da, db, acc, idesc);
-      else if (qb == NS - pa - 1) umma_i8_ca<A_LAST>(d, da, db, acc, idesc);
-      else umma_i8_ca<A_USE>(d, da, db, acc, idesc);
+      else if (qb == 0) umma_i8_ca<A_FILL>(d, da, db, acc);
+      else if (qb == NS - pa - 1) umma_i8_ca<A_LAST>(d, da, db, acc);
+      else umma_i8_ca<A_USE>(d, da, db, acc);
     }
   }
   return ready;
@@ -270,12 +262,6 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
   const uint32_t cd = __byte_perm(static_cast<uint32_t>(c), static_cast<uint32_t>(d), 0x0040);
   return __byte_perm(ab, cd, 0x5410);
 }
-// (re, im) byte pairs -> (-im, re): the (m, im) row of A' from its (m, re) row
-__device__ __forceinline__ uint32_t rotate_pairs(uint32_t w) {
-  const uint32_t sw = __byte_perm(w, 0, 0x2301);           // [im0, re0, im1, re1]
-  return (__vneg4(sw) & 0x00FF00FFu) | (sw & 0xFF00FF00u);
-}
-
 // the extent of the chi0 weights of sign `sign` in bin b (0: the pass has nothing to do there)
 __device__ __forceinline__ double w_extent(const double* wr, int b, double sign) {
   return sign < 0.0 ? wr[2 * b] : wr[2 * b + 1];
@@ -547,17 +533,23 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 // =====================================================================================
-// chi0: C(:, :, slab_b) += sign sum_{e in bin b} conj(y_e(0:M)) y_e(row_b0 : row_b0 + N)^T,
-// y_e = sqrt(sign w_e) z_col(e) sliced in HBM as Y8[slice][row][K'] (the (m, re) rows of A' and
-// the rows of B are both rows of Y8; the (m, im) rows are rotated from them in shared memory)
+// chi0: C(:, :, slab_b) += sign sum_{e in bin b} conj(y_e(0:M)) y_e(row_b0 : row_b0 + N)^T, y_e = sqrt(sign w_e)
+// z_col(e) sliced in HBM, real and imaginary parts apart: Y8[chunk][slice][re, im][row][KB pairs].  A tile of
+// 64 rows is the 128 rows [Re y; Im y], and ONE real product of two tiles holds all of a complex 64 x 64 block
+// in its quadrants:
+//   Re C = Re.Re + Im.Im,   Im C = Re.Im - Im.Re
+// added as 64-bit integers at the end.  Nothing is built in shared memory between TMA and MMA (interleaved
+// pairs needed the rows [-Im, Re], which twelve warps rotated there, and 64-byte rows, which cost the TMA unit
+// twice the rows for the same bytes), and the tiles on the diagonal load one operand for both.
 struct HerkParams {
   int M, N;                   // output rows / columns
   int ntm;                    // 64-row tiles
-  int herm;
+  int herm;                   // M == N, row_b0 == 0: lower tiles only (grid x = triangle), mirrored
   int row_b0;
-  int Rows;                   // rows of Y8 per slice
-  const long long* bin_k0;    // first K chunk of bin b in Y8
-  const int* bin_nch;         // K chunks of bin b
+  int Rows;                   // rows of Y8 per slice and part
+  const long long* bin_k0;    // first chunk of bin b in Y8
+  const int* bin_nch;         // chunks of bin b
+  const int* bin_cnt;         // pairs of bin b
   const int* bin_slab;
   const double* wrange;       // [bin][2]: largest -w and largest w (0 when none)
   const double* mu;           // [bin][Rows] row scales of y
@@ -570,15 +562,14 @@ struct HerkParams {
 
 template <int NS>
 __global__ void __launch_bounds__(THREADS, 1)
-    oz_herk_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                   const HerkParams p) {
-  using L = Cfg<NS>;
-  constexpr int NST = L::NST;
+    oz_herk_kernel(const __grid_constant__ CUtensorMap mapY, const HerkParams p) {
+  using L = HerkCfg<NS>;
+  constexpr int NST = L::NST, KB = L::KB, SL = L::SL;
   constexpr int PER = L::MAX_PERIOD;
-  constexpr int HALF = SLA8 / 2;      // the (m, re) half of an A' slice: 64 rows x 64 B
-  const int mt = blockIdx.x % p.ntm, nt = blockIdx.x / p.ntm;
+  int mt, nt;
+  if (p.herm) tri_decode(blockIdx.x, mt, nt);
+  else { mt = blockIdx.x % p.ntm; nt = blockIdx.x / p.ntm; }
   const int bin = blockIdx.y;
-  if (p.herm && mt * 64 + 63 < nt * BN) return;              // strictly upper tile: mirrored
   if (!(w_extent(p.wrange, bin, p.sign) > 0.0)) return;       // no weight of this sign in the bin
   const int nch = p.bin_nch[bin];
   const int per_split = (nch + gridDim.z - 1) / gridDim.z;
@@ -586,29 +577,27 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int nchunk = min(nch, cbeg + per_split) - cbeg;
   if (nchunk <= 0) return;
   const int kc0 = static_cast<int>(p.bin_k0[bin] + cbeg);    // first chunk of this CTA in Y8
+  // 32-pair K steps of the CTA's last chunk (whole but for the bin's last one)
+  const int klast = cbeg + nchunk < nch ? KB / 32 : (p.bin_cnt[bin] - (nch - 1) * KB + 31) / 32;
+  const bool diag = p.herm && mt == nt;                       // A and B are the same rows
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char* sA = sm + L::OFF_A;
-  unsigned char* sB = sm + L::OFF_B;
+  unsigned char* sB = diag ? sA : sm + L::OFF_B;
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::OFF_BAR);
-  uint64_t* full = bar;                  // [NST] TMA -> converters
-  uint64_t* cfull = bar + NST;           // [NST] converters -> MMA
-  uint64_t* empty = bar + 2 * NST;       // [NST] MMA -> TMA
-  uint64_t* accfull = bar + 3 * NST;
+  uint64_t* full = bar;                  // [NST] TMA -> MMA
+  uint64_t* empty = bar + NST;           // [NST] MMA -> TMA
+  uint64_t* accfull = bar + 2 * NST;
   uint64_t* accempty = accfull + 1;
   uint64_t* done = accempty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L::OFF_MISC + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nper = (nchunk + PER - 1) / PER;
-  // the tile whose 64 rows are the first 64 of its 128 columns: the other columns lie above the diagonal and
-  // come from the mirror, so its MMAs are 64 columns wide
-  const bool half = p.herm && mt * 64 + 63 < nt * BN + 64;
-  const uint32_t idesc = idesc_i8(half ? BN / 2 : BN);
 
   if (tid == 0) {
-    for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&cfull[i], NCONV); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     mbar_init(accfull, 1);
     mbar_init(accempty, NDW);
     mbar_init(done, 1);
@@ -626,8 +615,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer: the (m, re) half of the A' tile and the B tile, NS slices each
-    constexpr uint32_t bytes = NS * (HALF + SLB8);
+    // ---------------- TMA producer: the A tile and (off the diagonal) the B tile, NS slices each
+    const uint32_t bytes = NS * SL * (diag ? 1u : 2u);
     int issued = 0, st = 0, ph = 0;
     for (int c = 0; c < nchunk; ++c) {
       if (c >= NST && !mbar_wait(&empty[st], ph ^ 1, abort_flag)) break;
@@ -635,30 +624,38 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_expect_tx(&full[st], bytes);
 #pragma unroll
       for (int q = 0; q < NS; ++q) {
-        tma_load_4d(sA + (st * NS + q) * SLA8, &mapA, &full[st], 0, mt * 64, q, kc0 + c);
-        tma_load_4d(sB + (st * NS + q) * SLB8, &mapB, &full[st], 0, p.row_b0 + nt * BN, q, kc0 + c);
+        tma_load_4d(sA + (st * NS + q) * SL, &mapY, &full[st], 0, mt * 64, 2 * q, kc0 + c);
+        if (!diag) tma_load_4d(sB + (st * NS + q) * SL, &mapY, &full[st], 0, p.row_b0 + nt * 64, 2 * q, kc0 + c);
       }
       if (++st == NST) { st = 0; ph ^= 1; }
     }
     for (int c = max(0, issued - NST); c < issued; ++c) mbar_drain(&full[c % NST], (c / NST) & 1);
   } else if (warp == 1 && lane == 0) {
     // ---------------- MMA issuer: periods of at most PER chunks (exact INT32 levels)
-    const uint64_t dA0 = sw64_desc(smem_u32(sA)), dB0 = sw64_desc(smem_u32(sB));
+    const uint64_t dA0 = KB == 128 ? sw128_desc(smem_u32(sA)) : sw64_desc(smem_u32(sA));
+    const uint64_t dB0 = KB == 128 ? sw128_desc(smem_u32(sB)) : sw64_desc(smem_u32(sB));
     int st = 0, ph = 0, cin = 0, per = 0;
-    uint32_t ready = 0;                              // the chunk's stage was seen converted by the last test
+    uint32_t ready = 0;                              // the chunk's stage was seen full by the last test
     for (int c = 0; c < nchunk && !*abort_flag; ++c) {
       const bool first = cin == 0;
       const bool last = cin == PER - 1 || c == nchunk - 1;
       if (first && per >= 1 && !mbar_wait(accempty, (per - 1) & 1, abort_flag)) break;
-      if (!ready && !mbar_wait(&cfull[st], ph, abort_flag)) break;
+      if (!ready && !mbar_wait(&full[st], ph, abort_flag)) break;
       tc_fence_after();
-      const uint32_t nbar = c + 1 < nchunk ? smem_u32(&cfull[st + 1 == NST ? 0 : st + 1]) : 0u;
+      const uint32_t nbar = c + 1 < nchunk ? smem_u32(&full[st + 1 == NST ? 0 : st + 1]) : 0u;
       const uint32_t npar = st + 1 == NST ? (ph ^ 1) : ph;
+      const uint64_t dA = dA0 + static_cast<uint32_t>((st * NS * SL) >> 4), dB = dB0 + static_cast<uint32_t>((st * NS * SL) >> 4);
+      if (c + 1 < nchunk || klast == KB / 32) {
 #pragma unroll
-      for (int kk = 0; kk < K8 / 32; ++kk)
-        ready = slice_products<NS>(tmem, dA0 + static_cast<uint32_t>((st * NS * SLA8) >> 4) + 2 * kk,
-                                   dB0 + static_cast<uint32_t>((st * NS * SLB8) >> 4) + 2 * kk, SLA8 >> 4,
-                                   SLB8 >> 4, first && kk == 0, kk == K8 / 32 - 1 ? nbar : 0u, npar, idesc);
+        for (int kk = 0; kk < KB / 32; ++kk)
+          ready = slice_products<NS>(tmem, dA + 2 * kk, dB + 2 * kk, SL >> 4, SL >> 4, first && kk == 0,
+                                     kk == KB / 32 - 1 ? nbar : 0u, npar);
+        if (!nbar) ready = 0;
+      } else {                                       // the bin's last, partly filled chunk
+#pragma unroll 1
+        for (int kk = 0; kk < klast; ++kk)
+          slice_products<NS>(tmem, dA + 2 * kk, dB + 2 * kk, SL >> 4, SL >> 4, first && kk == 0);
+      }
       umma_commit(&empty[st]);
       if (last) umma_commit(accfull);
       if (++st == NST) { st = 0; ph ^= 1; }
@@ -667,51 +664,20 @@ __global__ void __launch_bounds__(THREADS, 1)
     umma_commit(done);
     mbar_drain(done, 0);
   } else if (warp >= 2) {
-    // ---------------- converters + drain (warps 2..17)
-    // The converters are the 12 warps off the MMA warp's sub-partition (warp mod 4 != 1): the
-    // MMA thread blocks in every MMA issue, so issue slots taken from it idle the tensor core.
-    // The other four (they own TMEM lanes 32..63) only drain.
+    // ---------------- drain (warps 2..17): TMEM lanes 32 (warp mod 4) .. +31, 32 columns a warp
     const int dw = warp - 2;
-    const bool conv = (warp & 3) != 1;
-    const int ct = (dw - (dw + 1) / 4) * 32 + lane;      // 0..383 over the converter warps
     const int quad = warp & 3;
     const int c_lo = (dw >> 2) * 32;
-    const int row = quad * 32 + lane;
+    const int row = quad * 32 + lane;                // 0..63 Re y_m, 64..127 Im y_m; columns likewise
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     long long acc[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) acc[j] = 0;
     bool ok = true;
-    int st = 0, ph = 0, cin = 0, per = 0;
-    for (int c = 0; c < nchunk; ++c) {
-      if (conv) {
-        if (!mbar_wait_warp(&full[st], ph, abort_flag)) { ok = false; break; }
-        // the (m, im) rows [-Im y, Re y] from the (m, re) rows [Re y, Im y]: same swizzled offsets
-        // (rows r and r + 64 share their 64-byte swizzle pattern)
-        for (int i = ct; i < NS * (HALF / 16); i += NCONV * 32) {
-          const int q = i / (HALF / 16), j = i % (HALF / 16);
-          const uint4 v = *reinterpret_cast<const uint4*>(sA + (st * NS + q) * SLA8 + j * 16);
-          uint4 o;
-          o.x = rotate_pairs(v.x); o.y = rotate_pairs(v.y); o.z = rotate_pairs(v.z); o.w = rotate_pairs(v.w);
-          *reinterpret_cast<uint4*>(sA + (st * NS + q) * SLA8 + HALF + j * 16) = o;
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&cfull[st]);
-      }
-      if (++st == NST) { st = 0; ph ^= 1; }
-      const bool last = cin == PER - 1 || c == nchunk - 1;
-      if (!last) { ++cin; continue; }
-      cin = 0;
-      // drain the period: exact int64 sums of the combined levels
+    for (int per = 0; per < nper && ok; ++per) {
+      // exact int64 sums of the combined levels
       if (!mbar_wait_warp(accfull, per & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      if (half && c_lo >= BN / 2) {                    // nothing was accumulated there
-        __syncwarp();
-        if (lane == 0) mbar_arrive(accempty);
-        ++per;
-        continue;
-      }
 #pragma unroll
       for (int blk = 0; blk < 8; ++blk) {
         uint32_t v[NS][4];
@@ -732,26 +698,29 @@ __global__ void __launch_bounds__(THREADS, 1)
           acc[blk * 4 + j] += comb;
         }
       }
-      ++per;
     }
-    // The tile leaves through the stage buffers (free: the last period's MMAs are done), so its columns and
-    // the columns of its mirror image are whole runs.  Straight from the registers every mirrored element
-    // was an atomic on a sector of its own: about 15 us a CTA, most of a bin of few pairs.
-    double2* tile = reinterpret_cast<double2*>(sm);      // [column 0..127][row 0..63], pitch TP
-    constexpr int TP = 65;
-    static_assert(BN * TP * static_cast<int>(sizeof(double2)) <= L::OFF_W, "the tile fits the stage buffers");
-    const bool good = ok && per == nper;
-    if (!good) *abort_flag = 1;
-    {
-      const int ml = row & 63, part = row >= 64 ? 1 : 0;
+    // The quadrants meet, and the tile leaves, through the stage buffers (free: the last period's MMAs are
+    // done), so its columns and the columns of its mirror image are whole runs.
+    long long* xs = reinterpret_cast<long long*>(sm);                  // [column 0..127][Im row 0..63]
+    constexpr int XS = BN * 64 * 8, TP = 65;
+    double2* tile = reinterpret_cast<double2*>(sm + XS);               // [column 0..63][row 0..63], pitch TP
+    static_assert(XS + 64 * TP * static_cast<int>(sizeof(double2)) <= L::OFF_BAR, "the tile fits the stage buffers");
+    if (!ok) *abort_flag = 1;
+    if (row >= 64) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) xs[(c_lo + j) * 64 + row - 64] = acc[j];
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(NDW * 32) : "memory");
+    if (row < 64) {
       const double* mub = p.mu + static_cast<long long>(bin) * p.Rows;
-      const int m = mt * 64 + ml;
+      const int m = mt * 64 + row;
       const double fm = m < p.M ? mub[m] * p.post * p.sign : 0.0;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const int n = nt * BN + c_lo + j;
-        const double val = n < p.N ? static_cast<double>(acc[j]) * fm * mub[p.row_b0 + n] : 0.0;
-        reinterpret_cast<double*>(tile + (c_lo + j) * TP + ml)[part] = val;
+        const int c = c_lo + j, cn = c & 63, n = nt * 64 + cn;
+        const long long sum = c < 64 ? acc[j] + xs[(64 + cn) * 64 + row] : acc[j] - xs[cn * 64 + row];
+        const double val = n < p.N ? static_cast<double>(sum) * fm * mub[p.row_b0 + n] : 0.0;
+        reinterpret_cast<double*>(tile + cn * TP + row)[c < 64 ? 0 : 1] = val;
       }
     }
     asm volatile("bar.sync 1, %0;" ::"r"(NDW * 32) : "memory");
@@ -767,23 +736,23 @@ __global__ void __launch_bounds__(THREADS, 1)
           atomicAdd(&dst->y, v.y);
         }
       };
-      const int dt = dw * 32 + lane;                     // 0..511
+      const int lo = (dw * 32 + lane) & 63, hi = (dw * 32 + lane) >> 6;
       {
-        // columns: 64 rows of 8 columns at a time; the upper part of a Hermitian output comes from the mirror
-        const int ml = dt & 63, m = mt * 64 + ml;
+        // columns; the upper part of a Hermitian output comes from the mirror
+        const int m = mt * 64 + lo;
 #pragma unroll 4
-        for (int c = dt >> 6; c < BN; c += NDW * 32 / 64) {
-          const int n = nt * BN + c;
-          if (m < p.M && n < p.N && !(p.herm && m < n)) add(Cb + m + static_cast<long long>(n) * p.ldc, tile[c * TP + ml]);
+        for (int c = hi; c < 64; c += NDW * 32 / 64) {
+          const int n = nt * 64 + c;
+          if (m < p.M && n < p.N && !(p.herm && m < n)) add(Cb + m + static_cast<long long>(n) * p.ldc, tile[c * TP + lo]);
         }
       }
       if (p.herm) {                                      // C(n, m) = conj(C(m, n)), m > n
-        const int c = dt & (BN - 1), n = nt * BN + c;
+        const int n = nt * 64 + lo;
 #pragma unroll 4
-        for (int ml = dt >> 7; ml < 64; ml += NDW * 32 / BN) {
+        for (int ml = hi; ml < 64; ml += NDW * 32 / 64) {
           const int m = mt * 64 + ml;
           if (m < p.M && n < p.N && m > n) {
-            double2 v = tile[c * TP + ml];
+            double2 v = tile[lo * TP + ml];
             v.y = -v.y;
             add(Cb + n + static_cast<long long>(m) * p.ldc, v);
           }
@@ -946,103 +915,82 @@ __global__ void oz_mu_kernel(const unsigned long long* __restrict__ zmax, const 
   mu[i] = pow2_at_least(sqrt(w_extent(wr, b, sign)) * __longlong_as_double(static_cast<long long>(zmax[m])));
 }
 
-// chi0: Y8[q][m][k0_b + 2 e' + {0,1}] = slices of (Re, Im) of sqrt(max(sign w_e, 0)) z_col(e)(m).
-// blockIdx.y = bin; blockIdx.x strides over (entry block of 32, 64-row tile) items of the bin.
-// Thread (row mm, group g) slices the 8 consecutive entries 8 g .. 8 g + 7 of its row (loads
-// coalesced along m), the 16 bytes per slice go to a shared tile with 80-byte rows (no bank
-// conflicts), and 64 rows x 64 bytes per slice leave coalesced along K.
-// the NS slices of the 8 entries (f z) of one row as 16 bytes each: (re, im) int8 pairs in entry order
+// chi0: the NS slices of eight pairs (f z) of one row into Y8 (chunk-major, [chunk][slice][re, im][row][KB]):
+// eight bytes a slice and part at byte `off` of the row
 template <int NS>
-__device__ __forceinline__ void y_pack(uint4 (&out)[NS], const double (&f)[8], const double2 (&zv)[8],
-                                       double scale) {
-  uint32_t w[NS][4];
+__device__ __forceinline__ void y_put(int8_t* __restrict__ y8, long long chunk, int Rows, int m, int off,
+                                      const double (&f)[8], const double2 (&zv)[8], double scale) {
+  constexpr int KB = HerkCfg<NS>::KB;
+  uint2 re[NS], im[NS];
 #pragma unroll
-  for (int jp = 0; jp < 4; ++jp) {
-    int r0[NS], i0[NS], r1[NS], i1[NS];
-    // (f z) scale with scale a power of two is z (f scale), rounded the same way
-    const double fs0 = f[2 * jp] * scale, fs1 = f[2 * jp + 1] * scale;
-    slice<NS>(zv[2 * jp].x, fs0, r0);
-    slice<NS>(zv[2 * jp].y, fs0, i0);
-    slice<NS>(zv[2 * jp + 1].x, fs1, r1);
-    slice<NS>(zv[2 * jp + 1].y, fs1, i1);
+  for (int h = 0; h < 2; ++h) {
+    int r[4][NS], c[4][NS];
 #pragma unroll
-    for (int q = 0; q < NS; ++q) w[q][jp] = pack4(r0[q], i0[q], r1[q], i1[q]);
+    for (int i = 0; i < 4; ++i) {
+      // (f z) scale with scale a power of two is z (f scale), rounded the same way
+      const double fs = f[4 * h + i] * scale;
+      slice<NS>(zv[4 * h + i].x, fs, r[i]);
+      slice<NS>(zv[4 * h + i].y, fs, c[i]);
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      (h ? re[q].y : re[q].x) = pack4(r[0][q], r[1][q], r[2][q], r[3][q]);
+      (h ? im[q].y : im[q].x) = pack4(c[0][q], c[1][q], c[2][q], c[3][q]);
+    }
   }
 #pragma unroll
-  for (int q = 0; q < NS; ++q) out[q] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-}
-template <int NS>
-__device__ __forceinline__ void y_tile_pack(int8_t (*tile)[64][80], int mm, int g, const double (&f)[8],
-                                            const double2 (&zv)[8], double scale) {
-  uint4 out[NS];
-  y_pack<NS>(out, f, zv, scale);
-#pragma unroll
-  for (int q = 0; q < NS; ++q) *reinterpret_cast<uint4*>(&tile[q][mm][g * 16]) = out[q];
-}
-
-// Y8 is chunk-major: [chunk][slice][row][64 bytes], so one TMA box (64 or 128 rows of one chunk
-// and slice) is one contiguous block of HBM
-template <int NS>
-__device__ __forceinline__ void y_tile_store(int8_t* __restrict__ y8, const int8_t (*tile)[64][80], int Rows, int rt,
-                                             long long chunk) {
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  const int mo = rt * 64 + row;
-  if (mo < Rows) {
-#pragma unroll
-    for (int q = 0; q < NS; ++q)
-      *reinterpret_cast<uint4*>(y8 + ((chunk * NS + q) * Rows + mo) * 64 + part * 16) =
-          *reinterpret_cast<const uint4*>(&tile[q][row][part * 16]);
+  for (int q = 0; q < NS; ++q) {
+    int8_t* d = y8 + ((chunk * NS + q) * 2 * Rows + m) * KB + off;
+    *reinterpret_cast<uint2*>(d) = re[q];
+    *reinterpret_cast<uint2*>(d + static_cast<long long>(Rows) * KB) = im[q];
   }
 }
 
+// Items of 64 pairs x 32 rows: thread (row mm = tid / 8, group g = tid % 8) takes eight pairs of its row, so
+// a row's 64 bytes per slice and part leave as one run; pairs beyond the bin are zeros.  blockIdx.y = bin,
+// blockIdx.x strides over the bin's items.
 template <int NS>
 __global__ void __launch_bounds__(256)
     oz_slice_y_kernel(int8_t* __restrict__ y8, int Rows, const double2* __restrict__ z, long long ldz,
                       const int* __restrict__ ecol, const double* __restrict__ ew, const long long* __restrict__ ebeg,
                       const int* __restrict__ cnt, const long long* __restrict__ bin_k0,
                       const double* __restrict__ wr, const double* __restrict__ mu, double sign) {
-  __shared__ __align__(16) int8_t tile[NS][64][80];
+  constexpr int PER = HerkCfg<NS>::KB / 64;              // 64-pair items per chunk
   const int b = blockIdx.y;
   if (!(w_extent(wr, b, sign) > 0.0)) return;
   const int n = cnt[b];
-  const int neb = (n + 31) / 32;
-  const int nrt = (Rows + 63) / 64;
+  const int neb = (n + 63) / 64;
+  const int nrt = (Rows + 31) / 32;
   const long long e0 = ebeg[b];
   const long long kc = bin_k0[b];
   const double* mub = mu + static_cast<long long>(b) * Rows;
-  const int mm = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int mm = threadIdx.x >> 3, g = threadIdx.x & 7;
   for (long long item = blockIdx.x; item < static_cast<long long>(neb) * nrt; item += gridDim.x) {
     const int eb = static_cast<int>(item % neb), rt = static_cast<int>(item / neb);
-    const int m = rt * 64 + mm;
-    const double scale = (m < Rows) ? slice_unit<NS>() / mub[m] : 0.0;
+    const int m = rt * 32 + mm;
+    if (m >= Rows) continue;
     double f[8];
     double2 zv[8];
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) {
-      const int e = eb * 32 + g * 8 + jj;
+      const int e = eb * 64 + g * 8 + jj;
       f[jj] = 0.0;
       zv[jj] = make_double2(0.0, 0.0);
-      if (e < n && m < Rows) {
+      if (e < n) {
         const long long ge = e0 + e;
         const long long col = ecol ? ecol[ge] : e;
         f[jj] = sqrt(fmax(sign * ew[ge], 0.0));
         zv[jj] = z[m + col * ldz];
       }
     }
-    y_tile_pack<NS>(tile, mm, g, f, zv, scale);
-    __syncthreads();
-    y_tile_store<NS>(y8, tile, Rows, rt, kc + eb);
-    __syncthreads();
+    y_put<NS>(y8, kc + eb / PER, Rows, m, (eb % PER) * 64 + g * 8, f, zv, slice_unit<NS>() / mub[m]);
   }
 }
 
 // chi0, every bin over the same columns 0..n-1 in order (bin b's weights at ew[b * n + e]): z is read
-// once per (32-column block, 64-row tile) item and sliced for every bin with a weight of this sign.
-// Thread (row mm = tid / 4, group g = tid % 4) slices the 8 consecutive entries 8 g .. 8 g + 7 of
-// its row; their 16 bytes per slice are one piece of the row's 64-byte chunk, so a warp (8 rows x
-// 4 groups) stores 512 contiguous bytes per slice straight from registers and loads 4 x 128
-// contiguous bytes of z per entry.  The square roots of the weights of up to kDenseBins bins are
-// formed once per item in shared memory: two barriers per item and bin group, none per bin.
+// once per item and sliced for every bin with a weight of this sign.  The square roots of the weights of up
+// to kDenseBins bins are formed once per item in shared memory: two barriers per item and bin group, none
+// per bin.
 constexpr int kDenseBins = 32;
 template <int NS>
 __global__ void __launch_bounds__(256)
@@ -1050,24 +998,25 @@ __global__ void __launch_bounds__(256)
                             long long ldz, int n, int nbins, const double* __restrict__ ew,
                             const long long* __restrict__ bin_k0, const double* __restrict__ wr,
                             const double* __restrict__ mu, double sign) {
-  __shared__ double sf[kDenseBins][32];
-  const int neb = (n + 31) / 32;
-  const int nrt = (Rows + 63) / 64;
-  const int mm = threadIdx.x >> 2, g = threadIdx.x & 3;
+  constexpr int PER = HerkCfg<NS>::KB / 64;
+  __shared__ double sf[kDenseBins][64];
+  const int neb = (n + 63) / 64;
+  const int nrt = (Rows + 31) / 32;
+  const int mm = threadIdx.x >> 3, g = threadIdx.x & 7;
   for (long long item = blockIdx.x; item < static_cast<long long>(neb) * nrt; item += gridDim.x) {
     const int eb = static_cast<int>(item % neb), rt = static_cast<int>(item / neb);
-    const int m = rt * 64 + mm;
+    const int m = rt * 32 + mm;
     double2 zv[8];
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) {
-      const int e = eb * 32 + g * 8 + jj;
+      const int e = eb * 64 + g * 8 + jj;
       zv[jj] = (e < n && m < Rows) ? z[m + static_cast<long long>(e) * ldz] : make_double2(0.0, 0.0);
     }
     for (int b0 = 0; b0 < nbins; b0 += kDenseBins) {
       const int nb = min(kDenseBins, nbins - b0);
       __syncthreads();                                   // every read of the previous group's sf is done
-      for (int i = threadIdx.x; i < nb * 32; i += 256) {
-        const int bb = i >> 5, c = i & 31, e = eb * 32 + c;
+      for (int i = threadIdx.x; i < nb * 64; i += 256) {
+        const int bb = i >> 6, c = i & 63, e = eb * 64 + c;
         sf[bb][c] = (e < n) ? sqrt(fmax(sign * ew[static_cast<long long>(b0 + bb) * n + e], 0.0)) : 0.0;
       }
       __syncthreads();
@@ -1078,12 +1027,8 @@ __global__ void __launch_bounds__(256)
         double f[8];
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) f[jj] = sf[bb][g * 8 + jj];
-        uint4 out[NS];
-        y_pack<NS>(out, f, zv, slice_unit<NS>() / mu[static_cast<long long>(b) * Rows + m]);
-        const long long chunk = bin_k0[b] + eb;
-#pragma unroll
-        for (int q = 0; q < NS; ++q)
-          *reinterpret_cast<uint4*>(y8 + ((chunk * NS + q) * Rows + m) * 64 + g * 16) = out[q];
+        y_put<NS>(y8, bin_k0[b] + eb / PER, Rows, m, (eb % PER) * 64 + g * 8, f, zv,
+                  slice_unit<NS>() / mu[static_cast<long long>(b) * Rows + m]);
       }
     }
   }
@@ -1134,13 +1079,12 @@ static int launch_seg(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
 }
 
 template <int NS>
-static int launch_herk(const CUtensorMap& ma, const CUtensorMap& mb, const HerkParams& p, dim3 grid,
-                       cudaStream_t s) {
+static int launch_herk(const CUtensorMap& my, const HerkParams& p, dim3 grid, cudaStream_t s) {
   static uint64_t attr = 0;
-  int rc = smem_limit_once(reinterpret_cast<const void*>(oz_herk_kernel<NS>), Cfg<NS>::SMEM, attr);
+  int rc = smem_limit_once(reinterpret_cast<const void*>(oz_herk_kernel<NS>), HerkCfg<NS>::SMEM, attr);
   if (rc) return rc;
   const int pi = prof_begin("chi0_tc", s);
-  oz_herk_kernel<NS><<<grid, THREADS, Cfg<NS>::SMEM, s>>>(ma, mb, p);
+  oz_herk_kernel<NS><<<grid, THREADS, HerkCfg<NS>::SMEM, s>>>(my, p);
   prof_end(pi, s);
   count_launch();
   QSGW_LAUNCH_CHECK("oz_herk_kernel");
@@ -1477,18 +1421,21 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
   if (nbins == 0 || M <= 0 || N <= 0 || (classes & 3) == 0) return QSGW_OK;
   QSGW_ARG(nbins <= 65535, "chi0 split-i8: %d bins exceed the grid limit", nbins);
   const int Rows = std::max(M, row_b0 + N);
-  // bin layout in Y8: each bin padded to whole 64-byte chunks (32 entries)
+  // bin layout in Y8: each bin padded to whole chunks of kb pairs
+  const int kb = ns <= 3 ? HerkCfg<3>::KB : HerkCfg<4>::KB;
+  static_assert(HerkCfg<2>::KB == HerkCfg<3>::KB, "one chunk width up to 3 slices");
   std::vector<long long> k0(nbins);
   std::vector<int> nch(nbins);
   long long tot = 0;
-  int maxch = 0;
+  int maxch = 0, maxcnt = 0;
   for (int b = 0; b < nbins; ++b) {
     k0[b] = tot;
-    nch[b] = (bins.cnt[b] + 31) / 32;
+    nch[b] = (bins.cnt[b] + kb - 1) / kb;
     tot += nch[b];
     maxch = std::max(maxch, nch[b]);
+    maxcnt = std::max(maxcnt, bins.cnt[b]);
   }
-  const long long Ktot = tot * K8;
+  const long long Ktot = tot * 2 * kb;
   QSGW_ARG(tot < (1LL << 31), "chi0 split-i8: %lld K chunks exceed the TMA coordinate range", tot);
   int rc = g_y8.ensure(static_cast<size_t>(ns) * Rows * Ktot);
   if (rc) return rc;
@@ -1528,7 +1475,7 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
   }
   QSGW_CUDA(cudaMemsetAsync(g_wr.p, 0, static_cast<size_t>(2 * nbins) * sizeof(double), s));
   {
-    const int per = std::max(1, std::min(64, static_cast<int>((maxch * 32LL + 4095) / 4096)));
+    const int per = std::max(1, std::min(64, static_cast<int>((maxcnt + 4095LL) / 4096)));
     oz_wrange_kernel<<<dim3(static_cast<unsigned>(per), static_cast<unsigned>(nbins)), 256, 0, s>>>(
         ew_d, d_eb, d_cnt, reinterpret_cast<unsigned long long*>(g_wr.p));
     count_launch();
@@ -1536,38 +1483,34 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
   QSGW_LAUNCH_CHECK("chi0 int8 ranges");
   int8_t* Y8 = g_y8.as<int8_t>();
   double* mu = g_ymu.as<double>();
-  CUtensorMap ma, mb;
+  CUtensorMap my;
   {
-    // [chunk][slice][row][64 B]: rows beyond Rows read as zero, boxes never cross a slice
-    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(K8), static_cast<cuuint64_t>(Rows),
-                                static_cast<cuuint64_t>(ns), static_cast<cuuint64_t>(tot)};
-    const cuuint64_t str[3] = {static_cast<cuuint64_t>(K8), static_cast<cuuint64_t>(K8) * Rows,
-                               static_cast<cuuint64_t>(K8) * Rows * ns};
-    const cuuint32_t boxa[4] = {K8, 64, 1, 1};
-    const cuuint32_t boxb[4] = {K8, BN, 1, 1};
-    rc = make_tensor_map(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, Y8, 4, dims, str, boxa, CU_TENSOR_MAP_SWIZZLE_64B);
-    if (rc) return rc;
-    rc = make_tensor_map(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, Y8, 4, dims, str, boxb, CU_TENSOR_MAP_SWIZZLE_64B);
+    // [chunk][slice, re / im][row][kb]: a box is 64 rows of both parts of one slice; rows beyond Rows read as
+    // zero, boxes never cross a slice
+    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(kb), static_cast<cuuint64_t>(Rows),
+                                static_cast<cuuint64_t>(2 * ns), static_cast<cuuint64_t>(tot)};
+    const cuuint64_t str[3] = {static_cast<cuuint64_t>(kb), static_cast<cuuint64_t>(kb) * Rows,
+                               static_cast<cuuint64_t>(kb) * Rows * 2 * ns};
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(kb), 64, 2, 1};
+    rc = make_tensor_map(&my, CU_TENSOR_MAP_DATA_TYPE_UINT8, Y8, 4, dims, str, box,
+                         kb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
   }
-  const int ntm = (M + 63) / 64, ntn = (N + BN - 1) / BN;
-  long long units = 0;
-  for (int nt = 0; nt < ntn; ++nt)
-    for (int mt = 0; mt < ntm; ++mt)
-      if (!herm || mt * 64 + 63 >= nt * BN) ++units;
-  units *= nbins;
-  // K splits: whole waves of one CTA an SM, counted in chunk times; a CTA's start and end (TMEM, pipeline
-  // fill, the drain and the FP64 additions of its tile) cost about as much as 24 chunks.  The tiles of a
-  // (bin, K part) unit are adjacent in the grid and share its rows of Y8 through L2.  (Splitting until one
-  // wave held a whole unit gave 37 splits of 5 chunks at 180 rows and 6000 pairs: 208 us.)
-  const int maxsplit = std::max(1, std::min(maxch / 4, 64));
+  const int ntm = (M + 63) / 64, ntn = (N + 63) / 64;
+  const long long ntiles = herm ? ntm * (ntm + 1LL) / 2 : static_cast<long long>(ntm) * ntn;
+  const long long units = ntiles * nbins;
+  // K splits: whole waves of one CTA an SM, counted in K steps of 32 pairs; a CTA's start and end (TMEM,
+  // pipeline fill, the drain and the FP64 additions of its tile) cost about as much as 24 of them.  The tiles
+  // of a (bin, K part) unit are adjacent in the grid and share its rows of Y8 through L2.  (Splitting until
+  // one wave held a whole unit gave 37 splits of 160 pairs at 180 rows and 6000 pairs: 208 us.)
+  const int maxsplit = std::max(1, std::min(maxch / 2, 64));
   auto cost = [&](int sp) {
-    return static_cast<double>((units * sp + ctx().sm_count - 1) / ctx().sm_count) * ((maxch + sp - 1) / sp + 24);
+    const int steps = ((maxch + sp - 1) / sp) * (kb / 32);
+    return static_cast<double>((units * sp + ctx().sm_count - 1) / ctx().sm_count) * (steps + 24);
   };
   double tbest = cost(1);
   for (int sp = 2; sp <= maxsplit; ++sp) tbest = std::min(tbest, cost(sp));
   // of the counts within 2 % the largest: shorter parts keep the CTAs that share rows of Y8 closer together
-  // (600 rows, 390 834 pairs, 24 bins: 65.3 ms unsplit, 62.5 at 20)
   int heur = 1;
   for (int sp = 1; sp <= maxsplit; ++sp)
     if (cost(sp) <= 1.02 * tbest) heur = sp;
@@ -1576,7 +1519,7 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
   for (int b = 0; b < nbins && dense; ++b) dense = bins.cnt[b] == bins.cnt[0] && bins.ebeg[b] == static_cast<long long>(b) * bins.cnt[0];
   HerkParams p{};
   p.M = M; p.N = N; p.ntm = ntm; p.herm = herm ? 1 : 0; p.row_b0 = row_b0; p.Rows = Rows;
-  p.bin_k0 = d_k0; p.bin_nch = d_nch; p.bin_slab = d_slab; p.wrange = g_wr.as<double>(); p.mu = mu;
+  p.bin_k0 = d_k0; p.bin_nch = d_nch; p.bin_cnt = d_cnt; p.bin_slab = d_slab; p.wrange = g_wr.as<double>(); p.mu = mu;
   p.post = post_scale(ns);
   p.C = C; p.ldc = ldc; p.c_bs = c_bs;
   p.err = ctx().d_flags + 1;
@@ -1584,7 +1527,7 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
     const int nmu = nbins * Rows;
     oz_mu_kernel<<<(nmu + 255) / 256, 256, 0, s>>>(zmax, g_wr.as<double>(), Rows, nbins, sign, mu);
     count_launch();
-    const long long items = static_cast<long long>(maxch) * ((Rows + 63) / 64);   // (32-entry block, 64 rows)
+    const long long items = static_cast<long long>((maxcnt + 63) / 64) * ((Rows + 31) / 32);   // (64 pairs, 32 rows)
     const int pslice = prof_begin("chi0_slice_i8", s);
     if (dense) {
       const int n = bins.cnt[0];
@@ -1600,10 +1543,10 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
       prof_end(pslice, s);
       HerkParams q = p;
       q.sign = sign;
-      const dim3 grid(static_cast<unsigned>(ntm * ntn), static_cast<unsigned>(nbins), static_cast<unsigned>(splitk));
-      if (ns == 2) return launch_herk<2>(ma, mb, q, grid, s);
-      if (ns == 3) return launch_herk<3>(ma, mb, q, grid, s);
-      return launch_herk<4>(ma, mb, q, grid, s);
+      const dim3 grid(static_cast<unsigned>(ntiles), static_cast<unsigned>(nbins), static_cast<unsigned>(splitk));
+      if (ns == 2) return launch_herk<2>(my, q, grid, s);
+      if (ns == 3) return launch_herk<3>(my, q, grid, s);
+      return launch_herk<4>(my, q, grid, s);
     }
     const dim3 gy(static_cast<unsigned>(std::max<long long>(1, std::min<long long>(items, 4LL * ctx().sm_count))),
                   static_cast<unsigned>(nbins));
@@ -1618,10 +1561,10 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
     prof_end(pslice, s);
     HerkParams q = p;
     q.sign = sign;
-    const dim3 grid(static_cast<unsigned>(ntm * ntn), static_cast<unsigned>(nbins), static_cast<unsigned>(splitk));
-    if (ns == 2) return launch_herk<2>(ma, mb, q, grid, s);
-    if (ns == 3) return launch_herk<3>(ma, mb, q, grid, s);
-    return launch_herk<4>(ma, mb, q, grid, s);
+    const dim3 grid(static_cast<unsigned>(ntiles), static_cast<unsigned>(nbins), static_cast<unsigned>(splitk));
+    if (ns == 2) return launch_herk<2>(my, q, grid, s);
+    if (ns == 3) return launch_herk<3>(my, q, grid, s);
+    return launch_herk<4>(my, q, grid, s);
   };
   auto run = [&](int splitk, bool clear) -> int {
     if (clear) {
