@@ -915,15 +915,15 @@ __global__ void oz_mu_kernel(const unsigned long long* __restrict__ zmax, const 
   mu[i] = pow2_at_least(sqrt(w_extent(wr, b, sign)) * __longlong_as_double(static_cast<long long>(zmax[m])));
 }
 
-// chi0: the NS slices of eight pairs (f z) of one row into Y8 (chunk-major, [chunk][slice][re, im][row][KB]):
-// eight bytes a slice and part at byte `off` of the row
+// chi0: the NS slices of sixteen pairs (f z) of one row into Y8 (chunk-major, [chunk][slice][re, im][row][KB]):
+// 16 bytes a slice and part at byte `off` of the row
 template <int NS>
 __device__ __forceinline__ void y_put(int8_t* __restrict__ y8, long long chunk, int Rows, int m, int off,
-                                      const double (&f)[8], const double2 (&zv)[8], double scale) {
+                                      const double* __restrict__ f, const double2 (&zv)[16], double scale) {
   constexpr int KB = HerkCfg<NS>::KB;
-  uint2 re[NS], im[NS];
+  uint32_t re[NS][4], im[NS][4];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < 4; ++h) {
     int r[4][NS], c[4][NS];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -934,20 +934,21 @@ __device__ __forceinline__ void y_put(int8_t* __restrict__ y8, long long chunk, 
     }
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      (h ? re[q].y : re[q].x) = pack4(r[0][q], r[1][q], r[2][q], r[3][q]);
-      (h ? im[q].y : im[q].x) = pack4(c[0][q], c[1][q], c[2][q], c[3][q]);
+      re[q][h] = pack4(r[0][q], r[1][q], r[2][q], r[3][q]);
+      im[q][h] = pack4(c[0][q], c[1][q], c[2][q], c[3][q]);
     }
   }
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
     int8_t* d = y8 + ((chunk * NS + q) * 2 * Rows + m) * KB + off;
-    *reinterpret_cast<uint2*>(d) = re[q];
-    *reinterpret_cast<uint2*>(d + static_cast<long long>(Rows) * KB) = im[q];
+    *reinterpret_cast<uint4*>(d) = make_uint4(re[q][0], re[q][1], re[q][2], re[q][3]);
+    *reinterpret_cast<uint4*>(d + static_cast<long long>(Rows) * KB) = make_uint4(im[q][0], im[q][1], im[q][2], im[q][3]);
   }
 }
 
-// Items of 64 pairs x 32 rows: thread (row mm = tid / 8, group g = tid % 8) takes eight pairs of its row, so
-// a row's 64 bytes per slice and part leave as one run; pairs beyond the bin are zeros.  blockIdx.y = bin,
+// Items of 64 pairs x 64 rows: thread (row mm = tid / 4, group g = tid % 4) takes sixteen pairs of its row, so
+// a row's 64 bytes per slice and part leave as four 16-byte stores of one run and a warp reads 128 bytes of
+// z per pair; pairs beyond the bin are zeros.  blockIdx.y = bin,
 // blockIdx.x strides over the bin's items.
 template <int NS>
 __global__ void __launch_bounds__(256)
@@ -960,20 +961,20 @@ __global__ void __launch_bounds__(256)
   if (!(w_extent(wr, b, sign) > 0.0)) return;
   const int n = cnt[b];
   const int neb = (n + 63) / 64;
-  const int nrt = (Rows + 31) / 32;
+  const int nrt = (Rows + 63) / 64;
   const long long e0 = ebeg[b];
   const long long kc = bin_k0[b];
   const double* mub = mu + static_cast<long long>(b) * Rows;
-  const int mm = threadIdx.x >> 3, g = threadIdx.x & 7;
+  const int mm = threadIdx.x >> 2, g = threadIdx.x & 3;
   for (long long item = blockIdx.x; item < static_cast<long long>(neb) * nrt; item += gridDim.x) {
     const int eb = static_cast<int>(item % neb), rt = static_cast<int>(item / neb);
-    const int m = rt * 32 + mm;
+    const int m = rt * 64 + mm;
     if (m >= Rows) continue;
-    double f[8];
-    double2 zv[8];
+    double f[16];
+    double2 zv[16];
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-      const int e = eb * 64 + g * 8 + jj;
+    for (int jj = 0; jj < 16; ++jj) {
+      const int e = eb * 64 + g * 16 + jj;
       f[jj] = 0.0;
       zv[jj] = make_double2(0.0, 0.0);
       if (e < n) {
@@ -983,14 +984,15 @@ __global__ void __launch_bounds__(256)
         zv[jj] = z[m + col * ldz];
       }
     }
-    y_put<NS>(y8, kc + eb / PER, Rows, m, (eb % PER) * 64 + g * 8, f, zv, slice_unit<NS>() / mub[m]);
+    y_put<NS>(y8, kc + eb / PER, Rows, m, (eb % PER) * 64 + g * 16, f, zv, slice_unit<NS>() / mub[m]);
   }
 }
 
 // chi0, every bin over the same columns 0..n-1 in order (bin b's weights at ew[b * n + e]): z is read
 // once per item and sliced for every bin with a weight of this sign.  The square roots of the weights of up
 // to kDenseBins bins are formed once per item in shared memory: two barriers per item and bin group, none
-// per bin.
+// per bin.  Bound by the integer pipe (digits) and then by writing the slices: 390 834 pairs x 600 rows x 24 bins
+// at 3 slices in 10.5 ms, 3.2 TB/s of slices (11.8 ms with eight pairs a thread and 8-byte stores).
 constexpr int kDenseBins = 32;
 template <int NS>
 __global__ void __launch_bounds__(256)
@@ -1001,15 +1003,15 @@ __global__ void __launch_bounds__(256)
   constexpr int PER = HerkCfg<NS>::KB / 64;
   __shared__ double sf[kDenseBins][64];
   const int neb = (n + 63) / 64;
-  const int nrt = (Rows + 31) / 32;
-  const int mm = threadIdx.x >> 3, g = threadIdx.x & 7;
+  const int nrt = (Rows + 63) / 64;
+  const int mm = threadIdx.x >> 2, g = threadIdx.x & 3;
   for (long long item = blockIdx.x; item < static_cast<long long>(neb) * nrt; item += gridDim.x) {
     const int eb = static_cast<int>(item % neb), rt = static_cast<int>(item / neb);
-    const int m = rt * 32 + mm;
-    double2 zv[8];
+    const int m = rt * 64 + mm;
+    double2 zv[16];
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-      const int e = eb * 64 + g * 8 + jj;
+    for (int jj = 0; jj < 16; ++jj) {
+      const int e = eb * 64 + g * 16 + jj;
       zv[jj] = (e < n && m < Rows) ? z[m + static_cast<long long>(e) * ldz] : make_double2(0.0, 0.0);
     }
     for (int b0 = 0; b0 < nbins; b0 += kDenseBins) {
@@ -1024,10 +1026,7 @@ __global__ void __launch_bounds__(256)
       for (int bb = 0; bb < nb; ++bb) {
         const int b = b0 + bb;
         if (!(w_extent(wr, b, sign) > 0.0)) continue;
-        double f[8];
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) f[jj] = sf[bb][g * 8 + jj];
-        y_put<NS>(y8, bin_k0[b] + eb / PER, Rows, m, (eb % PER) * 64 + g * 8, f, zv,
+        y_put<NS>(y8, bin_k0[b] + eb / PER, Rows, m, (eb % PER) * 64 + g * 16, &sf[bb][g * 16], zv,
                   slice_unit<NS>() / mu[static_cast<long long>(b) * Rows + m]);
       }
     }
@@ -1527,7 +1526,7 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
     const int nmu = nbins * Rows;
     oz_mu_kernel<<<(nmu + 255) / 256, 256, 0, s>>>(zmax, g_wr.as<double>(), Rows, nbins, sign, mu);
     count_launch();
-    const long long items = static_cast<long long>((maxcnt + 63) / 64) * ((Rows + 31) / 32);   // (64 pairs, 32 rows)
+    const long long items = static_cast<long long>((maxcnt + 63) / 64) * ((Rows + 63) / 64);   // (64 pairs, 64 rows)
     const int pslice = prof_begin("chi0_slice_i8", s);
     if (dense) {
       const int n = bins.cnt[0];
