@@ -773,11 +773,17 @@ __global__ void __launch_bounds__(THREADS, 1)
 // =====================================================================================
 // operand preparation (HBM-bound)
 
+// matrix `slot` of a stack in two pieces
+__device__ __forceinline__ const double2* slot_ptr(const double2* a, const double2* b, int n1, int slot, long long stride) {
+  return slot < n1 ? a + slot * stride : b + (slot - n1) * stride;
+}
+
 // out[slot * ncols_out + j] = scale of column c = colmap[j] (or j) of the complex column-major
-// matrix src + slot * slot_stride (leading dimension ld): the max over k < K of max(|Re|, |Im|)
+// matrix `slot` (leading dimension ld; slots 0..n1-1 at src, the others at src2, slot_stride apart): the max over k < K of max(|Re|, |Im|)
 // itself (the base-256 slicing divides by it, so no power of two is needed, and the full
 // digit range is used); 1 for absent, zero or non-finite columns.  One warp per column.
-__global__ void oz_colscale_kernel(const double2* __restrict__ src, long long ld, long long slot_stride, int K,
+__global__ void oz_colscale_kernel(const double2* __restrict__ src, const double2* __restrict__ src2, int n1,
+                                   long long ld, long long slot_stride, int K,
                                    int ncols_valid, const int* __restrict__ colmap, int ncols_out,
                                    double* __restrict__ out) {
   const int slot = blockIdx.y;
@@ -787,7 +793,7 @@ __global__ void oz_colscale_kernel(const double2* __restrict__ src, long long ld
   const int c = colmap ? colmap[j] : (j < ncols_valid ? j : -1);
   double m = 0.0;
   if (c >= 0) {
-    const double2* col = src + static_cast<long long>(slot) * slot_stride + static_cast<long long>(c) * ld;
+    const double2* col = slot_ptr(src, src2, n1, slot, slot_stride) + static_cast<long long>(c) * ld;
     for (int k = lane; k < K; k += 32) {
       const double2 v = col[k];
       m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
@@ -797,21 +803,22 @@ __global__ void oz_colscale_kernel(const double2* __restrict__ src, long long ld
   if (lane == 0) out[static_cast<long long>(slot) * ncols_out + j] = (m > 0.0 && isfinite(m)) ? m : 1.0;
 }
 
-// Sigma_c A' slices from W (K x M per slot): A(m, k) = conj(W_slot[k + m ld]) into
+// Sigma_c A' slices from W (K x M per slot, slots as in oz_colscale_kernel): A(m, k) = conj(W_slot[k + m ld]) into
 // [q][slot_out0 + slot][t][half][64][Kp] int8; each thread four consecutive k of one row.
 // grid (ceil(Kp/2 / 128), nslot * T), block 256: warp w rows w, w + 8, ..
 // TAIL: only the first 32 complex rows of the last row tile t = T - 1 (grid y = slot), into the
 // half-height tail layout [q][slot_out0 + slot][half][32][Kp] that the paired tail tiles read.
 // Tw: row tiles written per slot (T, or T - 1 when the last one is read from the tail slices).
 template <int NS, bool TAIL = false>
-__global__ void oz_slice_w_kernel(int8_t* __restrict__ out, const double2* __restrict__ w, long long ld,
-                                  long long slot_stride, int M, int K, int T, int Tw, int nslot_total, int slot_out0,
+__global__ void oz_slice_w_kernel(int8_t* __restrict__ out, const double2* __restrict__ w,
+                                  const double2* __restrict__ w2, int n1, long long ld, long long slot_stride, int M, int K, int T, int Tw, int nslot_total, int slot_out0,
                                   int Kp, const double* __restrict__ mu) {
   const int st = blockIdx.y;                           // slot * Tw + t of this launch (TAIL: slot)
   const int t = TAIL ? T - 1 : st % Tw, slot = TAIL ? st : st / Tw;
   const int k0 = (blockIdx.x * 32 + (threadIdx.x & 31)) * 4;
   if (k0 >= Kp / 2) return;
   const int gslot = slot_out0 + slot;
+  const double2* ws = slot_ptr(w, w2, n1, slot, slot_stride);
   constexpr int ROWS = TAIL ? 32 : 64;
   for (int mm = threadIdx.x >> 5; mm < ROWS; mm += 8) {
     const int m = t * 64 + mm;
@@ -821,7 +828,7 @@ __global__ void oz_slice_w_kernel(int8_t* __restrict__ out, const double2* __res
     for (int i = 0; i < 4; ++i) {
       const int k = k0 + i;
       double2 v = make_double2(0.0, 0.0);
-      if (m < M && k < K) v = w[static_cast<long long>(slot) * slot_stride + k + static_cast<long long>(m) * ld];
+      if (m < M && k < K) v = ws[k + static_cast<long long>(m) * ld];
       slice8<NS>(v.x, inv, sr[i]);                     // Re a
       slice8<NS>(-v.y, inv, si[i]);                    // Im a  (a = conj(W))
       slice8<NS>(v.y, inv, sn[i]);                     // -Im a, sliced on its own (base-256 digits)
@@ -1207,15 +1214,10 @@ int OzSigcBatch::add(const SigcSplitArgs& a, cudaStream_t s) {
   double* mu = g_mu.as<double>();
   double* nu = g_nu.as<double>() + row0;
   // row scales of A' (= column scales of every W record) and column scales of B
-  oz_colscale_kernel<<<dim3((T * 64 + 7) / 8, a.nimag), 256, 0, s>>>(a.wi, a.ldw, wst, ngb, M, nullptr, T * 64,
-                                                                    mu + slot0 * T * 64);
+  oz_colscale_kernel<<<dim3((T * 64 + 7) / 8, nslot), 256, 0, s>>>(a.wi, a.wr, a.nimag, a.ldw, wst, ngb, M, nullptr,
+                                                                  T * 64, mu + slot0 * T * 64);
   count_launch();
-  if (a.nreal > 0) {
-    oz_colscale_kernel<<<dim3((T * 64 + 7) / 8, a.nreal), 256, 0, s>>>(a.wr, a.ldw, wst, ngb, M, nullptr, T * 64,
-                                                                      mu + (slot0 + a.nimag) * T * 64);
-    count_launch();
-  }
-  oz_colscale_kernel<<<dim3((nrows + 7) / 8, 1), 256, 0, s>>>(a.zmel, ldz, 0, ngb, 0, d_cols, nrows, nu);
+  oz_colscale_kernel<<<dim3((nrows + 7) / 8, 1), 256, 0, s>>>(a.zmel, nullptr, 1, ldz, 0, ngb, 0, d_cols, nrows, nu);
   count_launch();
   QSGW_LAUNCH_CHECK("oz_colscale_kernel");
   const int pslice = prof_begin("sigc_slice_i8", s);
@@ -1226,27 +1228,23 @@ int OzSigcBatch::add(const SigcSplitArgs& a, cudaStream_t s) {
   const dim3 gk(static_cast<unsigned>((Kp / 2 + 127) / 128));
   const bool tail = paired_tail(M);
   const int Tw = tail ? T - 1 : T;                     // the last row tile goes to the tail slices instead
-  auto slice_w = [&](const double2* w, int n, int gslot0) {
+  auto slice_w = [&](auto nsc) {                       // both stacks in one launch, the last row tile half height
+    constexpr int N = decltype(nsc)::value;
+    const int g0 = static_cast<int>(slot0);
     if (Tw > 0) {
-      const dim3 g(gk.x, static_cast<unsigned>(n * Tw));
-      if (ns == 2) oz_slice_w_kernel<2><<<g, 256, 0, s>>>(A8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
-      else if (ns == 3) oz_slice_w_kernel<3><<<g, 256, 0, s>>>(A8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
-      else oz_slice_w_kernel<4><<<g, 256, 0, s>>>(A8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
+      oz_slice_w_kernel<N><<<dim3(gk.x, static_cast<unsigned>(nslot * Tw)), 256, 0, s>>>(
+          A8, a.wi, a.wr, a.nimag, a.ldw, wst, M, ngb, T, Tw, nst, g0, Kp, mu);
       count_launch();
     }
-    if (tail) {                                        // the last row tile, half height
-      int8_t* T8 = g_t8.as<int8_t>();
-      const dim3 gt(gk.x, static_cast<unsigned>(n));
-      if (ns == 2)
-        oz_slice_w_kernel<2, true><<<gt, 256, 0, s>>>(T8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
-      else if (ns == 3)
-        oz_slice_w_kernel<3, true><<<gt, 256, 0, s>>>(T8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
-      else oz_slice_w_kernel<4, true><<<gt, 256, 0, s>>>(T8, w, a.ldw, wst, M, ngb, T, Tw, nst, gslot0, Kp, mu);
+    if (tail) {
+      oz_slice_w_kernel<N, true><<<dim3(gk.x, static_cast<unsigned>(nslot)), 256, 0, s>>>(
+          g_t8.as<int8_t>(), a.wi, a.wr, a.nimag, a.ldw, wst, M, ngb, T, Tw, nst, g0, Kp, mu);
       count_launch();
     }
   };
-  slice_w(a.wi, a.nimag, static_cast<int>(slot0));
-  if (a.nreal > 0) slice_w(a.wr, a.nreal, static_cast<int>(slot0) + a.nimag);
+  if (ns == 2) slice_w(std::integral_constant<int, 2>());
+  else if (ns == 3) slice_w(std::integral_constant<int, 3>());
+  else slice_w(std::integral_constant<int, 4>());
   {
     const dim3 g(gk.x, static_cast<unsigned>((nrows + 7) / 8));
     if (ns == 2) oz_slice_z_kernel<2><<<g, 256, 0, s>>>(B8, a.zmel, ldz, ngb, d_cols, nrows, rs, Kp, nu);
