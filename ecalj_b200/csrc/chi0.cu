@@ -62,6 +62,12 @@ static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc)
   return (bt.maxcnt + ZG_BK - 1) / ZG_BK;
 }
 
+// Bins of at most this many pairs on average stay on the FP64 engine in the int8 mode too: it is the more
+// accurate and, there, the faster one, as the int8 path's slicing passes and its CTAs' start and end cost more
+// than the products.  Measured per call (FP64 / 3 slices, us): 300 rows, 80 bins of 32 pairs 170 / 288, of 128
+// 390 / 414, of 256 711 / 610; 600 rows, 40 bins of 32 226 / 405, of 128 426 / 433, of 256 747 / 528.
+constexpr int kFp64BinPairs = 128;
+
 static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int nwhis, int npm,
                          int ns1, int ns2, const double2* zmel, int nbb, int nm1, int nm2,
                          int nqtot, int icounkmink, int icounkmaxk, const int* itc, const int* itpc,
@@ -115,7 +121,7 @@ static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int n
       fill[b]++;
     }
   }
-  if (ctx().prec_mode == QSGW_PREC_SPLIT_I8) {
+  if (ctx().prec_mode == QSGW_PREC_SPLIT_I8 && tot > kFp64BinPairs * static_cast<long long>(bt.cnt.size())) {
     // the same bins on the int8 tensor-core path: the pair columns and weights go to the device,
     // each bin's entries form one K range; rcxq accumulates (no tuning trials)
     int rc = g_x0_idx.ensure(std::max<size_t>(tot, 1) * sizeof(int));

@@ -53,10 +53,11 @@ def test_chi0_hermitian_tiles(qsgw, i8, n, ns):
             assert np.array_equal(got[:, :, iw], got[:, :, iw].conj().T)
 
 
+@pytest.mark.parametrize("ncoun", [60, 640, 641, 1500])       # 128 pairs a bin: the FP64 engine up to there
 @pytest.mark.parametrize("npr,ipr_col,npr_col", [(130, 1, 130), (70, 3, 129)])
-def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col):
+def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col, ncoun):
     rng = np.random.default_rng(npr)
-    nbb, nm, nq, nwhis, ncoun = 140, 4, 6, 5, 60
+    nbb, nm, nq, nwhis = 140, 4, 6, 5
     z = _rc(rng, nbb, nm, nq)
     tabs = (rng.integers(1, nm + 1, ncoun), rng.integers(1, nq + 1, ncoun), np.ones(ncoun, int),
             *(2 * [rng.integers(1, nwhis + 1, ncoun)]), np.arange(1, ncoun + 1))
