@@ -12,7 +12,9 @@
 // two and lost a third of the cycles to issue waits and barriers.  1536^3:
 // 32 TFLOP/s, DMMA pipe 90 % busy (cuBLAS 35); the basis change of 24
 // matrices of 600: 1.70 -> 1.46 ms; chi0 of 260 rows, 12 800 pairs and 12
-// frequencies (with the tile rules below) 3.99 -> 2.28 ms.
+// frequencies (with the tile rules below) 3.99 -> 2.10 ms.  At 128 registers
+// the gathered modes spill easily: strides, conjugations and the tile's
+// columns kept out of registers there are worth 10 %.
 //
 // Three problem modes share the main loop:
 //   ZM_GEMM  C = alpha op(A) op(B) + beta C, batched, optional split-K.
@@ -69,6 +71,7 @@ struct ZSmem {
   double2 b[ZG_STAGES][ZG_BK][ZG_PB];
   double sk[ZG_STAGES][ZG_BK];
   double sn[ZG_STAGES][ZG_BN];
+  int col[ZG_BN];
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
@@ -105,6 +108,11 @@ __device__ __forceinline__ void tri_decode(int t, int& tm, int& tn) {
 
 template <int MODE, bool A_RC, bool B_RC>
 __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams p) {
+  // known in the two gathered modes: the contiguous operand direction and the conjugations
+  constexpr bool GATHER = MODE != ZM_GEMM;
+  const long long a_rs = GATHER && A_RC ? 1 : p.a_rs, a_ks = GATHER && !A_RC ? 1 : p.a_ks;
+  const long long b_rs = GATHER && B_RC ? 1 : p.b_rs, b_ks = GATHER && !B_RC ? 1 : p.b_ks;
+  const bool a_conj = MODE == ZM_GEMM ? p.a_conj != 0 : true, b_conj = MODE == ZM_GEMM ? p.b_conj != 0 : false;
   extern __shared__ __align__(16) unsigned char zg_smem_raw[];
   ZSmem& sm = *reinterpret_cast<ZSmem*>(zg_smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -159,12 +167,10 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
   const int ar0 = A_RC ? tid % ZG_BM : tid / ZG_BK, ak0 = A_RC ? tid / ZG_BM : tid % ZG_BK;
   const int br0 = B_RC ? tid % ZG_BN : tid / ZG_BK, bk0 = B_RC ? tid / ZG_BN : tid % ZG_BK;
   const int Klim = (MODE == ZM_CHI0) ? Kbin : p.K;
-  int bcol[EB], scol = -1;                       // SEG: the columns the thread loads, and scales
+  // SEG: the tile's columns (-1: none) stay in shared memory, a register apiece spilled the main loop
   if (MODE == ZM_SEG) {
-    const int* tc = p.tile_cols + tn * ZG_BN;
-#pragma unroll
-    for (int i = 0; i < EB; ++i) bcol[i] = tc[br0 + i * BR];
-    if (tid < ZG_BN) scol = tc[tid];
+    if (tid < ZG_BN) sm.col[tid] = p.tile_cols[tn * ZG_BN + tid];
+    __syncthreads();
   }
   int kidx[EA];                                  // CHI0: zmel columns of the next chunk's entries (A and B alike)
   auto fetch_cols = [&](int c) {
@@ -176,26 +182,26 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
   };
   if (MODE == ZM_CHI0) fetch_cols(ch0);
   int lseg = MODE == ZM_SEG ? ch0 / kch_seg : 0, lin = MODE == ZM_SEG ? ch0 - lseg * kch_seg : 0;
-  const double2* segA = Ab;                      // SEG: the segment load_chunk is in
-  const double* segW = nullptr;
+  const double2* segA = Ab;                      // SEG: the segment load_chunk is in, the thread's column scale
+  const double* segW = p.wts;
   auto next_seg = [&]() {
-    const ZSeg sg = p.segs[seg0 + lseg];
+    const ZSeg& sg = p.segs[seg0 + lseg];
     segA = sg.mat;
-    segW = scol >= 0 ? sg.scale + static_cast<long long>(scol) * sg.scale_cs : nullptr;
+    if (tid < ZG_BN) segW = sg.scale + static_cast<long long>(max(sm.col[tid], 0)) * sg.scale_cs;
   };
   if (MODE == ZM_SEG && ch0 < ch1) next_seg();
   auto load_chunk = [&](int c, int st) {         // chunks in ascending order
     const int kbase = (MODE == ZM_SEG ? lin : c) * ZG_BK;
-    const double2* pa = segA + (m0 + ar0) * p.a_rs;
-    const double2* pb = Bb + (MODE == ZM_SEG ? 0 : (n0 + br0) * p.b_rs);
+    const double2* pa = segA + (m0 + ar0) * a_rs;
+    const double2* pb = Bb + (MODE == ZM_SEG ? 0 : (n0 + br0) * b_rs);
     if (MODE != ZM_CHI0) {
-      pa += (kbase + ak0) * p.a_ks;
-      pb += (kbase + bk0) * p.b_ks;
+      pa += (kbase + ak0) * a_ks;
+      pb += (kbase + bk0) * b_ks;
     }
 #pragma unroll
     for (int i = 0; i < EA; ++i) {
       const bool ok = kbase + ak0 + i * AK < Klim && m0 + ar0 + i * AR < Mrows;
-      const double2* src = MODE == ZM_CHI0 ? pa + kidx[i] * p.a_ks : pa + i * (AR * p.a_rs + AK * p.a_ks);
+      const double2* src = MODE == ZM_CHI0 ? pa + kidx[i] * a_ks : pa + i * (AR * a_rs + AK * a_ks);
       cp_async16(&sm.a[st][ak0 + i * AK][ar0 + i * AR], ok ? src : p.A, ok);
     }
 #pragma unroll
@@ -203,11 +209,12 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
       bool ok = kbase + bk0 + i * BK < Klim;
       const double2* src;
       if (MODE == ZM_SEG) {
-        ok = ok && bcol[i] >= 0;
-        src = pb + bcol[i] * p.b_rs;
+        const int col = sm.col[br0 + i * BR];
+        ok = ok && col >= 0;
+        src = pb + col * b_rs;
       } else {
         ok = ok && n0 + br0 + i * BR < p.N;
-        src = MODE == ZM_CHI0 ? pb + kidx[i] * p.b_ks : pb + i * (BR * p.b_rs + BK * p.b_ks);
+        src = MODE == ZM_CHI0 ? pb + kidx[i] * b_ks : pb + i * (BR * b_rs + BK * b_ks);
       }
       cp_async16(&sm.b[st][bk0 + i * BK][br0 + i * BR], ok ? src : p.B, ok);
     }
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
       fetch_cols(c + 1);
     }
     if (MODE == ZM_SEG) {
-      if (tid < ZG_BN) cp_async8(&sm.sn[st][tid], scol >= 0 ? segW : reinterpret_cast<const double*>(p.B), scol >= 0);
+      if (tid < ZG_BN) cp_async8(&sm.sn[st][tid], segW, sm.col[tid] >= 0);
       if (++lin == kch_seg) {
         lin = 0;
         ++lseg;
@@ -237,8 +244,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
   // the upper half of a Hermitian diagonal tile, issue no DMMA for fragments nobody reads.
   int ncol_tile = p.N - n0;
   if (MODE == ZM_SEG) {                         // -1 columns fill the end of a tile
-    const int* tc = p.tile_cols + tn * ZG_BN;
-    const int v = (tc[lane] >= 0) + (tc[lane + 32] >= 0);
+    const int v = (sm.col[lane] >= 0) + (sm.col[lane + 32] >= 0);
     ncol_tile = __reduce_add_sync(0xffffffffu, v);
   }
   const int ni = min(2, max(0, (Mrows - m0 - wm * 32 + 15) / 16));
@@ -290,7 +296,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             ar[i][e] = v[e].x;
-            ai[i][e] = p.a_conj ? -v[e].y : v[e].y;
+            ai[i][e] = a_conj ? -v[e].y : v[e].y;
           }
         }
         double ska = 1.0, skb = 1.0;
@@ -303,7 +309,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
           double sa = ska, sb = skb;
           if (MODE == ZM_SEG) sa = sb = sm.sn[st][nn];
           const double bra = va.x * sa, brb = vb.x * sb;
-          const double bia = (p.b_conj ? -va.y : va.y) * sa, bib = (p.b_conj ? -vb.y : vb.y) * sb;
+          const double bia = (b_conj ? -va.y : va.y) * sa, bib = (b_conj ? -vb.y : vb.y) * sb;
           // the two products of an accumulator stand apart: issued back to back the second waits for the first
 #pragma unroll
           for (int i = 0; i < 2; ++i)
@@ -412,7 +418,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_f64_kernel(const ZParams 
                                 i2 + p.beta.x * o.y + p.beta.y * o.x);
           }
         } else {
-          const int col = p.tile_cols[tn * ZG_BN + cl];
+          const int col = sm.col[cl];
           if (row >= p.M || col < 0) continue;
           double2* dst = Cb + row + static_cast<long long>(col) * p.ldc;
           if (p.splitk > 1) { atomicAdd(&dst->x, vr); atomicAdd(&dst->y, vi); }
