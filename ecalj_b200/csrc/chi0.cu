@@ -43,15 +43,9 @@ static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc)
   memcpy(hb.data(), bt.off.data(), nb * sizeof(long long));
   memcpy(hb.data() + nb * sizeof(long long), bt.cnt.data(), nb * sizeof(int));
   memcpy(hb.data() + nb * (sizeof(long long) + sizeof(int)), bt.slab.data(), nb * sizeof(int));
-  if (ni) {
-    rc = check_cuda(cudaMemcpyAsync(g_x0_idx.p, bt.colidx.data(), ni * sizeof(int), cudaMemcpyHostToDevice, s), "H2D pair columns");
-    if (rc) return 0;
-    rc = check_cuda(cudaMemcpyAsync(g_x0_w.p, bt.wts.data(), ni * sizeof(double), cudaMemcpyHostToDevice, s), "H2D pair weights");
-    if (rc) return 0;
-  }
-  rc = check_cuda(cudaMemcpyAsync(g_x0_bins.p, hb.data(), bin_bytes, cudaMemcpyHostToDevice, s), "H2D bins");
-  if (rc) return 0;
-  // the pageable copies above are staged before returning, hb may die now
+  if ((rc = h2d(g_x0_idx.p, bt.colidx.data(), ni * sizeof(int), s))) return 0;
+  if ((rc = h2d(g_x0_w.p, bt.wts.data(), ni * sizeof(double), s))) return 0;
+  if ((rc = h2d(g_x0_bins.p, hb.data(), bin_bytes, s))) return 0;
   unsigned char* base = g_x0_bins.as<unsigned char>();
   p.bin_coff = reinterpret_cast<const long long*>(base);
   p.bin_woff = reinterpret_cast<const long long*>(base);
@@ -158,8 +152,6 @@ static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int n
   p.kch_per_split = (maxch + sk - 1) / sk;
   rc = zgemm_chi0_launch(p, nbins, herm, sk, s);
   if (rc) return rc;
-  // host vectors must outlive the async copies from pageable memory: they do,
-  // because pageable cudaMemcpyAsync stages the data before returning.
   return QSGW_OK;
 }
 
@@ -309,9 +301,16 @@ int chi0_lorentz_weights(int niw, const double* freq_i, int nk, const int* nocc,
     kp[k] = KPairs{c, std::max(nocc[k], 1), static_cast<int>(oo), static_cast<int>(uo), 0};
     // imaginary axis: w = -2 de / (de^2 + w^2) / nk has the sign of -de, de between the extremes of this k
     if (classes && nocc[k] > 0 && nun[k] > 0) {
-      const auto o = std::minmax_element(eocc + oo, eocc + oo + nocc[k]);
-      const auto u = std::minmax_element(eunocc + uo, eunocc + uo + nun[k]);
-      cl |= (*u.second - *o.first > 0.0 ? 1 : 0) | (*u.first - *o.second < 0.0 ? 2 : 0);
+      double olo = INFINITY, ohi = -INFINITY, ulo = INFINITY, uhi = -INFINITY;
+      for (int i = 0; i < nocc[k]; ++i) {              // fmin and fmax pass a NaN energy by, as its pairs have no sign
+        olo = std::fmin(olo, eocc[oo + i]);
+        ohi = std::fmax(ohi, eocc[oo + i]);
+      }
+      for (int i = 0; i < nun[k]; ++i) {
+        ulo = std::fmin(ulo, eunocc[uo + i]);
+        uhi = std::fmax(uhi, eunocc[uo + i]);
+      }
+      cl |= (uhi > olo ? 1 : 0) | (ulo < ohi ? 2 : 0);
     }
     c += static_cast<long long>(nocc[k]) * nun[k];
     oo += nocc[k];

@@ -74,6 +74,37 @@ def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col, ncoun
     assert np.linalg.norm(out[1] - out[0]) <= 6 * 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** -28 * inc + 1e-14 * np.linalg.norm(r0)
 
 
+@pytest.mark.parametrize("ncoun", [60, 1500])                # the FP64 engine's route and the int8 one
+def test_x0gemm_recorded_in_a_graph(qsgw, i8, ncoun):
+    """A recorded call replays with its own copy of the pair tables."""
+    import torch
+    rng = np.random.default_rng(ncoun)
+    n, nm, nq, nwhis = 40, 4, 6, 5
+    z = qsgw.to_device(_rc(rng, n, nm, nq))
+    tabs = [rng.integers(1, nm + 1, ncoun), rng.integers(1, nq + 1, ncoun), np.ones(ncoun, int),
+            *(2 * [rng.integers(1, nwhis + 1, ncoun)]), np.arange(1, ncoun + 1)]
+    w = rng.uniform(0.1, 1, ncoun)
+    r = torch.zeros(n * n * (nwhis + 1), dtype=torch.complex128, device="cuda")
+    i8(4)
+    call = lambda: qsgw.x0gemm(r, n, 1, n, nwhis, 1, 1, nm, z, 1, 1, ncoun, *tabs, w, zmel_shape=(n, nm, nq),
+                               device=True)
+    call()
+    qsgw.synchronize()
+    once = r.clone()
+    qsgw.graph_begin()
+    call()
+    qsgw.graph_end()
+    w[:] = 0.0
+    junk = [np.full(200000, 7) for _ in range(20)]             # whatever reuses the host tables' memory
+    r.zero_()
+    for _ in range(2):
+        qsgw.graph_launch()
+    qsgw.synchronize()
+    qsgw.graph_destroy()
+    assert len(junk) == 20
+    assert torch.linalg.vector_norm(r - 2 * once) <= 1e-12 * torch.linalg.vector_norm(once)
+
+
 def _sigma(qsgw, t, wi, wr, n, nm, ntq, keepwv=False):
     nwxi, nwx, ntmax = sched.get_nwx(t["omega"], t["ekc"], t["freq_r"], t["ef"], t["esmr"])
     if keepwv:
