@@ -4,9 +4,9 @@
 //
 // Parallel cyclic block Jacobi.  The matrix is cut into blocks of 16 rows; a
 // step pairs the blocks by a round-robin tournament (a sweep meets every
-// pair of blocks once) and is two kernels: jacobi_solve_kernel runs one
-// sweep of plane rotations over the 32 x 32 diagonal problem of each pair in
-// shared memory and leaves its unitary U, jacobi_apply_kernel forms
+// pair of blocks once) and is two kernels: jacobi_solve_kernel runs the
+// plane rotations of the 32 x 32 diagonal problem of each pair in shared
+// memory and leaves its unitary U, jacobi_apply_kernel forms
 // A <- U^H A U and V <- V U block by block.  A plane rotation first removes
 // the phase of a_pq, then applies the real Jacobi rotation with
 // t = sgn(tau) / (|tau| + sqrt(1 + tau^2)).  Sweeps stop when the
@@ -14,12 +14,18 @@
 //
 // What bounds it: chains of dependent steps, not arithmetic.  Rotations
 // between global steps cost a launch and an L2 round trip each (3.9 us at
-// n = 260, N-1 of them a sweep); inside a block's 32 x 32 problem a step is
-// two barriers and the angle's square roots (0.9 us).  Programmatic
-// dependent launch overlaps the launches.  n = 260: 29 us a solve and 10 us
-// an update, 17 of them a sweep: 10.0 ms (14.1 with a global step per
-// rotation set, 46.3 with three launches for each).  Angles formed in FP32
-// (rotations normalised in FP64) did not converge at n = 160.
+// n = 260, N-1 of them a sweep); inside a block's 32 x 32 problem a set of
+// rotations is two barriers and the angle's square roots (0.9 us).  So a
+// step rotates only the 256 pairs between its two blocks (16 sets), and the
+// pairs inside the blocks once a sweep: the sweeps needed are those of all
+// 31 sets in every step (15 against 16 at n = 260 with eigenvalues over five
+// decades, 30 against 29 with four eigenvalues in all), their length half.
+// The angles have a warp of their own, which forms the next set's while the
+// others bring U up to date.  Programmatic dependent launch overlaps the
+// launches.  n = 260: 23 us a step, 17 steps a sweep: 5.9 ms (10.0 with 31
+// sets in every step, 14.1 with a global step per rotation set, 46.3 with
+// three launches for each); updates by 128 threads a tile 6.2 ms.  Angles
+// formed in FP32 (rotations normalised in FP64) did not converge at n = 160.
 // The generalised problem (-v) z = lambda O z is reduced with O^-1/2 built
 // from a Jacobi solve of O.
 #include <algorithm>
@@ -76,6 +82,8 @@ __device__ __forceinline__ void rotate(double2& xp, double2& xq, const Rot& r, d
 }
 
 constexpr int JB = 16, JW = 2 * JB, JP = JW + 1;     // block width, pair width, shared-memory pitch
+constexpr int JT = JB * JB + 32;                     // threads of the solve: the 2 x 2 blocks and a warp for the angles
+constexpr int JA = 256, JV = JW * JB / JA;             // threads of an update, columns of its 2-row strips
 
 // global index of slot i (0..31) of the block pair (P, Q): P's rows, then Q's; n for an absent one
 __device__ __forceinline__ int slot_index(int i, int P, int Q, int n) {
@@ -83,63 +91,94 @@ __device__ __forceinline__ int slot_index(int i, int P, int Q, int n) {
   return g < n ? g : n;
 }
 
-// One sweep of the 32-slot problem of every block pair of step t; U[pair] (32 x 32, column-major) <- its
-// unitary.  Absent slots are zero rows and columns: nothing rotates with them.  Thread = one 2 x 2 block
-// of a step; two copies of the problem, as a step's angles come from blocks other threads are rotating.
+// The plane rotations of step t for every block pair (P, Q): the 16 x 16 pairs between the blocks, in the
+// first step of a sweep those inside the blocks as well, so that a sweep meets each pair once.  U[pair]
+// (32 x 32, column-major) <- the unitary.  Absent slots are zero rows and columns: nothing rotates with
+// them.  Thread = one 2 x 2 block of a rotation set, the ninth warp the set's angles; two copies of the
+// problem, as a set's angles come from blocks other threads are rotating.  U takes a set's rotations while
+// the next angles are formed.
 // No __restrict__ on A: the previous kernel, which may still run when these blocks start, writes it.
-__global__ void __launch_bounds__(JB * JB) jacobi_solve_kernel(const double2* A, double2* U, int n, int ne, int t) {
+__global__ void __launch_bounds__(JT) jacobi_solve_kernel(const double2* A, double2* U, int n, int ne, int t) {
   extern __shared__ double2 jac_smem[];
   double2* sa[2] = {jac_smem, jac_smem + JW * JP};
   double2* su = jac_smem + 2 * JW * JP;
   __shared__ Rot rot[JB];
-  const int tid = threadIdx.x, kb = tid & (JB - 1), lb = tid / JB;
+  const int tid = threadIdx.x, kb = tid & (JB - 1), lb = (tid / JB) & (JB - 1);
+  const bool work = tid < JB * JB, angle = tid >= JB * JB && tid < JB * JB + JB;
   int P, Q;
   pair_of(t, blockIdx.x, ne, P, Q);
+  const bool all = t == 0;                              // pairs inside the blocks too
+  const int nset = all ? JW - 1 : JB;
+  auto pair = [&](int st, int k, int& p, int& q) {
+    if (all) {
+      pair_of(st, k, JW, p, q);
+    } else {
+      p = k;
+      q = JB + ((k + st) & (JB - 1));
+    }
+  };
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (work) {
 #pragma unroll
-  for (int e = 0; e < JW * JW / (JB * JB); ++e) {
-    const int i = tid & (JW - 1), j = tid / JW + e * (JB * JB / JW);
-    const int gi = slot_index(i, P, Q, n), gj = slot_index(j, P, Q, n);
-    sa[0][i + j * JP] = (gi < n && gj < n) ? A[gi + static_cast<long long>(gj) * n] : make_double2(0.0, 0.0);
-    su[i + j * JP] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+    for (int e = 0; e < JW * JW / (JB * JB); ++e) {
+      const int i = tid & (JW - 1), j = tid / JW + e * (JB * JB / JW);
+      const int gi = slot_index(i, P, Q, n), gj = slot_index(j, P, Q, n);
+      sa[0][i + j * JP] = (gi < n && gj < n) ? A[gi + static_cast<long long>(gj) * n] : make_double2(0.0, 0.0);
+      su[i + j * JP] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+    }
   }
   __syncthreads();
-  for (int st = 0; st < JW - 1; ++st) {
-    const double2* cur = sa[st & 1];
-    double2* nxt = sa[(st & 1) ^ 1];
-    if (tid < JB) {
-      int p, q;
-      pair_of(st, tid, JW, p, q);
-      rot[tid] = rotation(cur, JP, p, q);
-    }
-    int p0, p1, q0, q1;
-    pair_of(st, kb, JW, p0, p1);
-    pair_of(st, lb, JW, q0, q1);
-    double2 a00 = cur[p0 + q0 * JP], a01 = cur[p0 + q1 * JP], a10 = cur[p1 + q0 * JP], a11 = cur[p1 + q1 * JP];
-    __syncthreads();
-    const Rot r = rot[kb], c = rot[lb];
-    rotate(a00, a01, c, c.ph);
-    rotate(a10, a11, c, c.ph);
-    const double2 cph = make_double2(r.ph.x, -r.ph.y);              // rows: the conjugate phase
-    rotate(a00, a10, r, cph);
-    rotate(a01, a11, r, cph);
-    nxt[p0 + q0 * JP] = a00;
-    nxt[p0 + q1 * JP] = a01;
-    nxt[p1 + q0 * JP] = a10;
-    nxt[p1 + q1 * JP] = a11;
+  Rot c{1.0, 0.0, make_double2(1.0, 0.0)};              // the columns' rotation, still to be applied to U
+  int u0 = 0, u1 = 0;
+  auto rotate_u = [&]() {                               // U's columns u0, u1: rows kb, kb + 16
     if (c.s != 0.0) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {                                  // U's columns q0, q1: rows kb, kb + 16
-        double2 *xp = su + (kb + h * JB) + q0 * JP, *xq = su + (kb + h * JB) + q1 * JP;
+      for (int h = 0; h < 2; ++h) {
+        double2 *xp = su + (kb + h * JB) + u0 * JP, *xq = su + (kb + h * JB) + u1 * JP;
         double2 x = *xp, y = *xq;
         rotate(x, y, c, c.ph);
         *xp = x;
         *xq = y;
       }
     }
+  };
+  for (int st = 0; st < nset; ++st) {
+    const double2* cur = sa[st & 1];
+    double2* nxt = sa[(st & 1) ^ 1];
+    if (angle) {
+      int p, q;
+      pair(st, kb, p, q);
+      rot[kb] = rotation(cur, JP, p, q);
+    }
+    int p0, p1, q0, q1;
+    double2 a00, a01, a10, a11;
+    if (work) {
+      pair(st, kb, p0, p1);
+      pair(st, lb, q0, q1);
+      a00 = cur[p0 + q0 * JP], a01 = cur[p0 + q1 * JP], a10 = cur[p1 + q0 * JP], a11 = cur[p1 + q1 * JP];
+      rotate_u();
+    }
+    __syncthreads();
+    if (work) {
+      const Rot r = rot[kb];
+      c = rot[lb];
+      u0 = q0, u1 = q1;
+      rotate(a00, a01, c, c.ph);
+      rotate(a10, a11, c, c.ph);
+      const double2 cph = make_double2(r.ph.x, -r.ph.y);              // rows: the conjugate phase
+      rotate(a00, a10, r, cph);
+      rotate(a01, a11, r, cph);
+      nxt[p0 + q0 * JP] = a00;
+      nxt[p0 + q1 * JP] = a01;
+      nxt[p1 + q0 * JP] = a10;
+      nxt[p1 + q1 * JP] = a11;
+    }
     __syncthreads();
   }
+  if (!work) return;
+  rotate_u();
+  asm volatile("bar.sync 1, %0;" ::"n"(JB * JB) : "memory");          // the working warps
   double2* Up = U + static_cast<long long>(blockIdx.x) * JW * JW;
 #pragma unroll
   for (int e = 0; e < JW * JW / (JB * JB); ++e) {
@@ -148,27 +187,27 @@ __global__ void __launch_bounds__(JB * JB) jacobi_solve_kernel(const double2* A,
   }
 }
 
-// out(2 x 4 per thread) = op(X) Y for 32 x 32 tiles in shared memory; CONJ: X^H
+// out(2 x JV per thread) = op(X) Y for 32 x 32 tiles in shared memory; CONJ: X^H
 template <bool CONJ>
-__device__ __forceinline__ void tile_product(double2 (&o)[2][4], const double2* X, const double2* Y, int i0, int j0) {
+__device__ __forceinline__ void tile_product(double2 (&o)[2][JV], const double2* X, const double2* Y, int i0, int j0) {
 #pragma unroll
   for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) o[u][v] = make_double2(0.0, 0.0);
+    for (int v = 0; v < JV; ++v) o[u][v] = make_double2(0.0, 0.0);
 #pragma unroll 4
   for (int k = 0; k < JW; ++k) {
-    double2 x[2], y[4];
+    double2 x[2], y[JV];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       x[u] = CONJ ? X[k + (i0 + 16 * u) * JP] : X[i0 + 16 * u + k * JP];
       if (CONJ) x[u].y = -x[u].y;
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) y[v] = Y[k + (j0 + v) * JP];
+    for (int v = 0; v < JV; ++v) y[v] = Y[k + (j0 + v) * JP];
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
+      for (int v = 0; v < JV; ++v) {
         o[u][v].x += x[u].x * y[v].x - x[u].y * y[v].y;
         o[u][v].y += x[u].x * y[v].y + x[u].y * y[v].x;
       }
@@ -177,11 +216,11 @@ __device__ __forceinline__ void tile_product(double2 (&o)[2][4], const double2* 
 
 // A <- U^H A U (blocks x < npair^2: pair of rows k, pair of columns l, in place) and V <- V U (the others: 32
 // rows of V, pair l)
-__global__ void __launch_bounds__(128) jacobi_apply_kernel(double2* A, double2* V, const double2* U, int n, int ne,
+__global__ void __launch_bounds__(JA) jacobi_apply_kernel(double2* A, double2* V, const double2* U, int n, int ne,
                                                            int t, int npair) {
   extern __shared__ double2 jac_smem[];
   double2 *sx = jac_smem, *sl = sx + JW * JP, *sk = sl + JW * JP;
-  const int tid = threadIdx.x, i0 = tid & 15, j0 = (tid >> 4) * 4;
+  const int tid = threadIdx.x, i0 = tid & 15, j0 = (tid >> 4) * JV;
   const bool isA = static_cast<int>(blockIdx.x) < npair * npair;
   const int b = isA ? blockIdx.x : blockIdx.x - npair * npair;
   const int l = b % npair, k = b / npair;               // V: k = row block
@@ -192,29 +231,29 @@ __global__ void __launch_bounds__(128) jacobi_apply_kernel(double2* A, double2* 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   double2* M = isA ? A : V;
 #pragma unroll
-  for (int e = 0; e < JW * JW / 128; ++e) {
-    const int i = tid & (JW - 1), j = tid / JW + e * (128 / JW);
+  for (int e = 0; e < JW * JW / JA; ++e) {
+    const int i = tid & (JW - 1), j = tid / JW + e * (JA / JW);
     const int gi = isA ? slot_index(i, R, S, n) : (k * JW + i < n ? k * JW + i : n), gj = slot_index(j, P, Q, n);
     sx[i + j * JP] = (gi < n && gj < n) ? M[gi + static_cast<long long>(gj) * n] : make_double2(0.0, 0.0);
     sl[i + j * JP] = U[static_cast<long long>(l) * JW * JW + i + j * JW];
     if (isA) sk[i + j * JP] = U[static_cast<long long>(k) * JW * JW + i + j * JW];
   }
   __syncthreads();
-  double2 o[2][4];
+  double2 o[2][JV];
   tile_product<false>(o, sx, sl, i0, j0);
   if (isA) {
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sx[i0 + 16 * u + (j0 + v) * JP] = o[u][v];
+      for (int v = 0; v < JV; ++v) sx[i0 + 16 * u + (j0 + v) * JP] = o[u][v];
     __syncthreads();
     tile_product<true>(o, sk, sx, i0, j0);
   }
 #pragma unroll
   for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
+    for (int v = 0; v < JV; ++v) {
       const int i = i0 + 16 * u;
       const int gi = isA ? slot_index(i, R, S, n) : (k * JW + i < n ? k * JW + i : n), gj = slot_index(j0 + v, P, Q, n);
       if (gi < n && gj < n) M[gi + static_cast<long long>(gj) * n] = o[u][v];
@@ -308,9 +347,9 @@ static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vecto
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t solve{}, apply{};
   solve.gridDim = dim3(static_cast<unsigned>(npair));
-  solve.blockDim = dim3(JB * JB);
+  solve.blockDim = dim3(JT);
   apply.gridDim = dim3(static_cast<unsigned>(npair * npair + nrow * npair));
-  apply.blockDim = dim3(128);
+  apply.blockDim = dim3(JA);
   for (cudaLaunchConfig_t* c : {&solve, &apply}) {
     c->dynamicSmemBytes = SMEM;
     c->stream = s;
@@ -320,7 +359,8 @@ static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vecto
   set_identity_kernel<<<grid_for(static_cast<long long>(n) * n), 256, 0, s>>>(V, n, n);
   count_launch();
   bool converged = (n <= 1);
-  for (int sweep = 0; sweep < 40 && !converged; ++sweep) {
+  // many equal eigenvalues are the slow case: 23, 30 and 34 sweeps at n = 64, 260 and 400 with four in all
+  for (int sweep = 0; sweep < 60 && !converged; ++sweep) {
     for (int t = 0; t < ne - 1; ++t) {
       QSGW_CUDA(cudaLaunchKernelEx(&solve, jacobi_solve_kernel, static_cast<const double2*>(cur), U, n, ne, t));
       QSGW_CUDA(cudaLaunchKernelEx(&apply, jacobi_apply_kernel, cur, V, static_cast<const double2*>(U), n, ne, t, npair));

@@ -25,3 +25,20 @@ def test_jacobi_block_edges(qsgw, n, pad):
     assert np.abs(v @ z[:n] - z[:n] * lam).max() <= tol * norm
     assert np.abs(z[:n].conj().T @ z[:n] - np.eye(n)).max() <= tol
     assert np.all(z[n:] == 7.0)
+
+
+@pytest.mark.parametrize("n", [48, 130, 257])
+def test_jacobi_equal_eigenvalues(qsgw, n):
+    """Four distinct eigenvalues: rotations within an eigenspace are arbitrary, the spaces are not."""
+    rng = np.random.default_rng(n)
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))
+    lam = np.repeat([7.0, 5.0, 2.0, 1.0], (n + 3) // 4)[:n]
+    v = (q * lam) @ q.conj().T
+    v = np.asfortranarray(0.5 * (v + v.conj().T))
+    d = qsgw.to_device(v)
+    got = qsgw.zhegv_d(d, n)
+    z = qsgw.from_device(d, v.shape)
+    tol = 64 * n * np.finfo(float).eps
+    assert np.abs(got - lam).max() <= tol * lam[0]
+    assert np.abs((z * got) @ z.conj().T - v).max() <= tol * lam[0]
+    assert np.abs(z.conj().T @ z - np.eye(n)).max() <= tol
