@@ -200,7 +200,7 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
   rc = g_zm_atoms.ensure(natom * sizeof(ZmelAtomDev));
   if (rc) return rc;
   if ((rc = g_zm_t.ensure(static_cast<size_t>(tsize) * sizeof(double2)))) return rc;
-  QSGW_CUDA(cudaMemcpyAsync(g_zm_atoms.p, h.data(), natom * sizeof(ZmelAtomDev), cudaMemcpyHostToDevice, s));
+  if ((rc = h2d(g_zm_atoms.p, h.data(), natom * sizeof(ZmelAtomDev), s))) return rc;   // h dies on return: a graph keeps its own copy
   // cphiq columns and one product function's valence block (99 KB at 96 channels)
   auto smem_of = [](int nv) {
     return static_cast<size_t>(nv) * ZM_TQ * sizeof(double2) + static_cast<size_t>(nv + 1) * nv * sizeof(double);

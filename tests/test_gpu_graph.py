@@ -92,3 +92,37 @@ def test_graph_refuses_scratch_growth(qsgw):
     lib.chi0_lorentz_d(chi, N, niw, p["freq_i"], p["nk"], p["nocc"], p["nun"], p["eocc_h"], p["eun_h"], z)
     lib.synchronize()
     assert float(torch.linalg.vector_norm(chi)) > 0
+
+
+def _replays_as_recorded(lib, call, out, spoil=lambda: None):
+    """`call` recorded, its host tables spoilt and their memory reused: the replay still gives the eager result."""
+    call()                                                # sizes the scratch
+    lib.synchronize()
+    ref = out.clone()
+    lib.graph_begin()
+    call()
+    lib.graph_end()
+    spoil()
+    junk = [np.full(50000, 7) for _ in range(20)]
+    out.zero_()
+    lib.graph_launch()
+    lib.synchronize()
+    lib.graph_destroy()
+    assert len(junk) == 20 and float(ref.abs().max()) > 0
+    assert rel_fro(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-13
+
+
+def _rc(rng, *shape):
+    return np.asfortranarray(rng.standard_normal(shape) + 1j * rng.standard_normal(shape))
+
+
+def test_muffin_tin_elements_recorded_in_a_graph(qsgw):
+    import torch
+    rng = np.random.default_rng(3)
+    nlnm, md, nm, ntp0 = 7, 5, 4, 3
+    ppb = [torch.from_numpy(rng.standard_normal(nlnm * nlnm * md)).cuda() for _ in range(2)]
+    atoms = [dict(nlnm=nlnm, nc=1, nv=6, ias=1 + 6 * i, ics=0, ims=1 + md * i, mdim=md, ncore=0, phase=1j ** i, ppb_d=p)
+             for i, p in enumerate(ppb)]
+    cphim, cphiq = qsgw.to_device(_rc(rng, 12, nm)), qsgw.to_device(_rc(rng, 12, ntp0))
+    zt = torch.zeros(2 * md * nm * ntp0, dtype=torch.complex128, device="cuda")
+    _replays_as_recorded(qsgw, lambda: qsgw.zmel_mt_d(zt, 2 * md, 1, nm, 0, ntp0, cphim, 12, cphiq, 12, atoms), zt)
