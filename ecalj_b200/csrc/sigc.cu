@@ -777,11 +777,12 @@ extern "C" int qsgw_sxcf_wgtim_d(double* wgtim_d, int niw, int ns1, int ns2, int
   if (rc) return rc;
   double* dt = g_sc_tabs.as<double>();
   double *d_x = dt, *d_wt = dt + niw, *d_ex = dt + 2 * niw, *d_om = dt + 3 * niw, *d_ekc = d_om + ntqxx;
-  QSGW_CUDA(cudaMemcpyAsync(d_x, freqx, niw * sizeof(double), cudaMemcpyHostToDevice, s));
-  QSGW_CUDA(cudaMemcpyAsync(d_wt, wwx, niw * sizeof(double), cudaMemcpyHostToDevice, s));
-  QSGW_CUDA(cudaMemcpyAsync(d_ex, expa, niw * sizeof(double), cudaMemcpyHostToDevice, s));
-  QSGW_CUDA(cudaMemcpyAsync(d_om, omega, ntqxx * sizeof(double), cudaMemcpyHostToDevice, s));
-  QSGW_CUDA(cudaMemcpyAsync(d_ekc, ekc, nekc * sizeof(double), cudaMemcpyHostToDevice, s));
+  // the caller's tables: a graph keeps its own copies
+  if ((rc = h2d(d_x, freqx, niw * sizeof(double), s))) return rc;
+  if ((rc = h2d(d_wt, wwx, niw * sizeof(double), s))) return rc;
+  if ((rc = h2d(d_ex, expa, niw * sizeof(double), s))) return rc;
+  if ((rc = h2d(d_om, omega, ntqxx * sizeof(double), s))) return rc;
+  if ((rc = h2d(d_ekc, ekc, nekc * sizeof(double), s))) return rc;
   const long long ncol = static_cast<long long>(nm) * ntqxx;
   wgtim_kernel<<<static_cast<int>((ncol + 7) / 8), 256, 0, s>>>(wgtim_d, niw, ns1, nm, ntqxx, nctot, d_om, d_ekc,
                                                                     esmr, wkkr, ua, d_x, d_wt, d_ex);

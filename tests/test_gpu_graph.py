@@ -126,3 +126,18 @@ def test_muffin_tin_elements_recorded_in_a_graph(qsgw):
     cphim, cphiq = qsgw.to_device(_rc(rng, 12, nm)), qsgw.to_device(_rc(rng, 12, ntp0))
     zt = torch.zeros(2 * md * nm * ntp0, dtype=torch.complex128, device="cuda")
     _replays_as_recorded(qsgw, lambda: qsgw.zmel_mt_d(zt, 2 * md, 1, nm, 0, ntp0, cphim, 12, cphiq, 12, atoms), zt)
+
+
+def test_imaginary_axis_weights_recorded_in_a_graph(qsgw):
+    import torch
+    t = synth.sigc_task(8, 3, 10, 6, 30, seed=2, esmr=0.02, ef=0.05)
+    tabs = [np.array(t[k]) for k in ("omega", "ekc", "x", "wx", "expa")]
+    om, ek, x, wx, ex = tabs
+    out = torch.zeros(7 * 10 * 3, dtype=torch.float64, device="cuda")
+
+    def spoil():
+        for a in tabs:
+            a[:] = 0.5
+
+    _replays_as_recorded(qsgw, lambda: qsgw.sxcf_wgtim_d(out, 6, 1, 10, 3, 0, om, ek, t["esmr"], 1 / 8, t["ua"], x, wx,
+                                                         ex), out, spoil)
