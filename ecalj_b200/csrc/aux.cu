@@ -90,8 +90,8 @@ extern "C" int qsgw_sxcf_exchange_d(double* zsec_d, int ntq, const double* zmel_
   rc = g_ex_tab.ensure((ngb + nm) * sizeof(double));
   if (rc) return rc;
   double* dv = g_ex_tab.as<double>();
-  QSGW_CUDA(cudaMemcpyAsync(dv, vcoud, ngb * sizeof(double), cudaMemcpyHostToDevice, s));
-  QSGW_CUDA(cudaMemcpyAsync(dv + ngb, wtff.data(), nm * sizeof(double), cudaMemcpyHostToDevice, s));
+  if ((rc = h2d(dv, vcoud, ngb * sizeof(double), s))) return rc;   // wtff dies on return: a graph keeps its own copies
+  if ((rc = h2d(dv + ngb, wtff.data(), nm * sizeof(double), s))) return rc;
   exchange_scale_kernel<<<grid_for(static_cast<long long>(ngb) * ncol), 256, 0, s>>>(
       g_ex_vz.as<double2>(), reinterpret_cast<const double2*>(zmel_d), dv, dv + ngb, ngb, nm, ncol);
   count_launch();

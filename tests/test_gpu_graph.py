@@ -141,3 +141,21 @@ def test_imaginary_axis_weights_recorded_in_a_graph(qsgw):
 
     _replays_as_recorded(qsgw, lambda: qsgw.sxcf_wgtim_d(out, 6, 1, 10, 3, 0, om, ek, t["esmr"], 1 / 8, t["ua"], x, wx,
                                                          ex), out, spoil)
+
+
+def test_exchange_recorded_in_a_graph(qsgw):
+    import torch
+    rng = np.random.default_rng(5)
+    ngb, nm, ntq = 20, 9, 4
+    z = qsgw.to_device(_rc(rng, ngb, nm, ntq))
+    vcoud, ekc = 10 ** rng.uniform(-2, 3, ngb), np.sort(rng.uniform(-1, 1, nm))
+    zsec = torch.zeros(ntq * ntq, dtype=torch.complex128, device="cuda")
+
+    def call():
+        zsec.zero_()
+        qsgw.sxcf_exchange_d(zsec, ntq, z, ngb, 1, nm, ntq, vcoud, ekc, 0, 0.1, 0.02, 0.125)
+
+    def spoil():
+        vcoud[:] = 1.0
+
+    _replays_as_recorded(qsgw, call, zsec, spoil)
