@@ -23,6 +23,10 @@ struct ZmelAtomDev {
 
 constexpr int ZM_NVMAX = 96;      // valence channels per atom
 constexpr int ZM_TQ = 16;         // target columns per block of the first product
+// Target columns are taken in slabs: T of a slab fits this scratch (unless ZM_TQ columns are more), and a slab is
+// one batch of the second product's grid (65 535 at most).  100 atoms of 25 channels and 60 functions need 2.4 MB a column.
+constexpr size_t ZM_SCRATCH = size_t(256) << 20;
+constexpr int ZM_SLAB = 65535 / ZM_TQ * ZM_TQ;
 
 // T(itp, i, a) = sum_b ppb(nc+b, nc+a, i) cphiq(ias+b, itp) (m_zmel.f90:358), a fastest, and the core rows
 // zmelt(ims+i, it, itp) = phase sum_b ppb(nc+b, it-ics, i) cphiq(b, itp) (:383).  One block per (product
@@ -180,7 +184,7 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
   std::vector<ZmelAtomDev> h(natom);
   const bool valence = nm2v >= nm1v;
   int nvmax = 1, mdmax = 0;
-  long long tsize = 0;
+  long long tcol = 0;                                              // T of one target column
   for (int ia = 0; ia < natom; ++ia) {
     const qsgw_zmel_atom& a = atoms[ia];
     QSGW_ARG(a.nv >= 1 && a.nv <= ZM_NVMAX && a.nc >= 0 && a.nc + a.nv <= a.nlnm && a.ppb_d,
@@ -189,17 +193,20 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
              "zmel_mt: atom %d offsets outside zmelt/cphi", ia);
     QSGW_ARG(a.ncore <= a.nc, "zmel_mt: atom %d ncore=%d > nc=%d", ia, a.ncore, a.nc);
     h[ia] = ZmelAtomDev{a.ppb_d, a.nlnm, a.nc, a.nv, a.ias, a.ics, a.ims, a.mdim, a.ncore, a.phase_re, a.phase_im,
-                        tsize};
-    tsize += static_cast<long long>(a.nv) * std::max(a.mdim, 0) * ntp0;
+                        tcol};
+    tcol += static_cast<long long>(a.nv) * std::max(a.mdim, 0);
     nvmax = std::max(nvmax, a.nv);
     mdmax = std::max(mdmax, a.mdim);
   }
   if (mdmax <= 0) return QSGW_OK;
+  const long long fit = static_cast<long long>(ZM_SCRATCH / sizeof(double2)) / tcol / ZM_TQ * ZM_TQ;
+  const int slab = static_cast<int>(std::min<long long>(ntp0, std::max<long long>(ZM_TQ, std::min<long long>(fit, ZM_SLAB))));
+  for (ZmelAtomDev& a : h) a.toff *= slab;
   cudaStream_t s = ctx().stream;
   const int nmtot = nm2 - nm1 + 1;
   rc = g_zm_atoms.ensure(natom * sizeof(ZmelAtomDev));
   if (rc) return rc;
-  if ((rc = g_zm_t.ensure(static_cast<size_t>(tsize) * sizeof(double2)))) return rc;
+  if ((rc = g_zm_t.ensure(static_cast<size_t>(tcol) * slab * sizeof(double2)))) return rc;
   if ((rc = h2d(g_zm_atoms.p, h.data(), natom * sizeof(ZmelAtomDev), s))) return rc;   // h dies on return: a graph keeps its own copy
   // cphiq columns and one product function's valence block (99 KB at 96 channels)
   auto smem_of = [](int nv) {
@@ -209,23 +216,27 @@ extern "C" int qsgw_zmel_mt_d(double* zmelt_d, int nbloch, int nm1, int nm2, int
   rc = smem_limit_once(reinterpret_cast<const void*>(zmel_ppb_kernel), static_cast<int>(smem_of(ZM_NVMAX)), attr);
   if (rc) return rc;
   const size_t smem = smem_of(nvmax);
-  double2* zt = reinterpret_cast<double2*>(zmelt_d);
-  zmel_ppb_kernel<<<dim3(mdmax, (ntp0 + ZM_TQ - 1) / ZM_TQ, natom), 256, smem, s>>>(
-      g_zm_t.as<double2>(), zt, nbloch, nm1, nmtot, nctot, ntp0, nm1c, nm2c,
-      reinterpret_cast<const double2*>(cphiq_d), ldq, g_zm_atoms.as<ZmelAtomDev>(), nvmax);
-  count_launch();
-  QSGW_LAUNCH_CHECK("zmel_ppb_kernel");
-  if (!valence) return QSGW_OK;
-  // zmelt(ims.., it, itp) = phase sum_a T(itp, i, a) conj(cphim(ias+a, it)) (:365): per target column one
-  // mdim x nmv product over nv
-  for (int ia = 0; ia < natom; ++ia) {
-    const ZmelAtomDev& a = h[ia];
-    rc = zgemm_f64(1, 3, a.mdim, nm2v - nm1v + 1, a.nv, make_double2(a.ph_re, a.ph_im), g_zm_t.as<double2>() + a.toff,
-                   a.nv, static_cast<long long>(a.nv) * a.mdim,
-                   reinterpret_cast<const double2*>(cphim_d) + (a.ias - 1), ldm, 0, make_double2(0.0, 0.0),
-                   zt + (a.ims - 1) + static_cast<long long>(nm1v - nm1) * nbloch, nbloch,
-                   static_cast<long long>(nbloch) * nmtot, ntp0, s);
-    if (rc) return rc;
+  for (int p0 = 0; p0 < ntp0; p0 += slab) {
+    const int np = std::min(slab, ntp0 - p0);
+    double2* zt = reinterpret_cast<double2*>(zmelt_d) + static_cast<long long>(p0) * nbloch * nmtot;
+    zmel_ppb_kernel<<<dim3(mdmax, (np + ZM_TQ - 1) / ZM_TQ, natom), 256, smem, s>>>(
+        g_zm_t.as<double2>(), zt, nbloch, nm1, nmtot, nctot, np, nm1c, nm2c,
+        reinterpret_cast<const double2*>(cphiq_d) + static_cast<long long>(p0) * ldq, ldq, g_zm_atoms.as<ZmelAtomDev>(),
+        nvmax);
+    count_launch();
+    QSGW_LAUNCH_CHECK("zmel_ppb_kernel");
+    if (!valence) continue;
+    // zmelt(ims.., it, itp) = phase sum_a T(itp, i, a) conj(cphim(ias+a, it)) (:365): per target column one
+    // mdim x nmv product over nv
+    for (int ia = 0; ia < natom; ++ia) {
+      const ZmelAtomDev& a = h[ia];
+      rc = zgemm_f64(1, 3, a.mdim, nm2v - nm1v + 1, a.nv, make_double2(a.ph_re, a.ph_im),
+                     g_zm_t.as<double2>() + a.toff, a.nv, static_cast<long long>(a.nv) * a.mdim,
+                     reinterpret_cast<const double2*>(cphim_d) + (a.ias - 1), ldm, 0, make_double2(0.0, 0.0),
+                     zt + (a.ims - 1) + static_cast<long long>(nm1v - nm1) * nbloch, nbloch,
+                     static_cast<long long>(nbloch) * nmtot, np, s);
+      if (rc) return rc;
+    }
   }
   return QSGW_OK;
 }

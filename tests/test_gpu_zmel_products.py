@@ -38,3 +38,24 @@ def test_muffin_tin_products(qsgw, nm1, nm2, nctot, ntp0):
         qsgw.zmel_m2e_d(out, zt, nbloch, 35, nm, ntp0, qsgw.to_device(m2e), False, conj)
         qsgw.synchronize()
         assert rel_fro(qsgw.from_device(out, (35, nm, ntp0)), zmel.zmel_m2e(ref, m2e, False, conj)) < 1e-13
+
+
+@pytest.mark.parametrize("nv,mdim,nm,ntp0", [(1, 1, 1, 65600),      # more targets than one batch of the grid takes
+                                             (96, 1500, 2, 300)])   # 690 MB of first products: several slabs
+def test_muffin_tin_target_slabs(qsgw, nv, mdim, nm, ntp0):
+    import torch
+    rng = np.random.default_rng(ntp0)
+    atom = dict(nc=0, nv=nv, ias=1, ics=0, ims=1, ncore=0)
+    ppb = rng.standard_normal((nv, nv, mdim))
+    cphim, cphiq = _rc(rng, nv, nm), _rc(rng, nv, ntp0)
+    t = np.tensordot(ppb, cphiq, axes=(0, 0))                 # (a, i, itp)
+    ref = np.tensordot(cphim.conj(), t, axes=(0, 0)).transpose(1, 0, 2)
+    zt = torch.zeros(mdim * nm * ntp0, dtype=torch.complex128, device="cuda")
+    dat = [dict(atom, nlnm=nv, mdim=mdim, phase=1.0, ppb_d=torch.from_numpy(ppb.reshape(-1, order="F").copy()).cuda())]
+    m, q = qsgw.to_device(cphim), qsgw.to_device(cphiq)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    qsgw.zmel_mt_d(zt, mdim, 1, nm, 0, ntp0, m, nv, q, nv, dat)
+    qsgw.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= 300 << 20
+    assert rel_fro(qsgw.from_device(zt, (mdim, nm, ntp0)), ref) < 1e-13
