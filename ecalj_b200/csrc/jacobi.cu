@@ -288,9 +288,40 @@ __global__ void set_identity_kernel(double2* V, long long ldv, int n) {
   }
 }
 
-__global__ void diag_kernel(const double2* A, long long lda, int n, double* d) {
+// the largest finite |Re|, |Im| of A as ordered bits (NaN and infinities are left to the norms)
+__global__ void absmax_kernel(const double2* __restrict__ A, long long lda, int n, unsigned long long* mx) {
+  double m = 0.0;
+  const long long nn = static_cast<long long>(n) * n;
+  for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < nn;
+       e += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const double2 v = A[e % n + e / n * lda];
+    const double x = fmax(fabs(v.x), fabs(v.y));
+    if (isfinite(x)) m = fmax(m, x);
+  }
+  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(mx, static_cast<unsigned long long>(__double_as_longlong(m)));
+}
+
+// The power of two that brings a small matrix up to entries of order one: squares of its entries would underflow.  A
+// large one stays: its squares overflow in the norm, which refuses it.
+__device__ __forceinline__ int small_exponent(const unsigned long long* mx) {
+  const double m = __longlong_as_double(static_cast<long long>(*mx));
+  return m > 0.0 ? min(ilogb(m), 0) : 0;
+}
+__global__ void scaled_copy_kernel(double2* __restrict__ out, const double2* __restrict__ A, long long lda, int n,
+                                   const unsigned long long* __restrict__ mx) {
+  const int ex = -small_exponent(mx);
+  const long long nn = static_cast<long long>(n) * n;
+  for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < nn;
+       e += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const double2 v = A[e % n + e / n * lda];
+    out[e] = make_double2(scalbn(v.x, ex), scalbn(v.y, ex));
+  }
+}
+
+__global__ void diag_kernel(const double2* A, long long lda, int n, const unsigned long long* mx, double* d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] = A[i + i * lda].x;
+  if (i < n) d[i] = scalbn(A[i + i * lda].x, small_exponent(mx));
 }
 
 // out(:, j) = V(:, perm[j]) * colscale[j]
@@ -327,17 +358,21 @@ static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vecto
   const int ne = nb + (nb & 1);                         // an odd block count pairs one block with an absent one
   const int npair = ne / 2, nrow = (n + JW - 1) / JW;
   const size_t nn = static_cast<size_t>(n) * n;
-  // working copy of A (ld n), then the pairs' unitaries
+  // working copy of A (ld n, scaled), then the pairs' unitaries
   int rc = g_jc_b.ensure((nn + static_cast<size_t>(npair) * JW * JW) * sizeof(double2));
   if (rc) return rc;
-  rc = g_jc_norm.ensure(2 * sizeof(double));
+  rc = g_jc_norm.ensure(2 * sizeof(double) + sizeof(unsigned long long));   // norms, largest entry
   if (rc) return rc;
   rc = g_jc_d.ensure(n * sizeof(double));
   if (rc) return rc;
   double2* cur = g_jc_b.as<double2>();
   double2* U = cur + nn;
-  const size_t row = static_cast<size_t>(n) * sizeof(double2);
-  QSGW_CUDA(cudaMemcpy2DAsync(cur, row, A, lda * sizeof(double2), row, n, cudaMemcpyDeviceToDevice, s));
+  unsigned long long* mx = reinterpret_cast<unsigned long long*>(g_jc_norm.as<double>() + 2);
+  QSGW_CUDA(cudaMemsetAsync(mx, 0, sizeof(*mx), s));
+  absmax_kernel<<<grid_for(static_cast<long long>(nn)), 256, 0, s>>>(A, lda, n, mx);
+  scaled_copy_kernel<<<grid_for(static_cast<long long>(nn)), 256, 0, s>>>(cur, A, lda, n, mx);
+  count_launch(2);
+  QSGW_LAUNCH_CHECK("scaled_copy_kernel");
   constexpr int SMEM = 3 * JW * JP * static_cast<int>(sizeof(double2));
   static uint64_t at_solve = 0, at_apply = 0;           // one bit per device
   if ((rc = smem_limit_once(reinterpret_cast<const void*>(jacobi_solve_kernel), SMEM, at_solve))) return rc;
@@ -383,7 +418,7 @@ static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vecto
     set_error("zhegv: Jacobi sweeps did not converge");
     return QSGW_ERR_NUMERIC;
   }
-  diag_kernel<<<(n + 127) / 128, 128, 0, s>>>(cur, n, n, g_jc_d.as<double>());
+  diag_kernel<<<(n + 127) / 128, 128, 0, s>>>(cur, n, n, mx, g_jc_d.as<double>());
   count_launch();
   d.resize(n);
   QSGW_CUDA(cudaMemcpyAsync(d.data(), g_jc_d.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));

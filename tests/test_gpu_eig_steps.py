@@ -42,3 +42,29 @@ def test_jacobi_equal_eigenvalues(qsgw, n):
     assert np.abs(got - lam).max() <= tol * lam[0]
     assert np.abs((z * got) @ z.conj().T - v).max() <= tol * lam[0]
     assert np.abs(z.conj().T @ z - np.eye(n)).max() <= tol
+
+
+@pytest.mark.parametrize("exp10", [-140, -155, -200, -300, 100])
+def test_jacobi_small_and_large_entries(qsgw, exp10):
+    """Rotations are chosen from squares of the entries: a small matrix is solved as its multiple of order one."""
+    n = 40
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    v = g + g.conj().T
+    d = qsgw.to_device(np.asfortranarray(v * 10.0 ** exp10))
+    lam = qsgw.zhegv_d(d, n) / 10.0 ** exp10
+    z = qsgw.from_device(d, v.shape)
+    tol = 64 * n * np.finfo(float).eps
+    norm = np.linalg.norm(v, 2)
+    assert np.abs(lam - np.linalg.eigvalsh(v)[::-1]).max() <= tol * norm
+    assert np.abs(v @ z - z * lam).max() <= tol * norm
+
+
+def test_jacobi_zero_and_non_finite(qsgw):
+    d = qsgw.to_device(np.zeros((20, 20), complex, order="F"))
+    assert np.array_equal(qsgw.zhegv_d(d, 20), np.zeros(20))
+    for bad in (np.nan, np.inf):
+        v = np.eye(20, dtype=complex, order="F") * 1e-200
+        v[3, 3] = bad
+        with pytest.raises(qsgw.QSGWError):
+            qsgw.zhegv_d(qsgw.to_device(v), 20)
