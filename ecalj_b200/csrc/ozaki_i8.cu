@@ -1581,8 +1581,9 @@ int chi0_split_i8(double2* C, long long ldc, long long c_bs, int M, int N, int r
     if (c <= maxsplit) cands.push_back(c);
   if (heur == 7 || heur > 8) cands.push_back(heur);
   char key[200];
-  std::snprintf(key, sizeof(key), "%s i8x%d M=%d N=%d bins=%d chunks~2^%.3f", tune_key ? tune_key : "-", ns, M, N, nbins,
-                std::round(8.0 * std::log2(static_cast<double>(std::max(1, maxch)))) / 8.0);
+  // pairs of the longest bin, not chunks: a chunk's width is the kernel's, and saved choices outlive it
+  std::snprintf(key, sizeof(key), "%s i8x%d M=%d N=%d bins=%d pairs~2^%.3f", tune_key ? tune_key : "-", ns, M, N, nbins,
+                std::round(8.0 * std::log2(static_cast<double>(std::max(1, maxcnt)))) / 8.0);
   if (!tune_key) return run(heur, false);              // accumulating callers: no trials
   int splitk = heur;
   bool tried = false;

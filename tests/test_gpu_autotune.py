@@ -84,3 +84,27 @@ def test_autotuned_sigc_f16_kernel(qsgw, tmp_path):
     keys = [k for k in out["report"] if k.startswith("sigc_f16 kernel ngb=150")]
     assert len(keys) == 1 and out["report"][keys[0]] in (0, 1, 2)
     assert max(out["errs"]) < 2e-5
+
+
+def test_saved_int8_choices_of_another_chunk_width_do_not_match(qsgw, tmp_path):
+    """Keys hold the pair count: a file written when a chunk was 32, 64 or 128 pairs wide is passed by."""
+    import torch
+    p = synth.chi0_problem(N=70, nk=5, nocc=3, nun=(40, 60), niw=3, seed=43)
+    n, npair = p["N"], int(np.sum(p["nocc"] * p["nun"]))
+    name = f"chi0_lorentz i8x3 M={n} N={n} bins=3"
+    text = lambda what, x: f"{name} {what}~2^{np.round(8 * np.log2(x)) / 8:.3f}"
+    old = {text("chunks", -(-npair // w)): 63 for w in (32, 64, 128)}
+    cache = tmp_path / "tune.json"
+    cache.write_text(json.dumps(old))
+    qsgw.set_precision(qsgw.PREC_SPLIT_I8, 3)
+    qsgw.set_autotune(1, cache)
+    try:
+        chi = torch.zeros(n * n * 3, dtype=torch.complex128, device="cuda")
+        qsgw.chi0_lorentz_d(chi, n, 3, p["freq_i"], p["nk"], p["nocc"], p["nun"], p["eocc_h"], p["eun_h"],
+                            qsgw.to_device(p["zcols"]))
+        qsgw.synchronize()
+        rep = qsgw.autotune_report()
+        assert rep[text("pairs", npair)] != 63
+    finally:
+        qsgw.set_autotune(0, None)
+        qsgw.set_precision(qsgw.PREC_FP64)
