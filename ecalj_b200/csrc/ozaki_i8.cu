@@ -275,7 +275,6 @@ struct SegParams {
   int cps;                    // K chunks per segment
   int klast;                  // 32-byte K steps of a segment's last chunk
   int nslot, T;               // A' tile coordinate (q nslot + slot) T + mt
-  int nrows;                  // B rows per slice (tile-ordered columns)
   const int* tile_group;
   const int* tile_cols;
   const int* group_seg_off;
@@ -287,7 +286,6 @@ struct SegParams {
   double post;                // 256^(NS - 1) / U8^2 (slice_unit8)
   double2* const* tile_out;   // [tile] output of the tile's task: column col at tile_out[t] + col ldc
   long long ldc;
-  int tail;                   // 1: M mod 64 <= 32 and the last row tile holds segment pairs (mapT)
   int* err;
 };
 
@@ -1332,14 +1330,12 @@ int OzSigcBatch::launch(cudaStream_t s) {
     rc = make_tensor_map(&mt, CU_TENSOR_MAP_DATA_TYPE_UINT8, g_t8.p, 4, dims, str, box, swz);
     if (rc) return rc;
   }
-  p.tail = tail ? 1 : 0;
   p.M = M_;
   p.ntm = T;
   p.cps = (Kp + static_cast<int>(kb) - 1) / static_cast<int>(kb);
   p.klast = (Kp - (p.cps - 1) * static_cast<int>(kb)) / 32;
   p.nslot = static_cast<int>(cap_slot_);
   p.T = T;
-  p.nrows = static_cast<int>(nrows);
   p.tile_cols = g_cols.as<int>();
   p.mu_a = g_mu.as<double>(); p.nu_b = g_nu.as<double>();
   p.post = post_scale8(ns);

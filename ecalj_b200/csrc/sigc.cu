@@ -265,10 +265,6 @@ static DevBuf g_sc_trial;                // Sigma_c of the slice-count trials
 // at ngb = 600), so the inputs of the next tasks keep the copy engine busy through a long kernel
 static HostRing g_sc_ring(12);
 
-static int grid_for(long long n) {
-  return static_cast<int>(std::max<long long>(1, std::min<long long>((n + 255) / 256, 16LL * ctx().sm_count)));
-}
-
 static int sxcf_check(const qsgw_sxcf_args* a) {
   QSGW_ARG(a, "sxcf: null args");
   QSGW_ARG(a->ngb >= 1 && a->ntqxx >= 0 && a->ntq >= a->ntqxx && a->niw >= 1 && a->nw >= 2,

@@ -229,7 +229,15 @@ int zgemm_f64(int opa, int opb, int m, int n, int k, double2 alpha,
   return launch_kernel<ZM_GEMM, false, false>(p, grid, s);
 }
 
+// The gathered modes' conjugations and contiguous directions are constants of the kernel.
+static int gather_check(const ZParams& p, bool contiguous) {
+  if (contiguous && p.a_conj && !p.b_conj) return QSGW_OK;
+  set_error("FP64 engine: the gathered modes form conj(A) B with contiguous operands");
+  return QSGW_ERR_ARG;
+}
+
 int zgemm_chi0_launch(ZParams p, int nbins, int herm, int splitk, cudaStream_t s) {
+  if (int rc = gather_check(p, p.a_rs == 1 && p.b_rs == 1)) return rc;
   p.herm = herm;
   p.splitk = splitk;
   const int ntiles = herm ? p.ntm * (p.ntm + 1) / 2 : p.ntm * p.ntn;
@@ -242,6 +250,7 @@ int zgemm_seg_launch(ZParams p, int ncol_tiles, int mean_nseg, cudaStream_t s) {
     set_error("segmented GEMM: %d column tiles exceed the grid limit", ncol_tiles);
     return QSGW_ERR_UNSUPPORTED;
   }
+  if (int rc = gather_check(p, (p.a_rs == 1 || p.a_ks == 1) && p.b_ks == 1)) return rc;
   p.ntm = (p.M + ZG_BM - 1) / ZG_BM;
   // few tiles (one task of a small cell): the segments are split over CTAs that add into C
   p.splitk = zgemm_splitk(static_cast<long long>(p.ntm) * ncol_tiles, mean_nseg * ((p.K + ZG_BK - 1) / ZG_BK));
