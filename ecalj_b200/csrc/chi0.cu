@@ -21,21 +21,20 @@ namespace qsgw {
 static DevBuf g_x0_idx, g_x0_w, g_x0_bins, g_x0_zm, g_x0_rc;
 
 struct BinTables {
-  std::vector<int> colidx;
-  std::vector<double> wts;
   std::vector<int> cnt, slab;
   std::vector<long long> off;
   int maxcnt = 0;
+  void add(int c, long long o, int sl) {
+    cnt.push_back(c);
+    off.push_back(o);
+    slab.push_back(sl);
+    maxcnt = std::max(maxcnt, c);
+  }
 };
 
-// Returns the number of chunks of the longest bin.
+// Returns the number of chunks of the longest bin; the pair columns and weights are on the device already.
 static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc) {
   const size_t nb = bt.cnt.size();
-  const size_t ni = bt.colidx.size();
-  rc = g_x0_idx.ensure(std::max<size_t>(ni, 1) * sizeof(int));
-  if (rc) return 0;
-  rc = g_x0_w.ensure(std::max<size_t>(ni, 1) * sizeof(double));
-  if (rc) return 0;
   const size_t bin_bytes = nb * (2 * sizeof(int) + sizeof(long long));
   rc = g_x0_bins.ensure(std::max<size_t>(bin_bytes, 64));
   if (rc) return 0;
@@ -43,8 +42,6 @@ static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc)
   memcpy(hb.data(), bt.off.data(), nb * sizeof(long long));
   memcpy(hb.data() + nb * sizeof(long long), bt.cnt.data(), nb * sizeof(int));
   memcpy(hb.data() + nb * (sizeof(long long) + sizeof(int)), bt.slab.data(), nb * sizeof(int));
-  if ((rc = h2d(g_x0_idx.p, bt.colidx.data(), ni * sizeof(int), s))) return 0;
-  if ((rc = h2d(g_x0_w.p, bt.wts.data(), ni * sizeof(double), s))) return 0;
   if ((rc = h2d(g_x0_bins.p, hb.data(), bin_bytes, s))) return 0;
   unsigned char* base = g_x0_bins.as<unsigned char>();
   p.bin_coff = reinterpret_cast<const long long*>(base);
@@ -56,11 +53,17 @@ static int upload_bins(const BinTables& bt, ZParams& p, cudaStream_t s, int& rc)
   return (bt.maxcnt + ZG_BK - 1) / ZG_BK;
 }
 
-// Bins of at most this many pairs on average stay on the FP64 engine in the int8 mode too: it is the more
-// accurate and, there, the faster one, as the int8 path's slicing passes and its CTAs' start and end cost more
-// than the products.  Measured per call (FP64 / 3 slices, us): 300 rows, 80 bins of 32 pairs 170 / 288, of 128
-// 390 / 414, of 256 711 / 610; 600 rows, 40 bins of 32 226 / 405, of 128 426 / 433, of 256 747 / 528.
-constexpr int kFp64BinPairs = 128;
+// In the int8 mode a bin of at most kFp64BinPairs pairs stays on the FP64 engine: it is the more accurate and, there,
+// the faster one, as the int8 path's slicing passes and its CTAs' start and end cost more than the products.  Per call
+// of 80 equal bins (FP64 / 3 slices, us): 300 rows, bins of 32 pairs 129 / 256, of 128 299 / 325, of 192 405 / 373; 600
+// rows 318 / 664, 723 / 769, 1002 / 847; 1000 rows, of 128 1749 / 1693, of 192 2456 / 1810.
+// The longer bins go to the int8 path together if they outweigh its fixed cost (scales, ranges, slicing launches:
+// about 35 us), counted in pairs beyond kFp64BinPairs times 64 x 64 output tiles -- 160 rows, 24 bins of 256 pairs
+// (18 000) 109 / 122, 80 of 256 (61 000) 307 / 308; 600 rows, 4 of 192 (14 000) 96 / 102, 24 of 192 (84 000) 334 / 300 --
+// or if one of them is so long that the FP64 engine's chain over its chunks (0.17 us a pair) would.  95 bins of 10 and
+// one of 8000 pairs at 300 and 600 rows: 255 and 508 us (all on FP64 2509 and 2704, all on int8 481 and 992).
+constexpr int kFp64BinPairs = 128, kFp64LongestBin = 512;
+constexpr long long kFp64PairTiles = 32768;
 
 static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int nwhis, int npm,
                          int ns1, int ns2, const double2* zmel, int nbb, int nm1, int nm2,
@@ -91,17 +94,12 @@ static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int n
     for (int iw = 1; iw <= nwhis; ++iw) {
       const int b = (jpm - 1) * nwhis + (iw - 1);
       start[b] = tot;
-      if (cnt[b] > 0) {
-        bt.cnt.push_back(cnt[b]);
-        bt.off.push_back(tot);
-        bt.slab.push_back(iw * (3 - 2 * jpm) - (1 - npm) * nwhis);
-        bt.maxcnt = std::max(bt.maxcnt, cnt[b]);
-      }
+      if (cnt[b] > 0) bt.add(cnt[b], tot, iw * (3 - 2 * jpm) - (1 - npm) * nwhis);
       tot += cnt[b];
     }
   if (bt.cnt.empty()) return QSGW_OK;
-  bt.colidx.resize(tot);
-  bt.wts.resize(tot);
+  std::vector<int> colidx(tot);
+  std::vector<double> wts(tot);
   std::vector<long long> fill(start);
   for (int icoun = icounkmink; icoun <= icounkmaxk; ++icoun) {
     const int c = icoun - 1;
@@ -110,45 +108,56 @@ static int x0gemm_device(double2* rcxq, int npr, int ipr_col, int npr_col, int n
     const int col = (it - nm1) + nmz * (itp - 1);
     for (int iw = iwini[c]; iw <= iwend[c]; ++iw) {
       const int b = (jpm - 1) * nwhis + (iw - 1);
-      bt.colidx[fill[b]] = col;
-      bt.wts[fill[b]] = whwc[iw - iwini[c] + icouini[c] - 1];   // x0gemm.f90:62
+      colidx[fill[b]] = col;
+      wts[fill[b]] = whwc[iw - iwini[c] + icouini[c] - 1];   // x0gemm.f90:62
       fill[b]++;
     }
   }
-  if (ctx().prec_mode == QSGW_PREC_SPLIT_I8 && tot > kFp64BinPairs * static_cast<long long>(bt.cnt.size())) {
-    // the same bins on the int8 tensor-core path: the pair columns and weights go to the device,
-    // each bin's entries form one K range; rcxq accumulates (no tuning trials)
-    int rc = g_x0_idx.ensure(std::max<size_t>(tot, 1) * sizeof(int));
-    if (rc) return rc;
-    rc = g_x0_w.ensure(std::max<size_t>(tot, 1) * sizeof(double));
-    if (rc) return rc;
-    if ((rc = h2d(g_x0_idx.p, bt.colidx.data(), tot * sizeof(int), s))) return rc;
-    if ((rc = h2d(g_x0_w.p, bt.wts.data(), tot * sizeof(double), s))) return rc;
-    OzChi0Bins ob;
-    ob.ebeg = bt.off;
-    ob.cnt = bt.cnt;
-    ob.slab = bt.slab;
+  int rc = g_x0_idx.ensure(tot * sizeof(int));
+  if (rc) return rc;
+  if ((rc = g_x0_w.ensure(tot * sizeof(double)))) return rc;
+  if ((rc = h2d(g_x0_idx.p, colidx.data(), tot * sizeof(int), s))) return rc;
+  if ((rc = h2d(g_x0_w.p, wts.data(), tot * sizeof(double), s))) return rc;
+  const int herm = (ipr_col == 1 && npr_col == npr) ? 1 : 0;
+  const int ntm = (npr + ZG_BM - 1) / ZG_BM, ntn = (npr_col + ZG_BN - 1) / ZG_BN;
+  const long long ntiles = herm ? ntm * (ntm + 1LL) / 2 : static_cast<long long>(ntm) * ntn;
+  if (ctx().prec_mode == QSGW_PREC_SPLIT_I8) {
+    BinTables longer, rest;
+    long long beyond = 0;
     int classes = 0;
-    for (double w : bt.wts) classes |= (w < 0.0 ? 1 : 0) | (w > 0.0 ? 2 : 0);
-    const bool herm = (ipr_col == 1 && npr_col == npr);
-    const int ns = ctx().nslices > 0 ? ctx().nslices : 4;   // rcxq accumulates: no trials, the accurate count
-    return chi0_split_i8(rcxq, npr, static_cast<long long>(npr) * npr_col, npr, npr_col, ipr_col - 1, herm, zmel, nbb,
-                         static_cast<long long>(nmz) * nqtot, g_x0_idx.as<int>(), g_x0_w.as<double>(), ob, classes,
+    for (size_t i = 0; i < bt.cnt.size(); ++i) {
+      if (bt.cnt[i] <= kFp64BinPairs) {
+        rest.add(bt.cnt[i], bt.off[i], bt.slab[i]);
+        continue;
+      }
+      longer.add(bt.cnt[i], bt.off[i], bt.slab[i]);
+      beyond += bt.cnt[i] - kFp64BinPairs;
+      for (long long e = bt.off[i]; e < bt.off[i] + bt.cnt[i]; ++e) classes |= (wts[e] < 0.0 ? 1 : 0) | (wts[e] > 0.0 ? 2 : 0);
+    }
+    if (beyond * ntiles >= kFp64PairTiles || longer.maxcnt > kFp64LongestBin) {
+      // the pair columns and weights of a bin form one K range; rcxq accumulates (no tuning trials)
+      OzChi0Bins ob;
+      ob.ebeg = longer.off;
+      ob.cnt = longer.cnt;
+      ob.slab = longer.slab;
+      const int ns = ctx().nslices > 0 ? ctx().nslices : 4;   // rcxq accumulates: no trials, the accurate count
+      rc = chi0_split_i8(rcxq, npr, static_cast<long long>(npr) * npr_col, npr, npr_col, ipr_col - 1, herm != 0, zmel,
+                         nbb, static_cast<long long>(nmz) * nqtot, g_x0_idx.as<int>(), g_x0_w.as<double>(), ob, classes,
                          ns, s, nullptr);
+      if (rc || rest.cnt.empty()) return rc;
+      bt = rest;
+    }
   }
   ZParams p{};
   p.M = npr; p.N = npr_col;
   p.A = zmel; p.a_rs = 1; p.a_ks = nbb; p.a_conj = 1;               // zw^H   (:76, :88 opA=C)
   p.B = zmel + (ipr_col - 1); p.b_rs = 1; p.b_ks = nbb; p.b_conj = 0;  // wzw   (:84)
   p.C = rcxq; p.ldc = npr; p.c_bs = static_cast<long long>(npr) * npr_col;
-  p.ntm = (npr + ZG_BM - 1) / ZG_BM; p.ntn = (npr_col + ZG_BN - 1) / ZG_BN;
-  int rc = 0;
+  p.ntm = ntm; p.ntn = ntn;
   const int maxch = upload_bins(bt, p, s, rc);
   if (rc) return rc;
-  const int herm = (ipr_col == 1 && npr_col == npr) ? 1 : 0;
-  const int ntiles = herm ? p.ntm * (p.ntm + 1) / 2 : p.ntm * p.ntn;
   const int nbins = static_cast<int>(bt.cnt.size());
-  const int sk = zgemm_splitk(static_cast<long long>(ntiles) * nbins, maxch);
+  const int sk = zgemm_splitk(ntiles * nbins, maxch);
   p.kch_per_split = (maxch + sk - 1) / sk;
   rc = zgemm_chi0_launch(p, nbins, herm, sk, s);
   if (rc) return rc;

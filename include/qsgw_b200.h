@@ -67,7 +67,10 @@ int qsgw_set_host_async(int on);
  * int8 slices per operand for SPLIT_I8 (2, 3 or 4: about 14, 21 or 28 bits
  * relative to the largest element of a row / column, products accumulated
  * exactly).  Applies to the chi0 (qsgw_chi0_lorentz*, qsgw_x0gemm*), Sigma_c
- * (qsgw_sxcf_correlation*) and zmel M->E (qsgw_zmel_m2e_d) contractions. */
+ * (qsgw_sxcf_correlation*) and zmel M->E (qsgw_zmel_m2e_d) contractions.
+ * With SPLIT_I8, qsgw_x0gemm* keeps in FP64 the bins of few pairs (128 at
+ * most), where FP64 is the faster one, and a call whose longer bins hold too
+ * little work for the int8 kernels. */
 int qsgw_set_precision(int mode, int nslices);
 /* Targets of the automatic slice count (SPLIT_I8 with nslices = 0): on the
  * first call of each problem shape the contraction runs at 4 slices and at 2

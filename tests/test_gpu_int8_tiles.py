@@ -53,7 +53,7 @@ def test_chi0_hermitian_tiles(qsgw, i8, n, ns):
             assert np.array_equal(got[:, :, iw], got[:, :, iw].conj().T)
 
 
-@pytest.mark.parametrize("ncoun", [60, 640, 641, 1500])       # 128 pairs a bin: the FP64 engine up to there
+@pytest.mark.parametrize("ncoun", [60, 640, 1500, 3000])      # FP64 up to 300 pairs a bin, int8 at 600
 @pytest.mark.parametrize("npr,ipr_col,npr_col", [(130, 1, 130), (70, 3, 129)])
 def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col, ncoun):
     rng = np.random.default_rng(npr)
@@ -74,7 +74,46 @@ def test_x0gemm_bins_add_to_what_is_there(qsgw, i8, npr, ipr_col, npr_col, ncoun
     assert np.linalg.norm(out[1] - out[0]) <= 6 * 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** -28 * inc + 1e-14 * np.linalg.norm(r0)
 
 
-@pytest.mark.parametrize("ncoun", [60, 1500])                # the FP64 engine's route and the int8 one
+def _bins(rng, cnts, nm, nq):
+    """Pair tables of bins with the given pair counts, in mixed order; weights of both signs."""
+    bin_ = rng.permutation(np.repeat(np.arange(1, len(cnts) + 1), cnts))
+    n = len(bin_)
+    return n, (rng.integers(1, nm + 1, n), rng.integers(1, nq + 1, n), np.ones(n, int), bin_, bin_,
+               np.arange(1, n + 1)), rng.uniform(-1, 1, n)
+
+
+@pytest.mark.parametrize("cnts,fp64,int8", [([128] * 5, 1, 0),             # short bins
+                                            ([129] * 5, 1, 0),             # longer ones that do not pay
+                                            ([10] * 40 + [513], 1, 1),     # one long bin among short ones
+                                            ([600, 700, 513], 0, 1)])
+def test_x0gemm_route_by_bins(qsgw, i8, cnts, fp64, int8):
+    """In the int8 mode each bin runs where it is faster; every bin is added once."""
+    import torch
+    rng = np.random.default_rng(len(cnts))
+    n, nm, nq = 70, 4, 6
+    z = _rc(rng, n, nm, nq)
+    ncoun, tabs, w = _bins(rng, cnts, nm, nq)
+    r0 = _rc(rng, n, n, len(cnts) + 1)
+    out = []
+    for ns in (0, 4):
+        if ns:
+            i8(ns)
+        r = qsgw.to_device(r0)
+        qsgw.profile(True)
+        qsgw.x0gemm(r, n, 1, n, len(cnts), 1, 1, nm, qsgw.to_device(z), 1, 1, ncoun, *tabs, w, zmel_shape=(n, nm, nq),
+                    device=True)
+        qsgw.synchronize()
+        launches = [qsgw.profile_get(t)[1] for t in ("chi0_dmma", "chi0_tc")]
+        qsgw.profile(False)
+        out.append(qsgw.from_device(r, r0.shape))
+    assert launches == [fp64, 2 * int8]                        # one int8 launch per sign of the weights
+    for b, c in enumerate(cnts, 1):
+        inc = np.linalg.norm(out[0][:, :, b] - r0[:, :, b])
+        tol = 1e-13 if c <= 128 or not int8 else 6 * 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** -28
+        assert np.linalg.norm(out[1][:, :, b] - out[0][:, :, b]) <= tol * inc + 1e-14 * np.linalg.norm(r0[:, :, b])
+
+
+@pytest.mark.parametrize("ncoun", [60, 3000])                # the FP64 engine's route and the int8 one
 def test_x0gemm_recorded_in_a_graph(qsgw, i8, ncoun):
     """A recorded call replays with its own copy of the pair tables."""
     import torch
