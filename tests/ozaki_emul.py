@@ -106,12 +106,14 @@ def complex_product(a, b, ns, mu_rows=None, nu_cols=None, bits=7):
     return (re + 1j * im) * mu_rows[:, None] * nu_cols[None, :]
 
 
-def chi0_dense(zcols, w, ns):
+def chi0_dense(zcols, w, ns, zmax=None):
     """Emulated chi0(:, :, j) = sum_p w[j, p] conj(z_p) z_p^T of the SPLIT_I8
     path for weights of one sign per slot: y = sqrt(|w|) z, rows scaled by
-    2^e >= sqrt(max |w_j|) max_p |z(m, p)| (max over Re and Im)."""
+    2^e >= sqrt(max |w_j|) max_p |z(m, p)| (max over Re and Im; zmax when the
+    call's columns are more than these)."""
     z = np.asarray(zcols)
-    zmax = np.maximum(np.abs(z.real), np.abs(z.imag)).max(axis=1)
+    if zmax is None:
+        zmax = np.maximum(np.abs(z.real), np.abs(z.imag)).max(axis=1)
     out = np.zeros((z.shape[0], z.shape[0], w.shape[0]), np.complex128, order='F')
     for j in range(w.shape[0]):
         wj = np.asarray(w[j])

@@ -44,6 +44,24 @@ def test_jacobi_equal_eigenvalues(qsgw, n):
     assert np.abs(z.conj().T @ z - np.eye(n)).max() <= tol
 
 
+def test_jacobi_equal_eigenvalues_of_the_largest_cell(qsgw):
+    """n = 1500, two distinct eigenvalues: the most sweeps met (44 of the 60 allowed)."""
+    import torch
+    n = 1500
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, _ = torch.linalg.qr(torch.randn(n, n, dtype=torch.complex128, device="cuda", generator=g))
+    lam = torch.repeat_interleave(torch.tensor([3.0, 1.0], dtype=torch.float64, device="cuda"), n // 2)
+    v = (q * lam) @ q.conj().T
+    v = 0.5 * (v + v.conj().T)
+    d = v.T.contiguous().reshape(-1).clone()                 # column-major
+    got = torch.from_numpy(qsgw.zhegv_d(d, n)).cuda()
+    z = d.view(n, n).T
+    tol = 64 * n * np.finfo(float).eps
+    assert (got - lam).abs().max() <= tol * 3
+    assert ((z * got) @ z.conj().T - v).abs().max() <= tol * 3
+    assert (z.conj().T @ z - torch.eye(n, device="cuda")).abs().max() <= tol
+
+
 @pytest.mark.parametrize("exp10", [-140, -155, -200, -300, 100])
 def test_jacobi_small_and_large_entries(qsgw, exp10):
     """Rotations are chosen from squares of the entries: a small matrix is solved as its multiple of order one."""

@@ -1,14 +1,14 @@
-"""The int8 kernels at the edges of their tiles and splits, against the FP64 path on the same inputs.
+"""The int8 kernels at the edges of their tiles and splits, against the CPU emulation of the same digits and kept
+slice pairs.
 
-Bounds: an operand element is rounded to 2^-(7 ns) (chi0) or about 2^-(8 ns - 1) (Sigma_c, M -> E) of the largest of
-its row or column, products below the last slice are dropped (ns of them), and the rounding errors of K terms add
-with random signs: relative to the row and column scales the error of an element stays below
-(ns + 2) unit sqrt(K) and the tests compare Frobenius norms of whole outputs."""
+Bounds: the integer products are exact, so kernel and emulation differ by the FP64 rounding of the scaled sums: some
+eps of the terms that are added, whatever the slice count."""
 import numpy as np
 import pytest
 
 from ecalj_b200 import sched, synth
 from oracle import sxcf
+from tests import ozaki_emul
 
 pytestmark = pytest.mark.gpu
 
@@ -34,22 +34,19 @@ def test_chi0_hermitian_tiles(qsgw, i8, n, ns):
     import torch
     for nun in (3, 40):
         p = synth.chi0_problem(N=n, nk=3, nocc=2, nun=(nun, nun + 2), niw=3, seed=n + nun)
-        z = qsgw.to_device(p["zcols"])
-        out = []
-        for mode in ("fp64", "i8"):
-            if mode == "i8":
-                i8(ns)
-            else:
-                qsgw.set_precision(qsgw.PREC_FP64, 1)
-            chi = torch.zeros(n * n * 3, dtype=torch.complex128, device="cuda")
-            qsgw.chi0_lorentz_d(chi, n, 3, p["freq_i"], 3, p["nocc"], p["nun"], p["eocc_h"], p["eun_h"], z)
-            qsgw.synchronize()
-            out.append(qsgw.from_device(chi, (n, n, 3)))
-        ref, got = out
+        oo, uo = (np.concatenate([[0], np.cumsum(p[k])]) for k in ("nocc", "nun"))
+        de = np.concatenate([(p["eun_h"][uo[k]:uo[k + 1]][None, :] - p["eocc_h"][oo[k]:oo[k + 1]][:, None])
+                             .reshape(-1, order="F") for k in range(3)])
+        w = -2.0 * de[None, :] / (de[None, :] ** 2 + p["freq_i"][:, None] ** 2) / 3
+        emu = ozaki_emul.chi0_dense(p["zcols"], w, ns)
+        i8(ns)
+        chi = torch.zeros(n * n * 3, dtype=torch.complex128, device="cuda")
+        qsgw.chi0_lorentz_d(chi, n, 3, p["freq_i"], 3, p["nocc"], p["nun"], p["eocc_h"], p["eun_h"],
+                            qsgw.to_device(p["zcols"]))
+        qsgw.synchronize()
+        got = qsgw.from_device(chi, (n, n, 3))
         for iw in range(3):
-            # row scale: sqrt(max |w|) max |z| rounded up to a power of two, against sqrt(|w|) |z| (weights span 80)
-            unit = 2.0 * PEAK * np.sqrt(80.0) * 2.0 ** (-7 * ns)
-            assert np.linalg.norm(got[:, :, iw] - ref[:, :, iw]) <= (ns + 2) * unit * np.linalg.norm(ref[:, :, iw])
+            assert np.linalg.norm(got[:, :, iw] - emu[:, :, iw]) <= 1e-12 * np.linalg.norm(emu[:, :, iw])
             assert np.array_equal(got[:, :, iw], got[:, :, iw].conj().T)
 
 
@@ -113,6 +110,29 @@ def test_x0gemm_route_by_bins(qsgw, i8, cnts, fp64, int8):
         assert np.linalg.norm(out[1][:, :, b] - out[0][:, :, b]) <= tol * inc + 1e-14 * np.linalg.norm(r0[:, :, b])
 
 
+@pytest.mark.parametrize("ns", [2, 3, 4])
+@pytest.mark.parametrize("npr,ipr_col,npr_col", [(130, 1, 130), (70, 3, 129)])
+def test_x0gemm_chunk_remainders(qsgw, i8, npr, ipr_col, npr_col, ns):
+    """Pair counts at the edges of the 128-, 64- and 32-pair pieces of a chunk, columns gathered from a list."""
+    rng = np.random.default_rng(ns)
+    cnts = [640, 641, 672, 673, 704, 705, 767]
+    nbb, nm, nq = 140, 5, 60
+    z = _rc(rng, nbb, nm, nq)
+    ncoun, tabs, w = _bins(rng, cnts, nm, nq)
+    r0 = _rc(rng, npr, npr_col, len(cnts) + 1)
+    got = r0.copy(order="F")
+    i8(ns)
+    qsgw.x0gemm(got, npr, ipr_col, npr_col, len(cnts), 1, 1, nm, z, 1, 1, ncoun, *tabs, w)
+    zf = z.reshape(nbb, -1, order="F")
+    zmax = np.maximum(np.abs(zf.real), np.abs(zf.imag)).max(axis=1)
+    for b in range(1, len(cnts) + 1):
+        sel = tabs[3] == b
+        col = (tabs[0] - 1 + nm * (tabs[1] - 1))[sel]
+        emu = ozaki_emul.chi0_dense(zf[:, col], w[sel][None, :], ns, zmax)[:npr, ipr_col - 1:ipr_col - 1 + npr_col, 0]
+        err = np.linalg.norm(got[:, :, b] - r0[:, :, b] - emu)
+        assert err <= 1e-12 * np.linalg.norm(emu) + 1e-15 * np.linalg.norm(r0[:, :, b])
+
+
 @pytest.mark.parametrize("ncoun", [60, 3000])                # the FP64 engine's route and the int8 one
 def test_x0gemm_recorded_in_a_graph(qsgw, i8, ncoun):
     """A recorded call replays with its own copy of the pair tables."""
@@ -166,14 +186,17 @@ def test_sigma_segment_splits_and_chunks(qsgw, i8, n, nm, ntq, ns):
     rng = np.random.default_rng(n)
     w = _rc(rng, n, n, 12)
     wi, wr = np.asfortranarray(w + w.conj().transpose(1, 0, 2)), _rc(rng, n, n, 30)
-    ref = _sigma(qsgw, t, wi, wr, n, nm, ntq)
     i8(ns)
     got = _sigma(qsgw, t, wi, wr, n, nm, ntq)
+    nwxi, nwx, ntmax = sched.get_nwx(t["omega"], t["ekc"], t["freq_r"], t["ef"], t["esmr"])
+    emu = np.zeros((ntq, ntq), complex, order="F")
+    ozaki_emul.correlation_block(emu, t["zmel"], 1, nm, min(nm, ntmax), nwxi, nwx, ntq, wi, wr, t["omega"], t["ekc"], 0,
+                                 t["ef"], t["esmr"], 1 / 8, t["ua"], t["x"], t["wx"], t["expa"], t["freq_r"], ns=ns)
     # Sigma adds nm n terms of czmelwc^H zmel; its elements cancel, so the scale is that of the unsigned sum
     wg = sxcf.wgtim(t["omega"], t["ekc"], 0, 1, nm, ntq, t["esmr"], 1 / 8, t["ua"], t["x"], t["wx"], t["expa"])
     scale = np.abs(wg).sum(0).max() * np.linalg.norm(t["zmel"]) ** 2 * max(np.linalg.norm(x, 2) for x in
                                                                           wi.transpose(2, 0, 1))
-    assert np.linalg.norm(got - ref) <= 2 * (ns + 2) * PEAK * 2.0 ** (1 - 8 * ns) * scale
+    assert np.linalg.norm(got - emu) <= 1e-14 * scale
 
 
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 65])

@@ -141,13 +141,15 @@ def test_chi0_i8_matches_emulation_and_oracle(i8, ns, cfg):
     assert e_ref < GATE[ns]
 
 
-@pytest.mark.parametrize("npr,ipr_col,npr_col,npm", [(200, 1, 200, 2), (131, 40, 61, 1), (65, 1, 65, 2)])
-def test_x0gemm_i8_vs_oracle(i8, npr, ipr_col, npr_col, npm):
+@pytest.mark.parametrize("ns", [2, 3, 4])
+@pytest.mark.parametrize("npr,ipr_col,npr_col,npm,ncoun", [(200, 1, 200, 2, 4800), (131, 40, 61, 1, 2400),
+                                                           (65, 1, 65, 2, 4800)])
+def test_x0gemm_i8_vs_oracle(i8, npr, ipr_col, npr_col, npm, ncoun, ns):
     """The reference's own chi0 boundary (pair/bin lists, jpm, ragged bins,
     ipr_col column blocks, weights of both signs, accumulation into rcxq) on the
-    int8 path."""
+    int8 path: bins of several hundred pairs, none short enough for FP64."""
     rng = np.random.default_rng(npr + npm)
-    nbb, nm1, nm2, nqtot, nwhis, ncoun = max(npr, ipr_col - 1 + npr_col) + 3, 3, 12, 17, 6, 400
+    nbb, nm1, nm2, nqtot, nwhis = max(npr, ipr_col - 1 + npr_col) + 3, 3, 12, 17, 6
     z = _rc(rng, nbb, nm2 - nm1 + 1, nqtot)
     itc = rng.integers(nm1, nm2 + 1, ncoun); itpc = rng.integers(1, nqtot + 1, ncoun)
     jpmc = rng.integers(1, npm + 1, ncoun); iwini = rng.integers(1, nwhis + 1, ncoun)
@@ -159,13 +161,17 @@ def test_x0gemm_i8_vs_oracle(i8, npr, ipr_col, npr_col, npm):
     ref = r0.copy(order='F')
     x0.x0gemm(ref, npr, ipr_col, npr_col, nwhis, npm, 4, 11, z, nm1, 5, ncoun - 3,
               itc, itpc, jpmc, iwini, iwend, icouini, whwc)
-    i8.set_precision(i8.PREC_SPLIT_I8, 4)
+    i8.set_precision(i8.PREC_SPLIT_I8, ns)
     got = r0.copy(order='F')
+    i8.profile(True)
     i8.x0gemm(got, npr, ipr_col, npr_col, nwhis, npm, 4, 11, z, nm1, 5, ncoun - 3,
               itc, itpc, jpmc, iwini, iwend, icouini, whwc)
+    launches = [i8.profile_get(t)[1] for t in ("chi0_dmma", "chi0_tc")]
+    i8.profile(False)
+    assert launches == [0, 2]                              # no bin in FP64, one launch per sign of the weights
     err = rel_fro(got - r0, ref - r0)
-    print(f"x0gemm i8x4 npr={npr} ipr_col={ipr_col} npr_col={npr_col} npm={npm}: added part vs oracle {err:.2e}")
-    assert err < GATE[4] * 10
+    print(f"x0gemm i8x{ns} npr={npr} ipr_col={ipr_col} npr_col={npr_col} npm={npm}: added part vs oracle {err:.2e}")
+    assert err < GATE[ns] * 10
 
 
 def test_set_precision_validates_i8_slices(qsgw):

@@ -23,15 +23,18 @@ def test_tetra_chain_vs_oracle(qsgw):
     _chain(qsgw, degenerate=False)
 
 
-@pytest.mark.parametrize("ns,tol", [(3, 3e-5), (4, 3e-7)])
-def test_tetra_chain_int8(qsgw, ns, tol):
-    """The same chain with x0gemm on the int8 Ozaki path (the reference's own
-    chi0 boundary: the pair/bin lists of the tetrahedron weights, accumulated
-    per k into rcxq), against the oracle chain with the same weights."""
+@pytest.mark.parametrize("ns", [3, 4])
+def test_tetra_chain_int8_mode(qsgw, ns):
+    """The same chain in the int8 mode: its bins of at most 18 pairs a k stay on
+    the FP64 engine, so the FP64 gates hold (x0gemm on the int8 kernel:
+    test_gpu_ozaki.py, test_gpu_int8_tiles.py)."""
     try:
         qsgw.set_precision(qsgw.PREC_SPLIT_I8, ns)
-        _chain(qsgw, degenerate=False, tol=tol)
+        qsgw.profile(True)
+        _chain(qsgw, degenerate=False)
+        assert qsgw.profile_get("chi0_tc")[1] == 0
     finally:
+        qsgw.profile(False)
         qsgw.set_precision(qsgw.PREC_FP64, 1)
 
 
@@ -42,8 +45,7 @@ def test_tetra_chain_degenerate_bands(qsgw):
     _chain(qsgw, degenerate=True)
 
 
-def _chain(qsgw, degenerate, tol=None):
-    """tol: the gate of a split-precision x0gemm (None: the FP64 gates)."""
+def _chain(qsgw, degenerate):
     import torch
     idt, qbzw, ek, ekq = synth.tetra_mesh(3)
     if degenerate:
@@ -92,9 +94,6 @@ def _chain(qsgw, degenerate, tol=None):
 
     ri, rr = oracle_chain(w)                                     # the GPU's weights
     print(f"tetra chain, same weights: imag {rel_fro(gi, ri):.2e} real {rel_fro(gr, rr):.2e}")
-    if tol is not None:
-        assert rel_fro(gi, ri) < tol and rel_fro(gr, rr) < tol
-        return
     assert rel_fro(gi, ri) < 1e-11
     assert rel_fro(gr, rr) < 1e-11
     wref, _ = tw.tetwt_hist(idt, qbzw, ek, ekq, ef, frhis, nocc, nunocc)
