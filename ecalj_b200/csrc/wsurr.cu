@@ -38,7 +38,7 @@ struct State {
   float* grad = nullptr;
   float* m1 = nullptr;
   float* m2 = nullptr;
-  float* red = nullptr;        // [0] = sum of w e^2, [1] = sum of w
+  double* red = nullptr;       // [0] = sum of w e^2, [1] = sum of w
   double* lsq = nullptr;       // normal equations of the heads: G[NTMAX][NIN*NIN], then H[NTMAX][NIN]
   int step = 0;
   int cap = 0;                 // batch capacity of the buffers below
@@ -97,16 +97,23 @@ __device__ __forceinline__ void store_run(__nv_bfloat16* dst, const uint32_t (&w
     reinterpret_cast<uint4*>(dst)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Forward pass, layer 1 and the linear head: one block = 32 samples, thread = hidden unit.
 // h1 = relu(x W1 + b1) in BF16 (row-major, and transposed into h1t when training, rows
 // beyond the batch up to the 32-row block zero); head[r] = C[t_r] . x_r (FP32 master
-// parameters).  With wt and sumw (training) the sum of the sample weights is added to *sumw.
+// parameters).  With wt and sumw (training) the sum of the sample weights is added to *sumw, in FP64: thousands of
+// FP32 additions in no fixed order moved the loss by 1.6e-6 from call to call.
 __global__ void __launch_bounds__(256) forward_l1_kernel(const float* __restrict__ x, const int* __restrict__ tix,
                                                          int batch, const __nv_bfloat16* __restrict__ w,
                                                          const float* __restrict__ master,
                                                          __nv_bfloat16* __restrict__ h1, __nv_bfloat16* __restrict__ h1t,
                                                          long long ldt, float* __restrict__ head,
-                                                         const float* __restrict__ wt, float* __restrict__ sumw) {
+                                                         const float* __restrict__ wt, double* __restrict__ sumw) {
   __shared__ float sx[32][NIN];
   const int s0 = blockIdx.x * 32;
   const int tid = threadIdx.x;
@@ -124,7 +131,10 @@ __global__ void __launch_bounds__(256) forward_l1_kernel(const float* __restrict
       for (int i = 0; i < NIN; ++i) a += c[i] * sx[tid][i];
     }
     head[s0 + tid] = a;
-    if (wt && sumw) atomicAdd(sumw, wt[s0 + tid]);
+  }
+  if (tid < 32 && wt && sumw) {
+    const double v = warp_sum(s0 + tid < batch ? wt[s0 + tid] : 0.0);
+    if (tid == 0) atomicAdd(sumw, v);
   }
   float wcol[NIN];
 #pragma unroll
@@ -376,24 +386,27 @@ __global__ void __launch_bounds__(256) backward_act_kernel(const float* __restri
                                                            const float* __restrict__ out, float* __restrict__ g2,
                                                            __nv_bfloat16* __restrict__ g2b,
                                                            __nv_bfloat16* __restrict__ g2t, long long ldt,
-                                                           float* __restrict__ grad, float* __restrict__ red) {
+                                                           float* __restrict__ grad, double* __restrict__ red) {
   __shared__ float sd[32];      // dL/dout for the MLP part (0 on linear-only rows)
   __shared__ float sdh[32];     // dL/dout for the head
   const int s0 = blockIdx.x * 32;
   const int tid = threadIdx.x;
-  const float inv_sumw = wt ? 1.f / fmaxf(red[1], 1e-30f) : 1.f / batch;
+  const float inv_sumw = wt ? 1.f / fmaxf(static_cast<float>(red[1]), 1e-30f) : 1.f / batch;
   if (tid < 32) {
     float d = 0.f;
+    double we2 = 0.0;
     int t = -1;
     if (s0 + tid < batch) {
       const float e = out[s0 + tid] - y[s0 + tid];
       const float wr = wt ? wt[s0 + tid] : 1.f;
       d = 2.f * wr * e * inv_sumw;
-      atomicAdd(&red[0], wr * e * e);
+      we2 = static_cast<double>(wr) * e * e;
       t = tix[s0 + tid];
     }
     sdh[tid] = d;
     sd[tid] = (t < NMLP) ? d : 0.f;
+    we2 = warp_sum(we2);
+    if (tid == 0) atomicAdd(&red[0], we2);
   }
   __syncthreads();
   // dC[t][i] += d_r x_r[i]
@@ -746,7 +759,7 @@ static void forward_pass(const float* x, const int* tix, int batch, bool train, 
 // forward + backward on (x, tix, y, wt) rows already on the device; gradient in g.grad, loss terms in g.red
 static int grad_pass(const float* x, const int* tix, const float* y, const float* wt, int batch, cudaStream_t s) {
   QSGW_CUDA(cudaMemsetAsync(g.grad, 0, NPARAM * sizeof(float), s));
-  QSGW_CUDA(cudaMemsetAsync(g.red, 0, 2 * sizeof(float), s));
+  QSGW_CUDA(cudaMemsetAsync(g.red, 0, 2 * sizeof(double), s));
   const int nb = (batch + 31) / 32;
   forward_pass(x, tix, batch, true, wt, s);
   backward_act_kernel<<<nb, NH, 0, s>>>(x, tix, y, wt, batch, g.w16, g.h2, g.out, g.g2, g.g2b, g.g2t, ldt(), g.grad,
@@ -785,10 +798,10 @@ static int adam_step(float lr, cudaStream_t s) {
 
 // host loss = sum w e^2 / sum w (or mean e^2 without weights)
 static int read_loss(float* loss_host, int batch, bool weighted, cudaStream_t s) {
-  float red[2];
+  double red[2];
   QSGW_CUDA(cudaMemcpyAsync(red, g.red, sizeof(red), cudaMemcpyDeviceToHost, s));
   QSGW_CUDA(cudaStreamSynchronize(s));
-  *loss_host = weighted ? red[0] / std::max(red[1], 1e-30f) : red[0] / batch;
+  *loss_host = static_cast<float>(weighted ? red[0] / std::max(red[1], 1e-30) : red[0] / batch);
   return QSGW_OK;
 }
 
@@ -822,7 +835,7 @@ extern "C" int qsgw_wsurr_init(unsigned long long seed) {
     QSGW_CUDA(cudaMalloc(&g.grad, NPARAM * sizeof(float)));
     QSGW_CUDA(cudaMalloc(&g.m1, NPARAM * sizeof(float)));
     QSGW_CUDA(cudaMalloc(&g.m2, NPARAM * sizeof(float)));
-    QSGW_CUDA(cudaMalloc(&g.red, 2 * sizeof(float)));
+    QSGW_CUDA(cudaMalloc(&g.red, 2 * sizeof(double)));
     QSGW_CUDA(cudaMalloc(&g.lsq, NTMAX * (NIN * NIN + NIN) * sizeof(double)));
     g.ready = true;
   }

@@ -69,3 +69,19 @@ def test_gradient_row_blocks(qsgw, batch):
     for a, b in ((mlp.OFF_W1, mlp.OFF_B1), (mlp.OFF_B1, mlp.OFF_W2), (mlp.OFF_B2, mlp.OFF_W3)):
         # BF16 neighbours of h1 and g2 (2^-9 of a term, random signs)
         assert np.linalg.norm(grad[a:b] - ref[a:b]) <= 2e-3 * np.linalg.norm(ref[a:b])
+
+
+def test_loss_does_not_depend_on_the_order_of_its_sums(qsgw):
+    """Eight calls on the same rows, and on the rows shuffled: one rounding of FP32 apart at most."""
+    import torch
+    p, rng = _net(qsgw, 12)
+    n = 8191
+    x = rng.uniform(-1, 1, (n, 16)).astype(np.float32)
+    tix = rng.integers(0, mlp.NTMAX, n).astype(np.int32)
+    ys, w = rng.standard_normal(n).astype(np.float32), rng.uniform(0.1, 1.1, n).astype(np.float32)
+    loss = []
+    for i in range(8):
+        o = rng.permutation(n) if i % 2 else np.arange(n)
+        dev = [torch.from_numpy(np.ascontiguousarray(a[o])).cuda() for a in (x, tix, ys, w)]
+        loss.append(qsgw.wsurr_grad_d(dev[0], dev[1], dev[2], n, dev[3])[0])
+    assert max(loss) - min(loss) <= 2.0 ** -23 * max(loss)
