@@ -37,6 +37,33 @@ def test_inference_rows(qsgw, n, shift):
     assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-4 * max(1.0, np.linalg.norm(ref))
 
 
+def test_layer_one_against_64_bits(qsgw):
+    """W2 the identity and W3 one unit: y is that unit's h1.  It is the BF16 rounding of the 64-bit sum but where the
+    sum lies within its own error of a rounding boundary: 17 FP32 roundings of sums of order 0.2 (3e-7 at most)
+    against BF16 steps of 5e-4 to 1e-3, one value in a thousand at most."""
+    import torch
+    p, rng = _net(qsgw, 11)
+    p[mlp.OFF_W2:mlp.OFF_B2] = np.eye(mlp.NH, dtype=np.float32).ravel()
+    p[mlp.OFF_B2:mlp.OFF_W3] = 0.0
+    p[mlp.OFF_B3:] = 0.0
+    bf16 = lambda v: torch.from_numpy(np.asarray(v)).to(torch.bfloat16).double().numpy()
+    n, units, off = 4096, (0, 7, 8, 15, 16, 100, 255), 0
+    x = rng.uniform(-1, 1, (n, 16)).astype(np.float32)
+    xd, td = torch.from_numpy(x.ravel()).cuda(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    y = torch.zeros(n, dtype=torch.float32, device="cuda")
+    w1, b1 = bf16(p[:mlp.OFF_B1]).reshape(16, mlp.NH), bf16(p[mlp.OFF_B1:mlp.OFF_W2])
+    for j in units:
+        p[mlp.OFF_W3:mlp.OFF_B3] = 0.0
+        p[mlp.OFF_W3 + j] = 1.0
+        qsgw.wsurr_params(p)
+        qsgw.wsurr_forward_d(xd, td, y, n)
+        qsgw.synchronize()
+        got, ref = y.cpu().numpy().astype(float), bf16(np.maximum(x.astype(float) @ w1[:, j] + b1[j], 0.0))
+        off += int((got != ref).sum())
+        assert np.all(np.abs(got - ref) <= 2.0 ** -7 * ref + 1e-6)
+    assert off <= 1e-3 * n * len(units)
+
+
 def test_inference_infinite_and_nan_inputs_stay_in_their_rows(qsgw):
     import torch
     p, rng = _net(qsgw, 5)
