@@ -394,7 +394,8 @@ static int jacobi_solve(double2* A, long long lda, double2* V, int n, std::vecto
   set_identity_kernel<<<grid_for(static_cast<long long>(n) * n), 256, 0, s>>>(V, n, n);
   count_launch();
   bool converged = (n <= 1);
-  // many equal eigenvalues are the slow case: 23, 30 and 34 sweeps at n = 64, 260 and 400 with four in all
+  // many equal eigenvalues are the slow case: 25, 32, 34, 38 and 40 sweeps at n = 64, 260, 400, 800 and 1500 with four
+  // in all, 27, 37, 34, 42 and 44 with two
   for (int sweep = 0; sweep < 60 && !converged; ++sweep) {
     for (int t = 0; t < ne - 1; ++t) {
       QSGW_CUDA(cudaLaunchKernelEx(&solve, jacobi_solve_kernel, static_cast<const double2*>(cur), U, n, ne, t));

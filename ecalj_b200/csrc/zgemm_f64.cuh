@@ -10,7 +10,7 @@
 // pipe needs several warps per SM sub-partition: two CTAs of 8 warps keep
 // four there (128 registers a thread) where 4-warp CTAs of 32x32 a warp kept
 // two and lost a third of the cycles to issue waits and barriers.  1536^3:
-// 32 TFLOP/s, DMMA pipe 90 % busy (cuBLAS 35); the basis change of 24
+// 32 TFLOP/s (cuBLAS 35), DMMA pipe 85 % busy in the chi0 mode at 600 rows; the basis change of 24
 // matrices of 600: 1.70 -> 1.46 ms; chi0 of 260 rows, 12 800 pairs and 12
 // frequencies (with the tile rules below) 3.99 -> 2.10 ms.  At 128 registers
 // the gathered modes spill easily: strides, conjugations and the tile's
