@@ -28,16 +28,23 @@ struct Context {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   std::vector<void*> graph_host;      // pinned copies of host tables the graph reads
+  std::vector<void*> graph_dev;       // outgrown scratch the graph's nodes point into
 };
 
 Context& ctx();
 void set_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
 
+// Graphs recorded so far, and the release of device scratch allocated when `born` of them were: what the recorded
+// graph may point into is kept until that graph goes.
+unsigned long long graphs_recorded();
+void scratch_free(void* p, unsigned long long born);
+
 // Grows-only device scratch buffer owned by the library.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  unsigned long long born = 0;        // graphs recorded when it was allocated
   int ensure(size_t n);
   void release();
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }

@@ -39,6 +39,13 @@ int check_cuda(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? QSGW_ERR_OOM : QSGW_ERR_CUDA;
 }
 
+static unsigned long long g_graphs = 0;   // outlives the context, as the scratch does
+unsigned long long graphs_recorded() { return g_graphs; }
+void scratch_free(void* p, unsigned long long born) {
+  if (p && g_ctx.graph_exec && born < g_graphs) g_ctx.graph_dev.push_back(p);
+  else if (p) cudaFree(p);
+}
+
 int DevBuf::ensure(size_t n) {
   if (n <= bytes && p) return QSGW_OK;
   if (g_ctx.capturing) {
@@ -47,7 +54,8 @@ int DevBuf::ensure(size_t n) {
               "qsgw_graph_begin", n);
     return QSGW_ERR_UNSUPPORTED;
   }
-  if (p) cudaFree(p);
+  scratch_free(p, born);
+  born = g_graphs;
   p = nullptr;
   bytes = 0;
   size_t want = n < 256 ? 256 : n;
@@ -310,6 +318,8 @@ static void graph_free() {
   c.graph = nullptr;
   for (void* p : c.graph_host) cudaFreeHost(p);
   c.graph_host.clear();
+  for (void* p : c.graph_dev) cudaFree(p);
+  c.graph_dev.clear();
 }
 
 extern "C" int qsgw_graph_begin(void) {
@@ -342,6 +352,7 @@ extern "C" int qsgw_graph_end(void) {
   c.graph = g;
   rc = check_cuda(cudaGraphInstantiate(&c.graph_exec, g, 0), "graph_end: cudaGraphInstantiate");
   if (rc) graph_free();
+  else ++g_graphs;
   return rc;
 }
 

@@ -42,6 +42,7 @@ struct State {
   double* lsq = nullptr;       // normal equations of the heads: G[NTMAX][NIN*NIN], then H[NTMAX][NIN]
   int step = 0;
   int cap = 0;                 // batch capacity of the buffers below
+  unsigned long long born = 0; // graphs recorded when they were allocated
   __nv_bfloat16* w2t = nullptr;  // W2 transposed [n][k] (BF16), the forward GEMM's B operand
   __nv_bfloat16* h1 = nullptr;   // layer-1 activations (batch x NH, BF16: the layer-2 GEMM's operand)
   __nv_bfloat16* h1t = nullptr;  // the same transposed (NH x cap), the weight-gradient GEMM's operand
@@ -697,9 +698,11 @@ static bool chol_solve(double* a, double* b, int n) {
 }
 
 static void free_batch() {
-  cudaFree(g.h1); cudaFree(g.h1t); cudaFree(g.h2); cudaFree(g.g1); cudaFree(g.g2); cudaFree(g.g2b);
-  cudaFree(g.g2t); cudaFree(g.head); cudaFree(g.out);
-  cudaFree(g.xb); cudaFree(g.yb); cudaFree(g.wb); cudaFree(g.tb);
+  for (void* p : {static_cast<void*>(g.h1), static_cast<void*>(g.h1t), static_cast<void*>(g.h2), static_cast<void*>(g.g1),
+                  static_cast<void*>(g.g2), static_cast<void*>(g.g2b), static_cast<void*>(g.g2t),
+                  static_cast<void*>(g.head), static_cast<void*>(g.out), static_cast<void*>(g.xb),
+                  static_cast<void*>(g.yb), static_cast<void*>(g.wb), static_cast<void*>(g.tb)})
+    scratch_free(p, g.born);
   g.h2 = g.g1 = g.g2 = g.head = g.out = g.xb = g.yb = g.wb = nullptr;
   g.h1 = g.h1t = g.g2b = g.g2t = nullptr;
   g.tb = nullptr;
@@ -731,6 +734,7 @@ static int ensure_cap(int batch) {
   QSGW_CUDA(cudaMalloc(&g.wb, b * sizeof(float)));
   QSGW_CUDA(cudaMalloc(&g.tb, b * sizeof(int)));
   g.cap = batch;
+  g.born = graphs_recorded();
   return QSGW_OK;
 }
 

@@ -393,6 +393,7 @@ int qsgw_autotune_report(char *buf, int len);
  * memory owned by the graph and replayed as recorded; device arrays are read
  * at replay time.  Record only after the same calls ran once (scratch must
  * not grow while recording: such a call fails with QSGW_ERR_UNSUPPORTED).
+ * Scratch that later calls outgrow is kept for the graph until it goes.
  * One graph per context; begin replaces the previous one.  The library
  * stream must not be the legacy default stream.                          */
 int qsgw_graph_begin(void);

@@ -159,3 +159,46 @@ def test_exchange_recorded_in_a_graph(qsgw):
         vcoud[:] = 1.0
 
     _replays_as_recorded(qsgw, call, zsec, spoil)
+
+
+def test_scratch_outgrown_after_recording_is_kept(qsgw):
+    """Later calls of a larger shape take new scratch; the graph goes on with the one it was recorded with."""
+    import torch
+    rng = np.random.default_rng(9)
+
+    def problem(ngb, nm, ntq):
+        z = qsgw.to_device(_rc(rng, ngb, nm, ntq))
+        vcoud, ekc = 10 ** rng.uniform(-2, 3, ngb), np.sort(rng.uniform(-1, 1, nm))
+        zsec = torch.zeros(ntq * ntq, dtype=torch.complex128, device="cuda")
+        x = torch.from_numpy(rng.uniform(-1, 1, (ngb, 16)).astype(np.float32).ravel()).cuda()
+        buf = torch.zeros(ngb * 16 + 4, dtype=torch.float32, device="cuda")
+        buf[1:1 + ngb * 16] = x                               # not 16-byte aligned: the layer-by-layer route
+        y, tix = torch.zeros(ngb, device="cuda"), torch.zeros(ngb, dtype=torch.int32, device="cuda")
+
+        def call():
+            zsec.zero_()
+            qsgw.sxcf_exchange_d(zsec, ntq, z, ngb, 1, nm, ntq, vcoud, ekc, 0, 0.1, 0.02, 0.125)
+            qsgw.wsurr_forward_d(buf[1:1 + ngb * 16], tix, y, ngb)
+        return call, zsec, y
+
+    qsgw.wsurr_init(3)
+    small, zs, ys = problem(20, 9, 4)
+    large, zl, yl = problem(70001, 2, 3)
+    small()
+    qsgw.synchronize()
+    ref = zs.clone(), ys.clone()
+    qsgw.graph_begin()
+    small()
+    qsgw.graph_end()
+    for _ in range(2):
+        large()
+    fill = [torch.full((1 << 22,), 3.0, device="cuda") for _ in range(8)]      # whatever reuses released memory
+    out = zl.clone(), yl.clone()
+    ys.zero_()
+    qsgw.graph_launch()
+    large()
+    qsgw.synchronize()
+    qsgw.graph_destroy()
+    assert len(fill) == 8
+    for a, b in zip((zs, ys, zl, yl), ref + out):
+        assert rel_fro(a.cpu().numpy(), b.cpu().numpy()) <= 1e-12 and float(b.abs().max()) > 0
